@@ -10,7 +10,7 @@
 // runs the same walk with the forward terms over the sources.
 #include <cuda_runtime.h>
 
-#include "device.cuh"
+#include "pairs.cuh"
 
 namespace qmbx {
 
@@ -581,19 +581,79 @@ struct DiagAdd : VisitorBase {
     }
 };
 
-// The first 32 bytes of a hit log: written by the forward call, checked by
-// the replay before it reads anything else.
+// Hits of a pair scan: (slot of the forward part | parity << 31, row of
+// configs_i, row of configs_j, 0), for the forward map (CONJ = false: from i
+// to j) or the adjoint (conjugated, from j to i).  Sums go to the output row
+// with FP64 atomics, the products formed as PivotHits forms them.
+template <int W, bool CONJ, bool F32>
+struct PairHits {
+    const void* val;        // amplitude per first row of the input side
+    const double2* coef;    // forward part
+    const float4* coef32;
+    double2* res;           // per first row of the output side
+    HitLog log;
+    __device__ __forceinline__ void record(const int4* q, int n, int lane) const {
+        if (log.hits == nullptr || n <= 0) return;
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(log.count, (unsigned long long)n);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (lane < n && base + lane < (unsigned long long)log.cap) {
+            const int4 h = q[lane];
+            log.hits[base + lane] = make_int4(h.y, h.z, h.x, 0);
+        }
+    }
+    __device__ __forceinline__ void apply(int4 h) const {
+        const int64_t slot = h.x & 0x7fffffff;
+        const int from = CONJ ? h.z : h.y, to = CONJ ? h.y : h.z;
+        double re, im;
+        if (F32) {
+            const float4 cf = __ldg(coef32 + slot);
+            const float2 p = __ldg(static_cast<const float2*>(val) + from);
+            const float chi = CONJ ? -cf.z : cf.z, cli = CONJ ? -cf.w : cf.w;
+            float x1, e1, x2, e2;
+            two_prod(cf.x, p.x, x1, e1);
+            two_prod(chi, p.y, x2, e2);
+            float lo = __fadd_rn(__fsub_rn(e1, e2), __fsub_rn(__fmul_rn(cf.y, p.x), __fmul_rn(cli, p.y)));
+            re = ((double)x1 - (double)x2) + (double)lo;
+            two_prod(cf.x, p.y, x1, e1);
+            two_prod(chi, p.x, x2, e2);
+            lo = __fadd_rn(__fadd_rn(e1, e2), __fadd_rn(__fmul_rn(cf.y, p.y), __fmul_rn(cli, p.x)));
+            im = ((double)x1 + (double)x2) + (double)lo;
+        } else {
+            const double2 cf = __ldg(coef + slot);
+            const double2 p = __ldg(static_cast<const double2*>(val) + from);
+            const double ci = CONJ ? -cf.y : cf.y;
+            re = cf.x * p.x - ci * p.y;
+            im = cf.x * p.y + ci * p.x;
+        }
+        if (h.x < 0) {
+            re = -re;
+            im = -im;
+        }
+        atomicAdd(&res[to].x, re);
+        atomicAdd(&res[to].y, im);
+    }
+};
+
+// The first bytes of a hit log: written by the forward call, checked by the
+// replay before it reads anything else.
 struct LogHead {
     unsigned long long count;  // hits found (more than the capacity: the log is incomplete)
     int32_t dir;               // 0: walked the input side, 1: the output side, 2: nothing walked
     int32_t magic;
     int64_t n_i, n_j;          // the forward call's row counts (n_j = n_i for same_configs)
     int64_t cap;               // and its capacity in hits
+    int32_t diag_dir;          // the side whose rows the diagonal records were made over (as dir)
+    int32_t pairs;             // 1: the forward scanned pairs, whose prepared rows it left in the buffer
 };
 constexpr int32_t kLogMagic = 0x51484c47;
 
-__global__ void log_head_kernel(LogHead* h, int dir, int64_t n_i, int64_t n_j, int64_t cap) {
-    h->dir = dir;
+// scan (device int, or NULL): whether the call scans pairs, whose hits run from configs_i
+__global__ void log_head_kernel(LogHead* h, int dir, const int* scan, int64_t n_i, int64_t n_j, int64_t cap) {
+    const bool pairs = scan != nullptr && *scan != 0;
+    h->dir = pairs ? 0 : dir;
+    h->diag_dir = dir;
+    h->pairs = pairs ? 1 : 0;
     h->magic = kLogMagic;
     h->n_i = n_i;
     h->n_j = n_j;
@@ -844,6 +904,68 @@ int walk_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_s
     return QMBX_OK;
 }
 
+// apply_within by the pair scan: hits of the changing terms added into res
+// (cleared by the caller), then the diagonal terms over the side the walks
+// would take.  gate (device int): nothing is scanned when it is 0, and it is
+// the number of rows of the diagonal pass.
+template <int W>
+int pair_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_set, const PairWork& pairs,
+               const void* val, double2* res, const int* gate, cudaStream_t s, int group = kGroupEnumerate,
+               int diag_group = kGroupDiagonal) {
+    const PartView fwd = part_view(a.table_host, a.table_dev, QMBX_PART_FWD);
+    const PartView diag = part_view(a.table_host, a.table_dev, QMBX_PART_DIAG);
+    const bool f32 = a.prec == Prec::F32C;
+    int st = QMBX_OK;
+#define QMBX_PAIR_CASE(CONJ, F32)                                                                        \
+    {                                                                                                    \
+        PairHits<W, CONJ, F32> v{val, fwd.coef, fwd.coef32, res, a.log};                                 \
+        st = launch_pair_scan<W>(v, pairs, a.table_host, a.table_dev, gate, s, group);                   \
+    }
+    if (a.adjoint) {
+        if (f32) QMBX_PAIR_CASE(true, true) else QMBX_PAIR_CASE(true, false)
+    } else {
+        if (f32) QMBX_PAIR_CASE(false, true) else QMBX_PAIR_CASE(false, false)
+    }
+#undef QMBX_PAIR_CASE
+    if (st != QMBX_OK || diag.n == 0 || !(a.prec == Prec::F64 || a.include_diag)) return st;
+    const bool scatter = apply_scatter(a, in_set.n, out_set.n);
+    HashRows walk = scatter ? in_set : out_set;
+    walk.count = const_cast<int*>(gate);
+    const HashView look = scatter ? out_set.hash() : in_set.hash();
+#define QMBX_DIAG_CASE(CONJ, F32, SCATTER)                                                                      \
+    {                                                                                                           \
+        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res, a.log};      \
+        st = launch_diag<W>(dv, walk, fwd, diag, s, diag_group);                                                \
+    }
+    if (scatter) {
+        if (a.adjoint) {
+            if (f32) QMBX_DIAG_CASE(true, true, true) else QMBX_DIAG_CASE(true, false, true)
+        } else {
+            if (f32) QMBX_DIAG_CASE(false, true, true) else QMBX_DIAG_CASE(false, false, true)
+        }
+    } else {
+        if (a.adjoint) {
+            if (f32) QMBX_DIAG_CASE(true, true, false) else QMBX_DIAG_CASE(true, false, false)
+        } else {
+            if (f32) QMBX_DIAG_CASE(false, true, false) else QMBX_DIAG_CASE(false, false, false)
+        }
+    }
+#undef QMBX_DIAG_CASE
+    return st;
+}
+
+// The pair scan's scratch of a call behind the first `base` bytes of its
+// workspace; false when the sizes give it none or it does not fit.
+template <int W>
+bool take_pairs_behind(const ApplyArgs& a, const Arena& ws, uint64_t base, PairWork& pairs) {
+    const qmbx_table_header* h = header_of(a.table_host);
+    if (!pairs_scratch(h, a.n_i, a.n_j)) return false;
+    Arena rest = ws;
+    rest.used = base;
+    pairs = take_pair_work<W>(rest, a.n_i, a.n_j, a.same, h->n_sites);
+    return rest.fits();
+}
+
 // Forward maps amplitudes on configs_i (input side) to configs_j (output
 // side); the adjoint maps configs_j to configs_i.  Gather walks the output
 // side's distinct rows (daggered terms for the forward map) and sums in
@@ -870,7 +992,7 @@ int apply_impl(const ApplyArgs& a, Arena& ws, cudaStream_t s) {
     if (a.log.hits != nullptr) {
         // an empty record until the walk below fills it (direction 2: nothing walked)
         QMBX_CUDA_TRY(cudaMemsetAsync(a.log.count, 0, sizeof(unsigned long long), s));
-        QMBX_KERNEL(kGroupOther, s, log_head_kernel<<<1, 1, 0, s>>>(a.log_head, 2, a.n_i, a.n_j, a.log.cap));
+        QMBX_KERNEL(kGroupOther, s, log_head_kernel<<<1, 1, 0, s>>>(a.log_head, 2, nullptr, a.n_i, a.n_j, a.log.cap));
     }
     if (n_out == 0) return QMBX_OK;
     int st;
@@ -900,7 +1022,18 @@ int apply_impl(const ApplyArgs& a, Arena& ws, cudaStream_t s) {
 
     const bool scatter = apply_scatter(a, n_in, n_out);
     const HashRows& walked = scatter ? in_set : out_set;
-    if (scatter || choose_walk(walk_part_of(a, scatter), walked.n, !deterministic_mode()) == Walk::kPivot) {
+    PairWork pairs{};
+    bool scan = pairs_wanted(h, a.n_i, a.n_j);
+    if (scan) {
+        uint64_t needed = 0, with_pairs = 0;
+        if ((st = apply_within_workspace_for(a.table_host, a.n_i, a.n_j, a.same, &needed, &with_pairs)) != QMBX_OK) return st;
+        scan = take_pairs_behind<W>(a, ws, needed, pairs);
+    }
+    if (scan && ((st = build_pairs<W>(rs_i, rs_j, h->n_sites, pairs, s)) != QMBX_OK ||
+                 (st = choose_pairs<W>(pairs, walked, s)) != QMBX_OK)) {
+        return st;
+    }
+    if (scan || scatter || choose_walk(walk_part_of(a, scatter), walked.n, !deterministic_mode()) == Walk::kPivot) {
         QMBX_CUDA_TRY(cudaMemsetAsync(res, 0, (size_t)n_out * sizeof(double2), s));
     }
     if (a.log.hits != nullptr) {
@@ -908,9 +1041,11 @@ int apply_impl(const ApplyArgs& a, Arena& ws, cudaStream_t s) {
         // direction (every record the replay reads, not only the walked
         // side's: the replay runs over max(n_i, n_j) of them)
         QMBX_CUDA_TRY(cudaMemsetAsync(a.log.diag_rows, 0xff, (size_t)a.log_rows * sizeof(int2), s));
-        QMBX_KERNEL(kGroupOther, s, log_head_kernel<<<1, 1, 0, s>>>(a.log_head, scatter ? 0 : 1, a.n_i, a.n_j, a.log.cap));
+        QMBX_KERNEL(kGroupOther, s, log_head_kernel<<<1, 1, 0, s>>>(a.log_head, scatter ? 0 : 1, scan ? pairs.gate : nullptr, a.n_i, a.n_j, a.log.cap));
     }
-    if ((st = walk_apply<W>(a, in_set, out_set, val, res, nullptr, s)) != QMBX_OK) return st;
+    // the device chooses one of the two; the other finds no rows
+    if (scan && (st = pair_apply<W>(a, in_set, out_set, pairs, val, res, pairs.gate, s)) != QMBX_OK) return st;
+    if ((st = walk_apply<W>(a, in_set, out_set, val, res, scan ? pairs.gate + 1 : nullptr, s)) != QMBX_OK) return st;
     QMBX_KERNEL(kGroupOther, s, apply_finalize_kernel<<<grid_for(n_out, kThreads), kThreads, 0, s>>>(res, out_set.first, n_out, a.adjoint ? 1 : 0, a.out64, a.out32));
     QMBX_LAUNCH_CHECK("apply_finalize_kernel");
     return QMBX_OK;
@@ -987,8 +1122,10 @@ namespace qmbx {
 
 // Workspace of an apply_within call on n_i x n_j rows, for one value of
 // same_configs (one row set instead of two when it is set): the largest of
-// the forward / adjoint, FP64 / FP32 layouts (they differ by one value array).
-int apply_within_workspace_for(const void* table_host, int64_t n_i, int64_t n_j, bool same, uint64_t* bytes) {
+// the forward / adjoint, FP64 / FP32 layouts (they differ by one value array),
+// and the same with the pair scan's scratch behind it.
+int apply_within_workspace_for(const void* table_host, int64_t n_i, int64_t n_j, bool same, uint64_t* needed,
+                               uint64_t* with_pairs) {
     const qmbx_table_header* h = header_of(table_host);
     if (h == nullptr || h->magic != QMBX_MAGIC) return fail(QMBX_ERR_ARGUMENT, "not a compiled qmbx table");
     ApplyArgs a{};
@@ -1005,7 +1142,18 @@ int apply_within_workspace_for(const void* table_host, int64_t n_i, int64_t n_j,
         if (st != QMBX_OK) return st;
         if (probe.used > most) most = probe.used;
     }
-    *bytes = most;
+    *needed = *with_pairs = most;
+    if (pairs_scratch(h, a.n_i, a.n_j)) {
+        Arena rest(nullptr, 0);
+        rest.used = most;
+        switch (h->n_words) {
+            case 1: take_pair_work<1>(rest, a.n_i, a.n_j, same, h->n_sites); break;
+            case 2: take_pair_work<2>(rest, a.n_i, a.n_j, same, h->n_sites); break;
+            case 3: take_pair_work<3>(rest, a.n_i, a.n_j, same, h->n_sites); break;
+            default: take_pair_work<4>(rest, a.n_i, a.n_j, same, h->n_sites); break;
+        }
+        *with_pairs = rest.used;
+    }
     return QMBX_OK;
 }
 
@@ -1015,7 +1163,8 @@ extern "C" int qmbx_apply_within_workspace(const void* table_host, int64_t n_i, 
     clear_error();
     if (bytes == nullptr) return fail(QMBX_ERR_ARGUMENT, "bytes must not be NULL");
     // sized for two row sets, which also covers same_configs calls
-    return apply_within_workspace_for(table_host, n_i, n_j, false, bytes);
+    uint64_t needed = 0;
+    return apply_within_workspace_for(table_host, n_i, n_j, false, &needed, bytes);
 }
 
 extern "C" int qmbx_apply_within(const void* table_host, const void* table_dev, const uint8_t* configs_i,
@@ -1093,7 +1242,7 @@ namespace qmbx {
 namespace {
 
 struct LogLayout {
-    uint64_t gate, diag_rows, diag_val, res, hits, ws, ws_bytes, total;
+    uint64_t gate, diag_rows, diag_val, res, hits, ws, ws_needed, ws_bytes, total;  // ws_needed: without the pair scan's scratch
 };
 
 // Device flags of one adjoint replay, written by log_gate_kernel.
@@ -1101,15 +1250,15 @@ struct LogGate {
     int valid;   // the header is a logged forward's with these row counts and capacity
     int replay;  // valid and the record holds every hit: replay it
     int rows;    // valid and the record is incomplete: rows the adjoint walk takes (else 0)
-    int pad;
+    int pairs;   // or, where both calls scan pairs, rows of the scan's diagonal pass (else 0)
 };
 
 // The log buffer: header, gate, diagonal records, the adjoint's per-row
 // sums, cap hit records, then the forward's own workspace (its row sets,
 // which the adjoint reuses).
 int log_layout(const void* table_host, int64_t n_i, int64_t n_j, bool same, int64_t cap, LogLayout& L) {
-    uint64_t ws_bytes = 0;
-    int st = apply_within_workspace_for(table_host, n_i, same ? n_i : n_j, same, &ws_bytes);
+    uint64_t ws_needed = 0, ws_bytes = 0;
+    int st = apply_within_workspace_for(table_host, n_i, same ? n_i : n_j, same, &ws_needed, &ws_bytes);
     if (st != QMBX_OK) return st;
     if (same) n_j = n_i;
     Arena a(nullptr, 0);
@@ -1126,6 +1275,7 @@ int log_layout(const void* table_host, int64_t n_i, int64_t n_j, bool same, int6
     L.hits = a.used;
     a.take<int4>((uint64_t)(cap > 0 ? cap : 1));
     L.ws = a.used;
+    L.ws_needed = ws_needed;
     L.ws_bytes = ws_bytes;
     a.take<unsigned char>(ws_bytes > 0 ? ws_bytes : 1);
     L.total = a.used;
@@ -1165,13 +1315,15 @@ int attach_log(ApplyArgs& a, void* log, uint64_t log_bytes, int64_t cap, void** 
 // walked set's distinct rows) when it is incomplete, neither when the buffer
 // holds no matching log (the output is then NaN).
 __global__ void log_gate_kernel(const LogHead* __restrict__ h, int64_t n_i, int64_t n_j, int64_t cap,
-                                const int* __restrict__ walk_rows, LogGate* __restrict__ g) {
+                                const int* __restrict__ walk_rows, int may_scan, LogGate* __restrict__ g) {
     const bool valid = h->magic == kLogMagic && h->dir >= 0 && h->dir <= 2 && h->n_i == n_i && h->n_j == n_j &&
                        h->cap == cap;
     const bool complete = valid && h->count <= (unsigned long long)cap;
     g->valid = valid ? 1 : 0;
     g->replay = complete && h->dir != 2 ? 1 : 0;
-    g->rows = valid && !complete ? *walk_rows : 0;
+    const bool scan = may_scan && h->pairs;
+    g->rows = valid && !complete && !scan ? *walk_rows : 0;
+    g->pairs = valid && !complete && scan ? *walk_rows : 0;
 }
 
 __global__ void log_poison_kernel(const LogGate* __restrict__ g, int64_t n, double2* out64, float2* out32) {
@@ -1343,7 +1495,7 @@ __global__ void log_diag_adjoint_kernel(const int2* __restrict__ rows, const dou
     if (i >= n || !gate->replay) return;
     const int2 d = rows[i];
     if (d.y < 0) return;
-    const int dir = head->dir;
+    const int dir = head->diag_dir;
     const int out = dir == 0 ? d.x : d.y;
     const int in = dir == 0 ? d.y : d.x;
     const double2 v = vals[i];
@@ -1382,8 +1534,10 @@ int adjoint_from_log_impl(const void* table_host, const void* table_dev, char* b
                 g, out64, out32, include_diag, {}, nullptr, 0};
     const bool scatter = apply_scatter(a, n_j, n_i);
     const HashRows& walked = scatter ? rs_j : rs_i;
+    PairWork pairs{};
+    const bool scan = pairs_wanted(header_of(table_host), n_i, n_j) && take_pairs_behind<W>(a, ws, L.ws_needed, pairs);
     QMBX_CUDA_TRY(cudaMemsetAsync(res, 0, (size_t)n_i * sizeof(double2), s));
-    QMBX_KERNEL(kGroupOther, s, log_gate_kernel<<<1, 1, 0, s>>>(head, n_i, n_j, cap, walked.count, gate));
+    QMBX_KERNEL(kGroupOther, s, log_gate_kernel<<<1, 1, 0, s>>>(head, n_i, n_j, cap, walked.count, scan ? 1 : 0, gate));
     const PartView fwd = part_view(table_host, table_dev, QMBX_PART_FWD);
     const PartView adj = part_view(table_host, table_dev, QMBX_PART_ADJ);
     const int64_t nw = n_i > n_j ? n_i : n_j;
@@ -1402,6 +1556,12 @@ int adjoint_from_log_impl(const void* table_host, const void* table_dev, char* b
     // an incomplete record: the adjoint walk (its walked rows gated by the device count; 0 otherwise)
     int st = walk_apply<W>(a, rs_j, rs_i, g, res, &gate->rows, s, kGroupSpmv, kGroupSpmv);
     if (st != QMBX_OK) return st;
+    // or the scan again, over the prepared rows the forward left in the buffer
+    if (scan) {
+        pairs.i.count = rs_i.count;
+        pairs.j.count = rs_j.count;
+        if ((st = pair_apply<W>(a, rs_j, rs_i, pairs, g, res, &gate->pairs, s, kGroupSpmv, kGroupSpmv)) != QMBX_OK) return st;
+    }
     QMBX_KERNEL(kGroupOther, s, apply_finalize_kernel<<<grid_for(n_i, kThreads), kThreads, 0, s>>>(res, rs_i.first, n_i, 1, out64, out32));
     QMBX_KERNEL(kGroupOther, s, log_poison_kernel<<<grid_for(n_i, kThreads), kThreads, 0, s>>>(gate, n_i, out64, out32));
     QMBX_LAUNCH_CHECK("adjoint from log");

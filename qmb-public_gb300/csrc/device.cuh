@@ -249,8 +249,11 @@ inline PartView part_view(const void* table_host, const void* table_dev, int whi
 
 int check_table(const void* table_host, const void* table_dev);
 
-// Workspace of an apply_within call for one value of same_configs (apply.cu).
-int apply_within_workspace_for(const void* table_host, int64_t n_i, int64_t n_j, bool same, uint64_t* bytes);
+// Workspace of an apply_within call for one value of same_configs (apply.cu): the part every call
+// needs, and with the pair scan's scratch behind it where the sizes give it one (calls with less
+// workspace walk the terms instead).
+int apply_within_workspace_for(const void* table_host, int64_t n_i, int64_t n_j, bool same, uint64_t* needed,
+                               uint64_t* with_pairs);
 
 // ---------------------------------------------------------------------------
 // the enumeration kernel: every (configuration, term) pair of one or two
@@ -1176,7 +1179,9 @@ int row_split(int64_t n_rows);
 //            to kTiledMaxTerms terms in groups of a few terms over
 //            kFewWideRows rows or more.
 // QMBX_WALK=pivot, grouped or tiled in the environment forces a kernel
-// (read at every call; pivot falls back to grouped where it cannot serve).
+// (read at every call; pivot falls back to grouped where it cannot serve);
+// QMBX_WALK=scan forces the pair scan (pairs.cuh) where the table and the
+// scratch allow it.
 constexpr int kPivotMeanGroup = 300;
 constexpr int64_t kFewRows = 8192;
 constexpr int64_t kFewWideRows = 65536;

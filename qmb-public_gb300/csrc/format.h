@@ -43,12 +43,27 @@
 // hold every term's four masks narrowed to their high 32 bits in one 16-byte
 // record, which the grouped walks read instead: half the bytes a term, one
 // load, and 32-bit tests.
+//
+// Tables whose changing terms all keep the particle number also index the
+// forward part by transition: the positions a term empties (r1 <= r2) and
+// fills (c1 <= c2), r1 == r2 and c1 == c2 for one of each, packed as
+// r1 | r2 << 8 | c1 << 16 | c2 << 24.  That key is exact (positions are below
+// 256, and 0 cannot occur: a position is not both emptied and filled), so two
+// rows that differ by it are connected by exactly the terms listed under it.
+// Buckets hold two (key, value) entries in 16 bytes, half full at most, the
+// first empty key ending a probe.  A value is the slot of the transition's
+// only term when that term tests no other site; otherwise it is bit 31 plus
+// the start of the transition's run in the list.  A list entry is a slot, with
+// bit 31 on the last one of a run, and what the term asks beyond the
+// transition: -1 nothing, a key position that must be occupied, or -2 for
+// anything else (and for terms whose parity mask is not that of the run's
+// first term).  The list is followed by 32 spare entries.
 #pragma once
 
 #include <stdint.h>
 
 #define QMBX_MAGIC 0x58424D51u  // "QMBX"
-#define QMBX_TABLE_VERSION 7u
+#define QMBX_TABLE_VERSION 8u
 #define QMBX_MAX_WORDS 4
 #define QMBX_ALIGN 256
 
@@ -86,6 +101,10 @@ struct qmbx_table_header {
     int64_t n_live;       // terms that can apply
     qmbx_table_part part[QMBX_PARTS];
     uint64_t total_bytes;
+    uint64_t off_class;      // uint32[n_class_buckets][4]: the transition index of the forward part
+    uint64_t off_class_list; // int32[n_class_list + 32][2]
+    int64_t n_class_buckets; // a power of two, at least 2 (0: no index)
+    int64_t n_class_list;
 };
 
 #ifdef __cplusplus
@@ -104,6 +123,7 @@ static inline int64_t qmbx_group_count(int words) {
 #endif
 
 #ifdef __cplusplus
+static inline QMBX_HD uint32_t qmbx_class_bucket(uint32_t key, int shift) { return (key * 0x9E3779B1u) >> shift; }
 static inline QMBX_HD int64_t qmbx_single_group(int kp) { return 1 + kp; }
 static inline QMBX_HD int64_t qmbx_pair_group(int words, int p, int q) {
     return 1 + 64 * (int64_t)words + (int64_t)q * (q - 1) / 2 + p;

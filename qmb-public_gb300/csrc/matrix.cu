@@ -14,7 +14,7 @@
 // different terms are separate entries.  Rows must be distinct.
 #include <cuda_runtime.h>
 
-#include "device.cuh"
+#include "pairs.cuh"
 
 namespace qmbx {
 namespace {
@@ -97,6 +97,27 @@ struct MatrixPivot : VisitorBase {
         }
         const double2 cf = __ldg(coef + (h.x & 0x7fffffff));
         const int64_t e = (int64_t)atomicAdd(reinterpret_cast<unsigned long long*>(cursor + row), 1ull);
+        col[e] = h.y;
+        val[e] = h.x < 0 ? make_double2(-cf.x, -cf.y) : cf;
+    }
+};
+
+// Pair scan: a hit is an entry in the row its term leads to.
+template <bool FILL>
+struct MatrixPairs {
+    const double2* coef;     // forward part
+    int32_t* count;
+    int64_t* cursor;
+    int32_t* col;
+    double2* val;
+    __device__ __forceinline__ void record(const int4*, int, int) const {}
+    __device__ __forceinline__ void apply(int4 h) const {
+        if (!FILL) {
+            atomicAdd(count + h.z, 1);
+            return;
+        }
+        const double2 cf = __ldg(coef + (h.x & 0x7fffffff));
+        const int64_t e = (int64_t)atomicAdd(reinterpret_cast<unsigned long long*>(cursor + h.z), 1ull);
         col[e] = h.y;
         val[e] = h.x < 0 ? make_double2(-cf.x, -cf.y) : cf;
     }
@@ -248,27 +269,48 @@ MatrixLayout take_matrix(Arena& ws, int64_t n) {
     return L;
 }
 
-// Walk the changing terms of every row (daggered terms, gather direction).
+// The pair scan's scratch behind the first ws.used bytes; false when the sizes
+// give it none or it does not fit.
+template <int W>
+bool take_matrix_pairs(const qmbx_table_header* h, const Arena& ws, int64_t n, PairWork& pairs) {
+    if (!pairs_scratch(h, n, n)) return false;
+    Arena rest = ws;
+    pairs = take_pair_work<W>(rest, n, n, true, h->n_sites);
+    return rest.fits();
+}
+
+// Walk the changing terms of every row (daggered terms, gather direction), or
+// scan the pairs of rows (pairs != NULL).
 template <int W, bool FILL>
 int matrix_walk(const void* table_host, const void* table_dev, const MatrixLayout& L, int64_t n, const int64_t* row_ptr,
-                int32_t* col, double2* val, cudaStream_t s) {
+                int32_t* col, double2* val, PairWork* pairs, cudaStream_t s) {
     PartView adj = part_view(table_host, table_dev, QMBX_PART_ADJ);
     PartView diag = part_view(table_host, table_dev, QMBX_PART_DIAG);
     PartView none = adj;
     none.n = 0;
     const HashView look = L.rows.hash();
     UniqueRows<W> src{L.rows.keys, L.rows.unique};
+    const int* walk_rows = L.rows.count;
+    if (adj.n > 0 && pairs != nullptr) {
+        // the device chooses the scan or the walk below; the other finds no rows
+        int st = build_pairs<W>(L.rows, L.rows, header_of(table_host)->n_sites, *pairs, s);
+        if (st != QMBX_OK || (st = choose_pairs<W>(*pairs, L.rows, s)) != QMBX_OK) return st;
+        walk_rows = pairs->gate + 1;
+        const PartView fwd = part_view(table_host, table_dev, QMBX_PART_FWD);
+        MatrixPairs<FILL> v{fwd.coef, L.count, L.cursor, col, val};
+        if ((st = launch_pair_scan<W>(v, *pairs, table_host, table_dev, pairs->gate, s, kGroupEnumerate)) != QMBX_OK) return st;
+    }
     if (adj.n > 0) {
         const Walk kind = choose_walk(adj, n, true);
         if (kind == Walk::kPivot) {
             MatrixPivot<W, FILL> v{{}, look, adj.coef, L.rows.unique, L.count, L.cursor, col, val};
-            QMBX_KERNEL(kGroupEnumerate, s, pivot_kernel<W><<<pivot_grid(), kThreads, 0, s>>>(v, src, L.rows.count, n, adj));
+            QMBX_KERNEL(kGroupEnumerate, s, pivot_kernel<W><<<pivot_grid(), kThreads, 0, s>>>(v, src, walk_rows, n, adj));
         } else {
             MatrixRows<W, FILL> v{{}, look, adj.coef, L.rows.unique, L.count, L.cursor, col, val};
             if (kind == Walk::kGrouped) {
-                QMBX_KERNEL(kGroupEnumerate, s, grouped_kernel<W><<<grouped_grid(n), kThreads, 0, s>>>(v, src, L.rows.count, n, adj, none));
+                QMBX_KERNEL(kGroupEnumerate, s, grouped_kernel<W><<<grouped_grid(n), kThreads, 0, s>>>(v, src, walk_rows, n, adj, none));
             } else {
-                QMBX_KERNEL(kGroupEnumerate, s, enumerate_kernel<W><<<grid_for(n, kThreads), kThreads, 0, s>>>(v, src, L.rows.count, n, adj, none));
+                QMBX_KERNEL(kGroupEnumerate, s, enumerate_kernel<W><<<grid_for(n, kThreads), kThreads, 0, s>>>(v, src, walk_rows, n, adj, none));
             }
         }
         QMBX_LAUNCH_CHECK("matrix walk");
@@ -296,7 +338,9 @@ int matrix_count(const void* table_host, const void* table_dev, const uint8_t* c
     int st;
     if ((st = build_hashrows<W>(configs, nq, L.rows, s)) != QMBX_OK) return st;
     QMBX_CUDA_TRY(cudaMemsetAsync(L.count, 0, (size_t)n * sizeof(int32_t), s));
-    if ((st = matrix_walk<W, false>(table_host, table_dev, L, n, nullptr, nullptr, nullptr, s)) != QMBX_OK) return st;
+    PairWork pairs{};
+    const bool scan = pairs_wanted(header_of(table_host), n, n) && take_matrix_pairs<W>(header_of(table_host), ws, n, pairs);
+    if ((st = matrix_walk<W, false>(table_host, table_dev, L, n, nullptr, nullptr, nullptr, scan ? &pairs : nullptr, s)) != QMBX_OK) return st;
     QMBX_CUDA_TRY(cudaMemsetAsync(L.total64, 0, sizeof(unsigned long long), s));
     QMBX_KERNEL(kGroupOther, s, plus_one_kernel<<<grid_for(n, kThreads), kThreads, 0, s>>>(L.count, n, L.total64));
     if ((st = exclusive_scan(L.count, L.count, n, L.total, L.scan, s)) != QMBX_OK) return st;
@@ -325,7 +369,9 @@ int matrix_fill(const void* table_host, const void* table_dev, const uint8_t* co
     if ((st = build_hashrows<W>(configs, nq, L.rows, s)) != QMBX_OK) return st;
     QMBX_KERNEL(kGroupOther, s, cursor_kernel<<<grid_for(n, kThreads), kThreads, 0, s>>>(row_ptr, n, L.cursor));
     QMBX_LAUNCH_CHECK("matrix cursors");
-    return matrix_walk<W, true>(table_host, table_dev, L, n, row_ptr, col, val, s);
+    PairWork pairs{};
+    const bool scan = pairs_wanted(header_of(table_host), n, n) && take_matrix_pairs<W>(header_of(table_host), ws, n, pairs);
+    return matrix_walk<W, true>(table_host, table_dev, L, n, row_ptr, col, val, scan ? &pairs : nullptr, s);
 }
 
 int matrix_args(const void* table_host, const void* table_dev, const uint8_t* configs, int64_t n, void* workspace) {
@@ -350,13 +396,20 @@ extern "C" int qmbx_matrix_workspace(const void* table_host, int64_t n, uint64_t
     if (h == nullptr || h->magic != QMBX_MAGIC) return fail(QMBX_ERR_ARGUMENT, "not a compiled qmbx table");
     if (bytes == nullptr) return fail(QMBX_ERR_ARGUMENT, "bytes must not be NULL");
     Arena probe(nullptr, 0);
+    const bool pairs = pairs_scratch(h, n, n);
+#define QMBX_MATRIX_BYTES(W)                                                        \
+    case W:                                                                         \
+        take_matrix<W>(probe, n);                                                   \
+        if (pairs) take_pair_work<W>(probe, n, n, true, h->n_sites);                \
+        break;
     switch (h->n_words) {
-        case 1: take_matrix<1>(probe, n); break;
-        case 2: take_matrix<2>(probe, n); break;
-        case 3: take_matrix<3>(probe, n); break;
-        case 4: take_matrix<4>(probe, n); break;
+        QMBX_MATRIX_BYTES(1)
+        QMBX_MATRIX_BYTES(2)
+        QMBX_MATRIX_BYTES(3)
+        QMBX_MATRIX_BYTES(4)
         default: return fail(QMBX_ERR_ARGUMENT, "unsupported word count");
     }
+#undef QMBX_MATRIX_BYTES
     *bytes = probe.used;
     return QMBX_OK;
 }

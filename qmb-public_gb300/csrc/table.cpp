@@ -43,6 +43,13 @@ struct Compiled {
     uint64_t par[QMBX_MAX_WORDS] = {0, 0, 0, 0};
     int pconst = 0;
     bool diagonal() const { return (flip[0] | flip[1] | flip[2] | flip[3]) == 0; }
+    bool keeps_number() const {
+        int change = 0;
+        for (int q = 0; q < QMBX_MAX_WORDS; ++q) {
+            change += __builtin_popcountll(flip[q] & val[q]) - __builtin_popcountll(flip[q] & ~val[q]);
+        }
+        return change == 0;
+    }
 };
 
 struct Below {
@@ -239,7 +246,99 @@ void group_part(char* blob, qmbx_table_part& p, int words, const std::vector<int
     for (size_t k = 0; k < gid.size(); ++k) dest[k] = cursor[(size_t)gid[k]]++;
 }
 
-qmbx_table_header make_header(int64_t n_terms, int32_t n_qubytes, int32_t particle_cut, int64_t n_off, int64_t n_diag) {
+// Buckets of the transition index over n terms (see format.h): two entries each, at most half of them used.
+int64_t class_buckets(int64_t n) {
+    int64_t b = 2;
+    while (b < n) b <<= 1;
+    return b;
+}
+
+// Key of a changing term that keeps the particle number: the key positions it empties and fills.
+// *asks: what it tests beyond them (format.h).
+uint32_t transition_key(const uint64_t* test, const uint64_t* apply, const qmbx_table_part& p, int words, int64_t slot,
+                        int32_t* asks) {
+    int pos[2][2] = {{-1, -1}, {-1, -1}};  // emptied, filled
+    *asks = -1;
+    for (int q = 0; q < words; ++q) {
+        const uint64_t at = ((uint64_t)q * (uint64_t)p.n + (uint64_t)slot) * 2;
+        const uint64_t mask = test[at], val = test[at + 1], flip = apply[at];
+        for (uint64_t m = mask & ~flip; m != 0; m &= m - 1) {
+            const int bit = __builtin_ctzll(m);
+            *asks = *asks == -1 && (val >> bit & 1) ? 64 * q + bit : -2;
+        }
+        for (int side = 0; side < 2; ++side) {
+            for (uint64_t m = side == 0 ? flip & val : flip & ~val; m != 0; m &= m - 1) {
+                const int kp = 64 * q + __builtin_ctzll(m);
+                pos[side][pos[side][0] < 0 ? 0 : 1] = kp;
+            }
+        }
+    }
+    for (auto& two : pos) {
+        if (two[1] < 0) two[1] = two[0];
+    }
+    return (uint32_t)pos[0][0] | (uint32_t)pos[0][1] << 8 | (uint32_t)pos[1][0] << 16 | (uint32_t)pos[1][1] << 24;
+}
+
+// Fill the transition index of the forward part (its terms are written already).
+void build_classes(char* blob, const qmbx_table_header& h) {
+    if (h.n_class_buckets == 0) return;
+    const qmbx_table_part& p = h.part[QMBX_PART_FWD];
+    const uint64_t* test = reinterpret_cast<const uint64_t*>(blob + p.off_test);
+    const uint64_t* apply = reinterpret_cast<const uint64_t*>(blob + p.off_apply);
+    uint32_t* buckets = reinterpret_cast<uint32_t*>(blob + h.off_class);
+    int32_t* list = reinterpret_cast<int32_t*>(blob + h.off_class_list);
+    const uint64_t mask = (uint64_t)h.n_class_buckets - 1;
+    int shift = 32;
+    for (int64_t b = h.n_class_buckets; b > 1; b >>= 1) --shift;
+    // number the transitions in order of appearance: the entry's value is its number for now
+    std::vector<int32_t> number((size_t)p.n), count;
+    std::vector<uint32_t*> entry;
+    std::vector<int32_t> asks((size_t)p.n);
+    for (int64_t t = 0; t < p.n; ++t) {
+        const uint32_t key = transition_key(test, apply, p, h.n_words, t, &asks[(size_t)t]);
+        uint64_t b = qmbx_class_bucket(key, shift);
+        uint32_t* e = nullptr;
+        while (e == nullptr) {
+            uint32_t* two = buckets + 4 * b;
+            for (int k = 0; k < 2 && e == nullptr; ++k) {
+                if (two[2 * k] == key || two[2 * k] == 0) e = two + 2 * k;
+            }
+            b = (b + 1) & mask;
+        }
+        if (e[0] == 0) {
+            e[0] = key;
+            e[1] = (uint32_t)count.size();
+            count.push_back(0);
+            entry.push_back(e);
+        }
+        number[(size_t)t] = (int32_t)e[1];
+        ++count[e[1]];
+    }
+    std::vector<int32_t> next(count.size());
+    int32_t run = 0;
+    for (size_t k = 0; k < count.size(); ++k) {
+        next[k] = run;
+        entry[k][1] = 0x80000000u | (uint32_t)run;
+        run += count[k];
+    }
+    for (int64_t t = 0; t < p.n; ++t) {
+        const size_t k = (size_t)number[(size_t)t];
+        const bool last = --count[k] == 0;
+        const int32_t start = (int32_t)(entry[k][1] & 0x7fffffffu);
+        if (start == next[k] && last && asks[(size_t)t] == -1) entry[k][1] = (uint32_t)t;
+        int32_t* e = list + 2 * (int64_t)next[k]++;
+        e[0] = (int32_t)((uint32_t)t | (last ? 0x80000000u : 0u));
+        e[1] = asks[(size_t)t];
+        const int64_t head = list[2 * (int64_t)start] & 0x7fffffff;
+        for (int q = 0; q < h.n_words; ++q) {
+            const uint64_t base = (uint64_t)q * (uint64_t)p.n;
+            if (apply[(base + (uint64_t)t) * 2 + 1] != apply[(base + (uint64_t)head) * 2 + 1]) e[1] = -2;
+        }
+    }
+}
+
+qmbx_table_header make_header(int64_t n_terms, int32_t n_qubytes, int32_t particle_cut, int64_t n_off, int64_t n_diag,
+                              bool keeps_number) {
     qmbx_table_header h;
     std::memset(&h, 0, sizeof(h));
     h.magic = QMBX_MAGIC;
@@ -255,14 +354,23 @@ qmbx_table_header make_header(int64_t n_terms, int32_t n_qubytes, int32_t partic
     layout_part(h.part[QMBX_PART_FWD], n_off, h.n_words, narrow, cursor);
     layout_part(h.part[QMBX_PART_ADJ], n_off, h.n_words, narrow, cursor);
     layout_part(h.part[QMBX_PART_DIAG], n_diag, h.n_words, narrow, cursor);
+    if (keeps_number && n_off > 0) {
+        h.n_class_buckets = class_buckets(n_off);
+        h.n_class_list = n_off;
+        h.off_class = cursor;
+        cursor = align_up(cursor + (uint64_t)h.n_class_buckets * 16);
+        h.off_class_list = cursor;
+        cursor = align_up(cursor + (uint64_t)(n_off + 32) * 8);
+    }
     h.total_bytes = cursor;
     return h;
 }
 
 void count_terms(const int16_t* site, const uint8_t* kind, int64_t n_terms, int32_t n_qubytes, int32_t particle_cut,
-                 int64_t& n_off, int64_t& n_diag) {
+                 int64_t& n_off, int64_t& n_diag, bool& keeps_number) {
     Below below(8 * n_qubytes, (n_qubytes + 7) / 8);
     n_off = n_diag = 0;
+    keeps_number = true;
     for (int64_t t = 0; t < n_terms; ++t) {
         Compiled c = compile_term(site + 4 * t, kind + 4 * t, particle_cut == 1, false, below);
         if (!c.live) continue;
@@ -270,6 +378,7 @@ void count_terms(const int16_t* site, const uint8_t* kind, int64_t n_terms, int3
             ++n_diag;
         } else {
             ++n_off;
+            if (!c.keeps_number()) keeps_number = false;
         }
     }
 }
@@ -326,8 +435,9 @@ extern "C" int qmbx_table_bytes(const int16_t* site, const uint8_t* kind, int64_
     int st = validate(site, kind, n_terms, n_qubytes, particle_cut);
     if (st != QMBX_OK) return st;
     int64_t n_off, n_diag;
-    count_terms(site, kind, n_terms, n_qubytes, particle_cut, n_off, n_diag);
-    *bytes = make_header(n_terms, n_qubytes, particle_cut, n_off, n_diag).total_bytes;
+    bool keeps_number;
+    count_terms(site, kind, n_terms, n_qubytes, particle_cut, n_off, n_diag, keeps_number);
+    *bytes = make_header(n_terms, n_qubytes, particle_cut, n_off, n_diag, keeps_number).total_bytes;
     return QMBX_OK;
 }
 
@@ -339,8 +449,9 @@ extern "C" int qmbx_table_build(const int16_t* site, const uint8_t* kind, const 
     if (n_terms > 0 && coef == nullptr) return fail(QMBX_ERR_ARGUMENT, "coef must not be NULL");
     if (blob == nullptr) return fail(QMBX_ERR_ARGUMENT, "blob must not be NULL");
     int64_t n_off, n_diag;
-    count_terms(site, kind, n_terms, n_qubytes, particle_cut, n_off, n_diag);
-    qmbx_table_header h = make_header(n_terms, n_qubytes, particle_cut, n_off, n_diag);
+    bool keeps_number;
+    count_terms(site, kind, n_terms, n_qubytes, particle_cut, n_off, n_diag, keeps_number);
+    qmbx_table_header h = make_header(n_terms, n_qubytes, particle_cut, n_off, n_diag, keeps_number);
     if (blob_bytes < h.total_bytes) {
         return fail(QMBX_ERR_ARGUMENT, "table blob holds %llu bytes, needs %llu", (unsigned long long)blob_bytes,
                     (unsigned long long)h.total_bytes);
@@ -379,6 +490,7 @@ extern "C" int qmbx_table_build(const int16_t* site, const uint8_t* kind, const 
             ++k_off;
         }
     }
+    build_classes(out, h);
     std::memcpy(out, &h, sizeof(h));
     return QMBX_OK;
 }
