@@ -1045,7 +1045,10 @@ int apply_impl(const ApplyArgs& a, Arena& ws, cudaStream_t s) {
     }
     // the device chooses one of the two; the other finds no rows
     if (scan && (st = pair_apply<W>(a, in_set, out_set, pairs, val, res, pairs.gate, s)) != QMBX_OK) return st;
-    if ((st = walk_apply<W>(a, in_set, out_set, val, res, scan ? pairs.gate + 1 : nullptr, s)) != QMBX_OK) return st;
+    if ((st = walk_apply<W>(a, in_set, out_set, val, res, scan ? pairs.gate + 1 : nullptr, s,
+                            scan ? kGroupOther : kGroupEnumerate, scan ? kGroupOther : kGroupDiagonal)) != QMBX_OK) {
+        return st;
+    }
     QMBX_KERNEL(kGroupOther, s, apply_finalize_kernel<<<grid_for(n_out, kThreads), kThreads, 0, s>>>(res, out_set.first, n_out, a.adjoint ? 1 : 0, a.out64, a.out32));
     QMBX_LAUNCH_CHECK("apply_finalize_kernel");
     return QMBX_OK;

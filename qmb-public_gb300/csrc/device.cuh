@@ -214,6 +214,7 @@ struct PartView {
     const float4* coef32;
     const int32_t* orig;
     const float* norm;
+    const float* bound;        // largest norm from a term to the end of its group (NULL in the adjoint part)
     const int2* groups;        // [start, end) of every pivot group
     const uint64_t* single_ne; // [W]
     const uint64_t* pair_ne;   // [64W][W]
@@ -236,6 +237,7 @@ inline PartView part_view(const void* table_host, const void* table_dev, int whi
     v.coef32 = reinterpret_cast<const float4*>(base + p.off_coef32);
     v.orig = reinterpret_cast<const int32_t*>(base + p.off_orig);
     v.norm = reinterpret_cast<const float*>(base + p.off_norm);
+    v.bound = h->off_bound[which] != 0 ? reinterpret_cast<const float*>(base + h->off_bound[which]) : nullptr;
     v.groups = reinterpret_cast<const int2*>(base + p.off_groups);
     v.single_ne = reinterpret_cast<const uint64_t*>(base + p.off_single_ne);
     v.pair_ne = reinterpret_cast<const uint64_t*>(base + p.off_pair_ne);

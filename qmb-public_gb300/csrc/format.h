@@ -105,6 +105,8 @@ struct qmbx_table_header {
     uint64_t off_class_list; // int32[n_class_list + 32][2]
     int64_t n_class_buckets; // a power of two, at least 2 (0: no index)
     int64_t n_class_list;
+    uint64_t off_bound[QMBX_PARTS]; // float[n] of the forward and the diagonal part: the largest norm from a term to
+                                    // the end of its pivot group (0: none)
 };
 
 #ifdef __cplusplus

@@ -301,16 +301,17 @@ int matrix_walk(const void* table_host, const void* table_dev, const MatrixLayou
         if ((st = launch_pair_scan<W>(v, *pairs, table_host, table_dev, pairs->gate, s, kGroupEnumerate)) != QMBX_OK) return st;
     }
     if (adj.n > 0) {
+        const int group = pairs != nullptr ? kGroupOther : kGroupEnumerate;
         const Walk kind = choose_walk(adj, n, true);
         if (kind == Walk::kPivot) {
             MatrixPivot<W, FILL> v{{}, look, adj.coef, L.rows.unique, L.count, L.cursor, col, val};
-            QMBX_KERNEL(kGroupEnumerate, s, pivot_kernel<W><<<pivot_grid(), kThreads, 0, s>>>(v, src, walk_rows, n, adj));
+            QMBX_KERNEL(group, s, pivot_kernel<W><<<pivot_grid(), kThreads, 0, s>>>(v, src, walk_rows, n, adj));
         } else {
             MatrixRows<W, FILL> v{{}, look, adj.coef, L.rows.unique, L.count, L.cursor, col, val};
             if (kind == Walk::kGrouped) {
-                QMBX_KERNEL(kGroupEnumerate, s, grouped_kernel<W><<<grouped_grid(n), kThreads, 0, s>>>(v, src, walk_rows, n, adj, none));
+                QMBX_KERNEL(group, s, grouped_kernel<W><<<grouped_grid(n), kThreads, 0, s>>>(v, src, walk_rows, n, adj, none));
             } else {
-                QMBX_KERNEL(kGroupEnumerate, s, enumerate_kernel<W><<<grid_for(n, kThreads), kThreads, 0, s>>>(v, src, walk_rows, n, adj, none));
+                QMBX_KERNEL(group, s, enumerate_kernel<W><<<grid_for(n, kThreads), kThreads, 0, s>>>(v, src, walk_rows, n, adj, none));
             }
         }
         QMBX_LAUNCH_CHECK("matrix walk");

@@ -640,7 +640,7 @@ int launch_pair_scan(const H& h, const PairWork& p, const void* table_host, cons
     QMBX_KERNEL(group, s, pair_scan_kernel<W, H><<<grid, kThreads, shared, s>>>(
         context, b.planes, a.list, a.count, b.count, sites, pair_chunk(a.n, b.n, pair_tile<W>()), p.next, p.pairs, p.cap,
         static_cast<PairQueue*>(p.overflow), gate));
-    QMBX_KERNEL(group, s, pair_lookup_kernel<W, H><<<2 * pivot_grid(), kThreads, 0, s>>>(context, p.pairs, p.next + 1, p.cap));
+    QMBX_KERNEL(kGroupOther, s, pair_lookup_kernel<W, H><<<2 * pivot_grid(), kThreads, 0, s>>>(context, p.pairs, p.next + 1, p.cap));
     QMBX_LAUNCH_CHECK("pair scan");
     return QMBX_OK;
 }

@@ -5,8 +5,9 @@
 
 namespace qmbx {
 
-// kGroupEnumerate is the main term walk; kGroupDiagonal the separate
-// passes over diagonal terms that follow it; kGroupSort the radix sorts
+// kGroupEnumerate is the main term walk, or the pair scan that stands in for
+// it (its lookups and the walk launched beside it, one of which finds no rows,
+// count under kGroupOther); kGroupDiagonal the separate passes over diagonal terms that follow it; kGroupSort the radix sorts
 // (histogram, scan and scatter passes); kGroupSpmv the products with a
 // materialised matrix and the adjoint products formed from a hit log (the
 // replay, and the adjoint walk that stands in for an incomplete record,

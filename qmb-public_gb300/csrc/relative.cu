@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdlib>
 
 #include "device.cuh"
 
@@ -183,6 +184,210 @@ struct RelativeVisitor : VisitorBase {
     __device__ __forceinline__ void reduce(Acc&) const {}
     __device__ __forceinline__ void finish(Acc&, int64_t, const Key<W>&) const {}
 };
+
+// The same passes over parts whose groups hold many terms (PartView::wide),
+// bounded by the terms' norms.  A warp takes a row (or one of `split` shares
+// of it); the lanes take its pivot groups, and a group's terms are read, eight
+// lanes a group, only while the bound of the rest of the group (the norms
+// themselves for tables sorted by |coef|) can still reach the threshold.
+// Selections take few records of a row (121k of 5.7e7 for the top 50,000 of
+// 20,000 rows under 55,371 terms), so most groups end at their first bound:
+// the pass is a few instructions per group instead of a test per term, and is
+// bound by the latency of its reads.  On GB300,
+// emission passes against the walks: those rows 428 -> 70 us, the top
+// 1,000,000 of 8,192 rows under 3.1M terms 4.58 -> 0.50 ms (pivot-major walk
+// and diagonal pass), the top 200,000 of 4,099 rows under 669,579 terms 1.42
+// -> 0.21 ms; their histograms 124 -> 23, 473 -> 42 and 139 -> 19 us.
+//
+// The histogram reads the first `depth` steps of 32 terms of every group and
+// counts what applies: the records near the threshold are the first of their
+// groups.  Counts that miss deeper records only lower the threshold.
+//
+// Diagonal terms give the row itself: one exclusion lookup per row, and a
+// group a lane (their groups hold a term or two).
+template <int W, bool EMIT>
+__global__ void __launch_bounds__(kThreads) relative_bounded_kernel(RelativeArgs a, const uint64_t* __restrict__ keys,
+                                                                    int64_t n, int split, int depth) {
+    __shared__ int s_hist[EMIT ? 1 : kBuckets];
+    __shared__ uint8_t s_pos[kWarpsPerBlock][64 * W];
+    if (!EMIT) {
+        for (int k = threadIdx.x; k < kBuckets; k += kThreads) s_hist[k] = 0;
+        __syncthreads();
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    uint8_t* pos = s_pos[warp];
+    const int from = EMIT ? a.ctl->emit_from : 0;
+    // records whose estimate reaches the threshold, one a lane
+    auto take = [&](bool on, const Key<W>& img, int part, int parity, int64_t slot, int64_t row) {
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (m == 0) return;
+        unsigned long long at = 0;
+        if (lane == __ffs(m) - 1) at = atomicAdd(&a.ctl->n_emit, (unsigned long long)__popc(m));
+        at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1) + __popc(m & lt);
+        if (!on) return;
+        if ((int64_t)at >= a.cap_emit) {
+            a.ctl->overflow = 1;
+            return;
+        }
+        a.emit_rank[2 * at + 0] = (uint64_t)slot | ((uint64_t)part << 62) | ((uint64_t)parity << 63);
+        a.emit_rank[2 * at + 1] = (uint64_t)row;
+#pragma unroll
+        for (int q = 0; q < W; ++q) a.emit_keys[at * W + q] = img.w[q];
+    };
+    const int64_t items = n * split, stride = (int64_t)gridDim.x * kWarpsPerBlock;
+    for (int64_t u = (int64_t)blockIdx.x * kWarpsPerBlock + warp; u < items; u += stride) {
+        const int64_t row = u / split;
+        const int share = (int)(u - row * split);
+        const Key<W> c = load_key<W>(keys, row);
+        const double2 p = __ldg(a.psi + row);
+        const float px = (float)p.x, py = (float)p.y;
+        const float m = __fadd_rn(__fmul_rn(px, px), __fmul_rn(py, py));
+        // occupied key positions, ascending
+        int occ = 0;
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2 * W; ++h) {
+            const uint32_t bits = (uint32_t)(c.w[h >> 1] >> (32 * (h & 1)));
+            if (bits >> lane & 1u) pos[occ + __popc(bits & lt)] = (uint8_t)(32 * h + lane);
+            occ += __popc(bits);
+        }
+        __syncwarp();
+        // a term whose bound is not below the threshold (NaN: not known to be)
+        auto reaches = [&](float bound) {
+            const float e = __fmul_rn(bound, m);
+            return e != e || weight_bucket(e) >= from;
+        };
+        const bool row_excluded = hash_find<W>(a.excl, c) >= 0;
+        for (int part = 0; part < (row_excluded ? 1 : 2); ++part) {
+            const PartView& pv = part == 0 ? a.off : a.diag;
+            if (pv.n == 0) continue;
+            // i < 0: group 0 and the single groups; else the pairs (position i, a later one)
+            for (int i = share - 1; i < occ; i += split) {
+                const int count = i < 0 ? 1 + occ : occ - i - 1;
+                for (int k0 = 0; k0 < count; k0 += 32) {
+                    const int k = k0 + lane;
+                    int2 se = make_int2(0, 0);
+                    if (k < count) {
+                        const int64_t g = i >= 0 ? qmbx_pair_group(W, pos[i], pos[i + 1 + k])
+                                                 : (k == 0 ? 0 : qmbx_single_group(pos[k - 1]));
+                        se = __ldg(pv.groups + g);
+                    }
+                    bool alive = se.x < se.y;
+                    if (EMIT && alive) alive = reaches(__ldg(pv.bound + se.x));
+                    if (part == 1) {
+                        // a group a lane
+                        for (int t = se.x; __any_sync(0xffffffffu, alive && t < se.y); ++t) {
+                            bool on = false;
+                            int par = 0;
+                            if (alive && t < se.y) {
+                                TermRec<W> rec;
+                                load_test<W>(rec, pv, t);
+                                const int b = weight_bucket(__fmul_rn(__ldg(pv.norm + t), m));
+                                on = rec.applies(c) && b >= from;
+                                if (on) {
+                                    load_apply<W>(rec, pv, t);
+                                    Key<W> img;
+                                    par = rec.image(c, img);
+                                    if (!EMIT) atomicAdd(&s_hist[b], 1);
+                                }
+                            }
+                            if (EMIT) take(on, c, 1, par, t, row);
+                        }
+                        continue;
+                    }
+                    // emission: four groups at a time, eight lanes each (a group gives a record or
+                    // two); histogram: a group at a time
+                    constexpr int L = EMIT ? 8 : 32;
+                    const int sub = lane / L;
+                    for (unsigned todo = __ballot_sync(0xffffffffu, alive); todo != 0;) {
+                        int src = -1;
+#pragma unroll
+                        for (int k = 0; k < 32 / L; ++k) {
+                            const int next = __ffs(todo) - 1;
+                            if (sub == k) src = next;
+                            todo &= todo - 1;  // (0 stays 0)
+                        }
+                        const int start = __shfl_sync(0xffffffffu, se.x, src < 0 ? 0 : src);
+                        const int end = __shfl_sync(0xffffffffu, se.y, src < 0 ? 0 : src);
+                        const int stop = src < 0 ? start : (!EMIT && end - start > 32 * depth ? start + 32 * depth : end);
+                        int t = start + lane % L;
+                        bool open = src >= 0;
+                        while (__any_sync(0xffffffffu, open)) {
+                            // everything a term needs is read at once: one trip to L2 before its lookup
+                            bool in = open && t < stop;
+                            bool on = false;
+                            int par = 0;
+                            Key<W> img{};
+                            if (in) {
+                                TermRec<W> rec;
+                                bool narrow = false;
+                                if constexpr (W == 1) narrow = pv.narrow != nullptr;
+                                if (narrow) {
+                                    load_narrow<W>(rec, pv, t);
+                                } else {
+                                    load_test<W>(rec, pv, t);
+                                    if (EMIT) load_apply<W>(rec, pv, t);
+                                }
+                                const int b = weight_bucket(__fmul_rn(__ldg(pv.norm + t), m));
+                                if (EMIT) in = reaches(__ldg(pv.bound + t));
+                                on = in && b >= from && rec.applies(c);
+                                if (!EMIT && on) atomicAdd(&s_hist[b], 1);
+                                if (EMIT && on) {
+                                    par = rec.image(c, img);
+                                    on = hash_find<W>(a.excl, img) < 0;
+                                }
+                            }
+                            if (EMIT) take(on, img, 0, par, t, row);
+                            // the bounds fall: a group ends at the first lane that stops
+                            const unsigned ins = __ballot_sync(0xffffffffu, in);
+                            constexpr unsigned kAll = 0xffffffffu >> (32 - L);
+                            open = (ins >> (L * sub) & kAll) == kAll;
+                            t += L;
+                        }
+                    }
+                }
+            }
+        }
+    }
+    if (!EMIT) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < kBuckets; k += kThreads) {
+            const int v = s_hist[k];
+            if (v) atomicAdd(a.hist + k, (unsigned long long)v);
+        }
+    }
+}
+
+// Whether the bounded passes serve the part (QMBX_WALK forces the walks).
+bool relative_bounded(const PartView& off) {
+    const char* e = getenv("QMBX_WALK");
+    return off.n >= kGroupedMinTerms && off.wide && off.bound != nullptr &&
+           !(e != nullptr && (e[0] == 't' || e[0] == 'g' || e[0] == 'p'));
+}
+
+// Steps of 32 terms the bounded histogram reads of a group: rows reach at
+// least a dozen or so groups, so this is several times the records a group
+// gives to a selection of k.
+int histogram_depth(int64_t k, int64_t n_i) {
+    const int64_t steps = 1 + 2 * k / (n_i > 0 ? n_i : 1) / 128;
+    return (int)(steps < (1 << 20) ? steps : 1 << 20);
+}
+
+// Shares a row is split in for the emission: rows differ widely in the records
+// they give (|psi|^2), so that rows of many are cut into shares of about 32.
+int emission_split(int64_t k, int64_t n_i) {
+    const int64_t shares = 2 * k / (n_i > 0 ? n_i : 1) / 32;
+    const int64_t fill = row_split(n_i);
+    return (int)(shares > 16 ? 16 : shares > fill ? shares : fill);
+}
+
+template <int W, bool EMIT>
+int launch_bounded(const RelativeArgs& r, const uint64_t* keys, int64_t n, int split, int depth, cudaStream_t s) {
+    QMBX_KERNEL(kGroupEnumerate, s, relative_bounded_kernel<W, EMIT><<<grouped_grid(n * split), kThreads, 0, s>>>(r, keys, n, split, depth));
+    QMBX_LAUNCH_CHECK(EMIT ? "find_relative emission pass" : "find_relative histogram pass");
+    return QMBX_OK;
+}
 
 template <int W, bool EMIT>
 int launch_relative(const RelativeArgs& r, const uint64_t* keys_i, int64_t n_i, cudaStream_t s) {
@@ -585,6 +790,7 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
     // pass 1: bucket counts over every row, or every kSampleStride-th row of
     // large inputs; the threshold is chosen on the device (no host round trip)
     const bool sampled = a.n_i >= kSampleMinRows;
+    const bool bounded = relative_bounded(r.off);
     if (sampled) {
         const int64_t n_s = (a.n_i + kSampleStride - 1) / kSampleStride;
         QMBX_KERNEL(kGroupOther, s, sample_rows_kernel<W><<<grid_for(n_s, kThreads), kThreads, 0, s>>>(L.keys_i, r.psi, n_s, L.keys_s, L.psi_s));
@@ -593,14 +799,18 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
         rs.psi = L.psi_s;
         rs.n_i = n_s;
         rs.hist_exact = 0;  // an estimate: every record counted, no exclusion lookups
-        if ((st = launch_relative<W, false>(rs, L.keys_s, n_s, s)) != QMBX_OK) return st;
+        st = bounded ? launch_bounded<W, false>(rs, L.keys_s, n_s, row_split(n_s), histogram_depth(k, a.n_i), s)
+                     : launch_relative<W, false>(rs, L.keys_s, n_s, s);
+        if (st != QMBX_OK) return st;
         ++g_find_stats.walks;
         // aim at about twice k records above the chosen bucket, one more bucket of slack
         QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, (double)a.n_i / (double)n_s, 2.0 * (double)k, L.ctl));
     } else {
         RelativeArgs r1 = r;
         r1.hist_exact = 0;
-        if ((st = launch_relative<W, false>(r1, L.keys_i, a.n_i, s)) != QMBX_OK) return st;
+        st = bounded ? launch_bounded<W, false>(r1, L.keys_i, a.n_i, row_split(a.n_i), histogram_depth(k, a.n_i), s)
+                     : launch_relative<W, false>(r1, L.keys_i, a.n_i, s);
+        if (st != QMBX_OK) return st;
         ++g_find_stats.walks;
         QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, 1.0, (double)k, L.ctl));
     }
@@ -613,7 +823,8 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
     // pass (never seen on the benchmark shapes; the tests drive it).
     FindCtl ctl{};
     for (int attempt = 0;; ++attempt) {
-        if ((st = launch_relative<W, true>(r, L.keys_i, a.n_i, s)) != QMBX_OK) return st;
+        st = bounded ? launch_bounded<W, true>(r, L.keys_i, a.n_i, emission_split(k, a.n_i), 0, s) : launch_relative<W, true>(r, L.keys_i, a.n_i, s);
+        if (st != QMBX_OK) return st;
         ++g_find_stats.walks;
         QMBX_CUDA_TRY(cudaMemcpyAsync(&ctl, L.ctl, sizeof(FindCtl), cudaMemcpyDeviceToHost, s));
         QMBX_CUDA_TRY(cudaStreamSynchronize(s));

@@ -337,6 +337,23 @@ void build_classes(char* blob, const qmbx_table_header& h) {
     }
 }
 
+// Bounds of a part's norms (format.h); the input table is usually sorted by
+// |coef|, and the bounds are then the norms themselves.
+void build_bounds(char* blob, const qmbx_table_header& h, int which) {
+    const qmbx_table_part& p = h.part[which];
+    const int32_t* groups = reinterpret_cast<const int32_t*>(blob + p.off_groups);
+    const float* norm = reinterpret_cast<const float*>(blob + p.off_norm);
+    float* bound = reinterpret_cast<float*>(blob + h.off_bound[which]);
+    for (int64_t g = 0; g < p.n_groups; ++g) {
+        float most = 0.f;
+        for (int64_t t = groups[2 * g + 1]; t-- > groups[2 * g];) {
+            // a NaN norm stays in the bound: nothing is cut before it
+            most = norm[t] == norm[t] && !(norm[t] > most) ? most : norm[t];
+            bound[t] = most;
+        }
+    }
+}
+
 qmbx_table_header make_header(int64_t n_terms, int32_t n_qubytes, int32_t particle_cut, int64_t n_off, int64_t n_diag,
                               bool keeps_number) {
     qmbx_table_header h;
@@ -354,6 +371,10 @@ qmbx_table_header make_header(int64_t n_terms, int32_t n_qubytes, int32_t partic
     layout_part(h.part[QMBX_PART_FWD], n_off, h.n_words, narrow, cursor);
     layout_part(h.part[QMBX_PART_ADJ], n_off, h.n_words, narrow, cursor);
     layout_part(h.part[QMBX_PART_DIAG], n_diag, h.n_words, narrow, cursor);
+    for (int which : {QMBX_PART_FWD, QMBX_PART_DIAG}) {
+        h.off_bound[which] = cursor;
+        cursor = align_up(cursor + (uint64_t)h.part[which].n * 4);
+    }
     if (keeps_number && n_off > 0) {
         h.n_class_buckets = class_buckets(n_off);
         h.n_class_list = n_off;
@@ -491,6 +512,8 @@ extern "C" int qmbx_table_build(const int16_t* site, const uint8_t* kind, const 
         }
     }
     build_classes(out, h);
+    build_bounds(out, h, QMBX_PART_FWD);
+    build_bounds(out, h, QMBX_PART_DIAG);
     std::memcpy(out, &h, sizeof(h));
     return QMBX_OK;
 }
