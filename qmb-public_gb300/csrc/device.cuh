@@ -1216,60 +1216,6 @@ __device__ __forceinline__ double warp_sum(double x) {
 template <int W>
 int pack_rows(const uint8_t* rows, int64_t n, int n_qubytes, uint64_t* keys, cudaStream_t s);
 
-// keys -> rows; rows beyond *n_rows (when n_rows != NULL) are left untouched
-template <int W>
-int unpack_rows(const uint64_t* keys, const int* n_rows, int64_t n_max, int n_qubytes, uint8_t* rows,
-                cudaStream_t s);
-
-// Scratch of one radix sort of up to n keys.
-struct SortScratch {
-    uint64_t* keys;
-    int32_t* vals;
-    int32_t* counts;
-    int32_t* scan;
-};
-
-template <int W>
-SortScratch take_sort_scratch(Arena& ws, int64_t n);
-
-// Stable LSD radix sort of (key, value) pairs in lexicographic key order over
-// the first n_bytes row bytes (n_bytes passes of 8 bits).  vals_in == NULL
-// sorts the identity permutation.  keys_out/vals_out must not alias the inputs.
-template <int W>
-int sort_pairs(const uint64_t* keys_in, const int32_t* vals_in, uint64_t* keys_out, int32_t* vals_out, int64_t n,
-               int n_bytes, const SortScratch& sc, cudaStream_t s);
-
-// A sorted, de-duplicated row set (all buffers carved by take_rowset).
-struct RowSet {
-    uint64_t* packed;       // n x W: keys in input row order
-    uint64_t* sorted_keys;  // n x W, sorted (with repeats)
-    int32_t* perm;          // n: original row of each sorted position
-    uint64_t* keys;         // n x W: unique keys (first *count valid)
-    int32_t* first;         // n: original row of the first occurrence of each unique key
-    int32_t* start;         // n + 1: sorted position where each unique key's run starts
-    int* count;             // device int: number of unique keys
-    int32_t* head;
-    int32_t* pos;
-    uint64_t* slots;        // hash set over the unique keys
-    uint64_t slot_mask;
-    SortScratch sort;
-    int64_t n;
-    HashView hash() const {
-        return HashView{reinterpret_cast<const uint32_t*>(slots), keys, slot_mask, hash_shift(slot_mask + 1), nullptr, 0};
-    }
-};
-
-template <int W>
-RowSet take_rowset(Arena& ws, int64_t n);
-
-template <int W>
-int build_rowset(const uint8_t* rows, int n_qubytes, RowSet& out, cudaStream_t s);
-
-// Sort out.n keys by their first n_bytes row bytes and keep the distinct ones
-// (out.keys[0 .. *out.count)); builds no hash set.
-template <int W>
-int sort_unique_keys(const uint64_t* keys, int n_bytes, RowSet& out, cudaStream_t s);
-
 // A de-duplicated row set without sorting: every row's key is inserted in an
 // open-addressing hash set whose entries name the first (lowest) row holding
 // that key.  first[i] is that row for every row i; unique[0 .. *count) lists
@@ -1297,6 +1243,11 @@ HashRows take_hashrows(Arena& ws, int64_t n);
 
 template <int W>
 int build_hashrows(const uint8_t* rows, int n_qubytes, HashRows& out, cudaStream_t s);
+
+// The same without first rows and the list of distinct ones, for sets that
+// are only looked up (hash()).
+template <int W>
+int build_hashset(const uint8_t* rows, int n_qubytes, HashRows& out, cudaStream_t s);
 
 // Rows of a HashRows set visited by the enumeration kernels: walk index u
 // is the u-th unique row.

@@ -23,6 +23,7 @@
 //                  compacted, and their rows are sorted and de-duplicated.
 //   single_relative  one thread per row keeps the best Efraimidis-Spirakis
 //                  key of its candidates in registers.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -65,20 +66,15 @@ __device__ __forceinline__ double exact_weight(double2 cf, double2 p, int parity
 }
 
 // Device-side state of one find_relative call: the selection threshold of
-// the emission pass, its record count, and the radix select of the kept
-// records.  Read by the host once, after the emission pass.
+// the emission pass, its record count, and the selected and returned rows.
+// Read by the host once, at the end.
 struct FindCtl {
     unsigned long long n_emit;     // records emitted (atomic counter of the emission pass)
     unsigned long long n_zero;     // emitted records of zero exact weight
-    unsigned long long sel_p0;     // radix select: key prefix chosen so far (128 bits, MSB aligned)
-    unsigned long long sel_p1;
-    unsigned long long n_sel;      // records accepted by the compaction
-    long long sel_need;            // records still to accept below the prefix
+    unsigned long long n_sel;      // records selected
+    unsigned long long n_unique;   // distinct rows returned
     int overflow;
     int emit_from;                 // lowest bucket the emission pass keeps
-    int sel_bits;                  // key bits fixed so far
-    int sel_done;
-    int pad;
 };
 
 // The histogram (EMIT = false) and emission (EMIT = true) passes as
@@ -423,29 +419,6 @@ int launch_relative(const RelativeArgs& r, const uint64_t* keys_i, int64_t n_i, 
     return QMBX_OK;
 }
 
-// Replace every emitted record's (slot | part << 62 | parity << 63, row) by
-// its rank key (~weight bits, ~order << order_shift): the reference's exact
-// FP64 weight and its visiting order (term index, then row).  Orders are
-// below 2^(64 - order_shift), so the key's leading 8 + (64 - order_shift) / 8
-// bytes decide it and the radix sort skips the rest.  Records of zero weight
-// (the reference drops them) get the all-ones weight key, which sorts after
-// every other record, and are counted in *n_zero.
-__global__ void rank_records_kernel(uint64_t* __restrict__ rank, int64_t n, PartView off, PartView diag,
-                                    const double2* __restrict__ psi, int64_t n_i, int order_shift,
-                                    unsigned long long* __restrict__ n_zero) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint64_t info = rank[2 * i], row = rank[2 * i + 1];
-    const int64_t slot = (int64_t)(info & ((1ull << 62) - 1));
-    const bool in_diag = (info >> 62) & 1;
-    const int parity = (int)(info >> 63);
-    const double w = exact_weight(__ldg((in_diag ? diag.coef : off.coef) + slot), __ldg(psi + row), parity);
-    const uint64_t order = (uint64_t)__ldg((in_diag ? diag.orig : off.orig) + slot) * (uint64_t)n_i + row;
-    if (w == 0.0) atomicAdd(n_zero, 1ull);
-    rank[2 * i] = w == 0.0 ? ~0ull : ~(uint64_t)__double_as_longlong(w);
-    rank[2 * i + 1] = (~order) << order_shift;
-}
-
 // Inputs of 4,096 rows or more count records on every kSampleStride-th row
 // in pass 1.
 constexpr int64_t kSampleStride = 16;
@@ -531,17 +504,22 @@ __global__ void __launch_bounds__(kChooseThreads) choose_emit_kernel(unsigned lo
 }
 
 // ---------------------------------------------------------------------------
-// radix select of the count_selected smallest rank keys (128 bits: ~weight,
-// then ~visiting order; unique because visiting orders are).  Level by
-// level, a histogram of the next 12 key bits of the records that share the
-// prefix chosen so far, and one warp that picks the digit where the
-// remaining count is reached; it stops as soon as the records of that digit
-// are exactly the ones still needed.  Accepted records are those whose key
-// prefix is at most the final prefix.
+// The tail of a call in two cooperative launches (one block of 1,024 threads
+// per SM, the blocks in step through grid barriers) that take their counts
+// from the device: the selection of the count_selected heaviest records, and
+// the sort, de-duplication and unpacking of their rows.  As some 45 launches
+// with two host round trips between them the tail was bound by launching them
+// (the top 50,000 of 121k records: 156 us of kernels in 0.4 ms).
 // ---------------------------------------------------------------------------
 
-constexpr int kSelectBits = 12;
+namespace cg = cooperative_groups;
+
+constexpr int kTailThreads = 1024;
+constexpr int kTailWarps = kTailThreads / 32;
+
+constexpr int kSelectBits = 11;
 constexpr int kSelectBins = 1 << kSelectBits;
+static_assert(3 * kSelectBins * sizeof(unsigned int) <= kBuckets * sizeof(unsigned long long), "the bins reuse the histogram");
 
 // `cnt` key bits starting `from` bits below the most significant bit of (k0, k1).
 __device__ __forceinline__ uint32_t key_bits(uint64_t k0, uint64_t k1, int from, int cnt) {
@@ -564,71 +542,92 @@ __device__ __forceinline__ int prefix_cmp(uint64_t k0, uint64_t k1, uint64_t p0,
     return a < b ? -1 : (a > b ? 1 : 0);
 }
 
-__global__ void select_init_kernel(FindCtl* __restrict__ ctl, long long k, long long n,
-                                   unsigned int* __restrict__ bins) {
-    const long long valid = n - (long long)ctl->n_zero;
-    const long long need = k < valid ? k : valid;
-    for (int b = threadIdx.x; b < kSelectBins; b += blockDim.x) bins[b] = 0;
-    if (threadIdx.x == 0) {
-        ctl->sel_p0 = ctl->sel_p1 = 0;
-        ctl->sel_bits = 0;
-        ctl->sel_need = need;
-        ctl->sel_done = need <= 0 ? 1 : 0;
-        ctl->n_sel = 0;
-    }
-}
-
-__global__ void select_hist_kernel(const uint64_t* __restrict__ rank, int64_t n, int key_bits_total,
-                                   const FindCtl* __restrict__ ctl, unsigned int* __restrict__ bins) {
-    __shared__ unsigned int sh[kSelectBins];
-    if (ctl->sel_done) return;
-    const uint64_t p0 = ctl->sel_p0, p1 = ctl->sel_p1;
-    const int fixed = ctl->sel_bits;
-    const int cnt = key_bits_total - fixed < kSelectBits ? key_bits_total - fixed : kSelectBits;
-    for (int b = threadIdx.x; b < kSelectBins; b += blockDim.x) sh[b] = 0;
-    __syncthreads();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t k0 = rank[2 * i], k1 = rank[2 * i + 1];
-        if (prefix_cmp(k0, k1, p0, p1, fixed) != 0) continue;
-        atomicAdd(&sh[key_bits(k0, k1, fixed, cnt)], 1u);
-    }
-    __syncthreads();
-    for (int b = threadIdx.x; b < kSelectBins; b += blockDim.x) {
-        const unsigned int v = sh[b];
-        if (v) atomicAdd(bins + b, v);
-    }
-}
-
-// One warp: the digit where the remaining count is reached; clears the bins.
-__global__ void __launch_bounds__(kChooseThreads) select_choose_kernel(int key_bits_total, FindCtl* __restrict__ ctl,
-                                                                       unsigned int* __restrict__ bins) {
-    __shared__ long long s_warp[32];
-    if (ctl->sel_done) return;
-    const int t = threadIdx.x;
-    const int fixed = ctl->sel_bits;
-    const int cnt = key_bits_total - fixed < kSelectBits ? key_bits_total - fixed : kSelectBits;
-    const int nbins = 1 << cnt;
-    const int per = (nbins + kChooseThreads - 1) / kChooseThreads;
-    const int lo = t * per;
-    long long mine = 0;
-    for (int b = lo; b < lo + per && b < nbins; ++b) mine += bins[b];
-    const long long run = block_inclusive_scan(mine, s_warp);
-    const long long need = ctl->sel_need;
-    // the records under the prefix hold at least `need`: exactly one thread's bins reach it
-    if (run >= need && run - mine < need) {
-        long long acc = run - mine;
-        int digit = lo + per - 1 < nbins - 1 ? lo + per - 1 : nbins - 1;
-        for (int b = lo; b < lo + per && b < nbins; ++b) {
-            if (acc + (long long)bins[b] >= need) {
-                digit = b;
-                break;
-            }
-            acc += bins[b];
+// The k heaviest of the emitted records: their row keys to `out`, in no
+// particular order, their number to ctl->n_sel.
+//
+// First every record's (slot | part << 62 | parity << 63, row) becomes its
+// rank key (~weight bits, ~order << order_shift): the reference's exact FP64
+// weight and its visiting order (term index, then row).  Orders are below
+// 2^(64 - order_shift), so the key's leading key_bits_total bits decide it.
+// Records of zero weight (the reference drops them) get the all-ones weight
+// key, which sorts after every other record, and are never taken.
+//
+// Then a radix select finds the k-th smallest rank key (keys are unique
+// because visiting orders are): level by level a histogram of the next 11 key
+// bits of the records that share the prefix chosen so far, whose digit every
+// block picks for itself, so that a level is one grid barrier.  It stops as
+// soon as the records of a digit are exactly the ones still needed.  Bins of
+// three levels in turn: those of the next level are cleared while a level is
+// counted, two barriers after they were last read.
+//
+// Nothing is done when the emission has to be repeated (more records than
+// places, or fewer than k above a threshold): the host sees the same counts.
+template <int W>
+__global__ void __launch_bounds__(kTailThreads)
+    find_select_kernel(uint64_t* __restrict__ rank, const uint64_t* __restrict__ keys, int64_t cap, PartView off,
+                       PartView diag, const double2* __restrict__ psi, int64_t n_i, int order_shift,
+                       int key_bits_total, int64_t k, FindCtl* ctl, unsigned int* bins, uint64_t* __restrict__ out) {
+    __shared__ unsigned int s_bins[kSelectBins];
+    __shared__ int s_warp[32];
+    __shared__ int s_pick[3];  // digit, records below it, records at it
+    const cg::grid_group grid = cg::this_grid();
+    const int64_t e = (int64_t)ctl->n_emit;
+    if (ctl->overflow || e > cap || e == 0 || (ctl->emit_from > 0 && e < k)) return;  // (the same for every block)
+    const int lane = threadIdx.x & 31;
+    const int64_t first = (int64_t)blockIdx.x * kTailThreads + threadIdx.x, step = (int64_t)gridDim.x * kTailThreads;
+    const int64_t rounded = (e + 31) / 32 * 32;  // whole warps
+    for (int64_t i = first; i < rounded; i += step) {
+        bool zero = false;
+        if (i < e) {
+            const uint64_t info = rank[2 * i], row = rank[2 * i + 1];
+            const int64_t slot = (int64_t)(info & ((1ull << 62) - 1));
+            const bool in_diag = (info >> 62) & 1;
+            const double w = exact_weight(__ldg((in_diag ? diag.coef : off.coef) + slot), __ldg(psi + row), (int)(info >> 63));
+            const uint64_t order = (uint64_t)__ldg((in_diag ? diag.orig : off.orig) + slot) * (uint64_t)n_i + row;
+            zero = w == 0.0;
+            rank[2 * i] = zero ? ~0ull : ~(uint64_t)__double_as_longlong(w);
+            rank[2 * i + 1] = (~order) << order_shift;
         }
-        const long long below = acc, at = bins[digit];
-        // place the digit below the fixed bits
-        uint64_t p0 = ctl->sel_p0, p1 = ctl->sel_p1;
-        const uint64_t d = (uint64_t)digit;
+        const unsigned z = __ballot_sync(0xffffffffu, zero);
+        if (z != 0 && lane == 0) atomicAdd(&ctl->n_zero, (unsigned long long)__popc(z));
+    }
+    grid.sync();
+    const int64_t valid = e - (int64_t)*(volatile unsigned long long*)&ctl->n_zero;
+    int64_t need = k < valid ? k : valid;
+    uint64_t p0 = 0, p1 = 0;
+    int fixed = 0;
+    // all of the valid records: those below the all-ones weight key
+    const bool every = need == valid;
+    for (int level = 0; !every && need > 0 && fixed < key_bits_total; ++level) {
+        unsigned int* const mine = bins + level % 3 * kSelectBins;
+        unsigned int* const next = bins + (level + 1) % 3 * kSelectBins;
+        for (int64_t b = first; b < kSelectBins; b += step) next[b] = 0;
+        const int cnt = key_bits_total - fixed < kSelectBits ? key_bits_total - fixed : kSelectBits;
+        for (int b = threadIdx.x; b < kSelectBins; b += kTailThreads) s_bins[b] = 0;
+        __syncthreads();
+        for (int64_t i = first; i < e; i += step) {
+            const uint64_t k0 = rank[2 * i], k1 = rank[2 * i + 1];
+            if (prefix_cmp(k0, k1, p0, p1, fixed) == 0) atomicAdd(&s_bins[key_bits(k0, k1, fixed, cnt)], 1u);
+        }
+        __syncthreads();
+        for (int b = threadIdx.x; b < kSelectBins; b += kTailThreads) {
+            const unsigned int v = s_bins[b];
+            if (v) atomicAdd(mine + b, v);
+        }
+        grid.sync();
+        // the digit where the remaining count is reached: two bins a thread (records number less than 2^31)
+        static_assert(kSelectBins == 2 * kTailThreads, "two bins a thread");
+        const int c0 = (int)((volatile unsigned int*)mine)[2 * threadIdx.x], c1 = (int)((volatile unsigned int*)mine)[2 * threadIdx.x + 1];
+        const int run = block_inclusive_scan(c0 + c1, s_warp);
+        const int before = run - c0 - c1;
+        if (run >= need && before < need) {
+            const bool second = before + c0 < need;
+            s_pick[0] = 2 * threadIdx.x + (second ? 1 : 0);
+            s_pick[1] = second ? before + c0 : before;
+            s_pick[2] = second ? c1 : c0;
+        }
+        __syncthreads();
+        const uint64_t d = (uint64_t)s_pick[0];
         if (fixed + cnt <= 64) {
             p0 |= d << (64 - fixed - cnt);
         } else if (fixed >= 64) {
@@ -638,37 +637,164 @@ __global__ void __launch_bounds__(kChooseThreads) select_choose_kernel(int key_b
             p0 |= d >> lo_bits;
             p1 |= d << (64 - lo_bits);
         }
-        ctl->sel_p0 = p0;
-        ctl->sel_p1 = p1;
-        ctl->sel_need = need - below;
-        if (at == need - below || fixed + cnt >= key_bits_total) ctl->sel_done = 1;
+        need -= s_pick[1];
+        fixed += cnt;
+        if (s_pick[2] == need) break;
+        __syncthreads();  // s_pick is written again
     }
-    __syncthreads();
-    // every thread has read ctl->sel_bits before it moves on (the fixed-bit count of this level)
-    if (t == 0) ctl->sel_bits = fixed + cnt;
-    for (int b = t; b < kSelectBins; b += kChooseThreads) bins[b] = 0;
+    // the records up to the chosen prefix
+    if (need <= 0) return;
+    for (int64_t i = first; i < rounded; i += step) {
+        bool take = false;
+        if (i < e) {
+            const uint64_t k0 = rank[2 * i], k1 = rank[2 * i + 1];
+            take = every ? k0 != ~0ull : prefix_cmp(k0, k1, p0, p1, fixed) <= 0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, take);
+        unsigned long long base = 0;
+        if (lane == 0 && m) base = atomicAdd(&ctl->n_sel, (unsigned long long)__popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (take) {
+            const unsigned long long at = base + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+            for (int q = 0; q < W; ++q) out[at * W + q] = keys[i * W + q];
+        }
+    }
 }
 
-// Keys of the accepted records (rank prefix at most the chosen prefix), in no particular order.
+// Blocks of the sort for up to k rows: one per SM, fewer for few rows.
+int64_t sort_blocks_for(int64_t k) {
+    const int64_t b = (k + 255) / 256;
+    return b < 1 ? 1 : b > 152 ? 152 : b;
+}
+
+// Sort ctl->n_sel keys (LSD radix, a row byte a pass, least significant
+// first), keep the distinct ones and write them as rows of nq bytes.  Block b
+// owns the b-th contiguous share of the keys and its warps contiguous pieces
+// of that, so a pass is stable: count digits per warp; (barrier) every digit's
+// counts are summed over the blocks by one warp; (barrier) every key goes
+// behind the smaller digits, the same digit of earlier blocks and warps, and
+// its own place within the warp; (barrier).  Keys travel alone, in two
+// buffers.  counts: 256 x gridDim.x + 256 values.
 template <int W>
-__global__ void select_compact_kernel(const uint64_t* __restrict__ rank, const uint64_t* __restrict__ keys, int64_t n,
-                                      FindCtl* __restrict__ ctl, uint64_t* __restrict__ out) {
-    const uint64_t p0 = ctl->sel_p0, p1 = ctl->sel_p1;
-    const int bits = ctl->sel_bits;
-    const bool none = ctl->sel_need <= 0 && bits == 0;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool take = false;
-    if (i < n && !none) take = prefix_cmp(rank[2 * i], rank[2 * i + 1], p0, p1, bits) <= 0;
-    const unsigned m = __ballot_sync(0xffffffffu, take);
-    const int lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    if (lane == 0 && m) base = atomicAdd(&ctl->n_sel, (unsigned long long)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (take) {
-        const unsigned long long at = base + __popc(m & ((1u << lane) - 1u));
+__global__ void __launch_bounds__(kTailThreads)
+    find_sort_kernel(uint64_t* keys, uint64_t* other, int32_t* counts, FindCtl* ctl, int nq, uint8_t* __restrict__ out) {
+    __shared__ int32_t s_cnt[kTailWarps][256];
+    __shared__ int32_t s_base[256];
+    __shared__ int s_warp[32];
+    const cg::grid_group grid = cg::this_grid();
+    const int64_t n = (int64_t)ctl->n_sel;
+    if (n == 0) return;  // (the same for every block)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int blocks = (int)gridDim.x, me = (int)blockIdx.x;
+    int32_t* const totals = counts + 256 * (int64_t)blocks;
+    const int64_t chunk = (n + blocks - 1) / blocks;
+    const int64_t lo = (int64_t)me * chunk < n ? (int64_t)me * chunk : n;
+    const int64_t hi = lo + chunk < n ? lo + chunk : n;
+    const int64_t piece = ((hi - lo + kTailWarps - 1) / kTailWarps + 31) / 32 * 32;
+    const int64_t wlo = lo + warp * piece < hi ? lo + warp * piece : hi;
+    const int64_t whi = wlo + piece < hi ? wlo + piece : hi;
+    uint64_t* src = keys;
+    uint64_t* dst = other;
+    for (int byte = nq - 1; byte >= 0; --byte) {
+        const int word = byte >> 3, shift = 8 * (7 - (byte & 7));
+        for (int d = lane; d < 256; d += 32) s_cnt[warp][d] = 0;
+        __syncwarp();
+        for (int64_t i = wlo + lane; i < whi; i += 32) atomicAdd(&s_cnt[warp][(unsigned)(src[i * W + word] >> shift) & 0xffu], 1);
+        __syncthreads();
+        if (threadIdx.x < 256) {
+            int32_t run = 0;
+            for (int w = 0; w < kTailWarps; ++w) {
+                const int32_t c = s_cnt[w][threadIdx.x];
+                s_cnt[w][threadIdx.x] = run;
+                run += c;
+            }
+            counts[(int64_t)threadIdx.x * blocks + me] = run;
+        }
+        grid.sync();
+        for (int d = me + warp * blocks; d < 256; d += kTailWarps * blocks) {
+            int32_t before = 0;
+            for (int b = 0; b < blocks; b += 32) {
+                const int32_t c = b + lane < blocks ? counts[(int64_t)d * blocks + b + lane] : 0;
+                int32_t x = c;
 #pragma unroll
-        for (int q = 0; q < W; ++q) out[at * W + q] = keys[i * W + q];
+                for (int s = 1; s < 32; s <<= 1) {
+                    const int32_t y = __shfl_up_sync(0xffffffffu, x, s);
+                    if (lane >= s) x += y;
+                }
+                if (b + lane < blocks) counts[(int64_t)d * blocks + b + lane] = before + x - c;
+                before += __shfl_sync(0xffffffffu, x, 31);
+            }
+            if (lane == 0) totals[d] = before;
+        }
+        grid.sync();
+        const int total = threadIdx.x < 256 ? totals[threadIdx.x] : 0;
+        const int up_to = block_inclusive_scan(total, s_warp);
+        if (threadIdx.x < 256) s_base[threadIdx.x] = up_to - total + counts[(int64_t)threadIdx.x * blocks + me];
+        __syncthreads();
+        for (int64_t base = wlo; base < whi; base += 32) {
+            const int64_t i = base + lane;
+            const bool in = i < whi;
+            uint64_t key[W];
+#pragma unroll
+            for (int q = 0; q < W; ++q) key[q] = in ? src[i * W + q] : 0;
+            const unsigned d = in ? (unsigned)(src[i * W + word] >> shift) & 0xffu : 256u;
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const int leader = __ffs(peers) - 1;
+            int at = 0;
+            if (in && lane == leader) {
+                at = s_cnt[warp][d];
+                s_cnt[warp][d] = at + __popc(peers);
+            }
+            at = __shfl_sync(0xffffffffu, at, leader);
+            if (in) {
+                const int64_t to = (int64_t)s_base[d] + at + __popc(peers & lt);
+#pragma unroll
+                for (int q = 0; q < W; ++q) dst[to * W + q] = key[q];
+            }
+            __syncwarp();
+        }
+        uint64_t* const t = src;
+        src = dst;
+        dst = t;
+        grid.sync();
     }
+    // the first of every run of equal keys
+    auto head = [&](int64_t i) {
+        bool h = i == 0;
+#pragma unroll
+        for (int q = 0; q < W; ++q) h = h || src[i * W + q] != src[(i - 1) * W + q];
+        return h;
+    };
+    int heads = 0;
+    for (int64_t base = wlo; base < whi; base += 32) {
+        heads += __popc(__ballot_sync(0xffffffffu, base + lane < whi && head(base + lane)));
+    }
+    // places: heads of earlier blocks (counts[b]), of earlier warps, of earlier lanes
+    const int in_block = block_inclusive_scan(lane == 0 ? heads : 0, s_warp);
+    if (threadIdx.x == kTailThreads - 1) counts[me] = in_block;
+    grid.sync();
+    int earlier = 0, all = 0;
+    for (int b = lane; b < blocks; b += 32) {
+        const int c = counts[b];
+        all += c;
+        if (b < me) earlier += c;
+    }
+    earlier = (int)__reduce_add_sync(0xffffffffu, (unsigned)earlier);
+    all = (int)__reduce_add_sync(0xffffffffu, (unsigned)all);
+    int64_t at = earlier + __shfl_sync(0xffffffffu, in_block, 0) - heads;
+    for (int64_t base = wlo; base < whi; base += 32) {
+        const int64_t i = base + lane;
+        const bool h = i < whi && head(i);
+        const unsigned m = __ballot_sync(0xffffffffu, h);
+        if (h) {
+            uint8_t* r = out + (at + __popc(m & lt)) * nq;
+            for (int b = 0; b < nq; ++b) r[b] = (uint8_t)(src[i * W + (b >> 3)] >> (8 * (7 - (b & 7))));
+        }
+        at += __popc(m);
+    }
+    if (me == 0 && threadIdx.x == 0) ctl->n_unique = (unsigned long long)all;
 }
 
 __global__ void zero_u64_kernel(unsigned long long* p, int n) {
@@ -698,11 +824,11 @@ struct FindLayout {
     uint64_t* keys_i;
     uint64_t* keys_s;       // every kSampleStride-th row of keys_i
     double2* psi_s;         // and its amplitude
-    unsigned long long* hist;
+    unsigned long long* hist;  // bucket counts; the selection's bins afterwards
     FindCtl* ctl;
-    unsigned int* bins;     // radix-select histogram
-    uint64_t* sel_keys;
-    RowSet final_set;       // sort and de-duplication of the selected rows
+    uint64_t* sel_keys;     // the selected rows' keys, and the buffer they are sorted with
+    uint64_t* sort_keys;
+    int32_t* sort_counts;
     // emission area
     uint64_t* emit_rank;
     uint64_t* emit_keys;
@@ -718,10 +844,10 @@ FindLayout<W> take_find(Arena& ws, int64_t n_i, int64_t k, int64_t n_ex, int64_t
     L.psi_s = ws.take<double2>((uint64_t)n_s);
     L.hist = ws.take<unsigned long long>(kBuckets);
     L.ctl = ws.take<FindCtl>(1);
-    L.bins = ws.take<unsigned int>(kSelectBins);
     int64_t kk = k > 0 ? k : 1;
     L.sel_keys = ws.take<uint64_t>((uint64_t)kk * W);
-    L.final_set = take_rowset<W>(ws, kk);
+    L.sort_keys = ws.take<uint64_t>((uint64_t)kk * W);
+    L.sort_counts = ws.take<int32_t>(256 * (uint64_t)sort_blocks_for(kk) + 256);
     int64_t c = cap > 0 ? cap : 1;
     L.emit_rank = ws.take<uint64_t>((uint64_t)c * 2);
     L.emit_keys = ws.take<uint64_t>((uint64_t)c * W);
@@ -764,10 +890,15 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
     g_find_stats = FindStats{};
     if (k == 0 || a.n_i == 0) return QMBX_OK;
     int st;
-    if ((st = build_hashrows<W>(a.configs_ex, nq, L.excl, s)) != QMBX_OK) return st;
-    if ((st = pack_rows<W>(a.configs_i, a.n_i, nq, L.keys_i, s)) != QMBX_OK) return st;
+    // the exclusion set is only looked up: no first rows, no list of distinct ones
+    if ((st = build_hashset<W>(a.configs_ex, nq, L.excl, s)) != QMBX_OK) return st;
+    const uint64_t* keys_i = L.excl.keys;
+    if (a.configs_i != a.configs_ex || a.n_i > a.n_ex) {
+        if ((st = pack_rows<W>(a.configs_i, a.n_i, nq, L.keys_i, s)) != QMBX_OK) return st;
+        keys_i = L.keys_i;
+    }
     QMBX_CUDA_TRY(cudaMemsetAsync(L.ctl, 0, sizeof(FindCtl), s));
-    QMBX_KERNEL(kGroupOther, s, zero_u64_kernel<<<grid_for(kBuckets, kThreads), kThreads, 0, s>>>(L.hist, kBuckets));
+    QMBX_CUDA_TRY(cudaMemsetAsync(L.hist, 0, kBuckets * sizeof(unsigned long long), s));
 
     RelativeArgs r{};
     r.psi = reinterpret_cast<const double2*>(a.psi_i);
@@ -793,7 +924,7 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
     const bool bounded = relative_bounded(r.off);
     if (sampled) {
         const int64_t n_s = (a.n_i + kSampleStride - 1) / kSampleStride;
-        QMBX_KERNEL(kGroupOther, s, sample_rows_kernel<W><<<grid_for(n_s, kThreads), kThreads, 0, s>>>(L.keys_i, r.psi, n_s, L.keys_s, L.psi_s));
+        QMBX_KERNEL(kGroupOther, s, sample_rows_kernel<W><<<grid_for(n_s, kThreads), kThreads, 0, s>>>(keys_i, r.psi, n_s, L.keys_s, L.psi_s));
         QMBX_LAUNCH_CHECK("sample_rows_kernel");
         RelativeArgs rs = r;
         rs.psi = L.psi_s;
@@ -808,24 +939,50 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
     } else {
         RelativeArgs r1 = r;
         r1.hist_exact = 0;
-        st = bounded ? launch_bounded<W, false>(r1, L.keys_i, a.n_i, row_split(a.n_i), histogram_depth(k, a.n_i), s)
-                     : launch_relative<W, false>(r1, L.keys_i, a.n_i, s);
+        st = bounded ? launch_bounded<W, false>(r1, keys_i, a.n_i, row_split(a.n_i), histogram_depth(k, a.n_i), s)
+                     : launch_relative<W, false>(r1, keys_i, a.n_i, s);
         if (st != QMBX_OK) return st;
         ++g_find_stats.walks;
         QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, 1.0, (double)k, L.ctl));
     }
     QMBX_LAUNCH_CHECK("choose_emit_kernel");
 
-    // pass 2: emit the records at or above emit_from.  Every record down to
-    // the k-th was emitted when at least k were (or the threshold is the
-    // lowest bucket); otherwise the sample put the threshold too high, and
-    // an unsampled histogram pass gives the exact one for a second emission
-    // pass (never seen on the benchmark shapes; the tests drive it).
+    // bits of the visiting order (term index * n_i + row < n_terms * n_i), in whole bytes
+    int order_bytes = 1;
+    {
+        const double span = (double)(h->n_terms > 0 ? h->n_terms : 1) * (double)a.n_i;
+        while (order_bytes < 8 && span > std::ldexp(1.0, 8 * order_bytes)) ++order_bytes;
+    }
+    int order_shift = 64 - 8 * order_bytes;
+    int key_bits_total = 64 + 8 * order_bytes;
+    const int sms = pivot_grid() / 4;
+    // pass 2: emit the records at or above emit_from, select and sort.  Every
+    // record down to the k-th was emitted when at least k were (or the
+    // threshold is the lowest bucket); otherwise the sample put the threshold
+    // too high, nothing is selected, and an unsampled histogram pass gives the
+    // exact one for a second round (never seen on the benchmark shapes; the
+    // tests drive it).
     FindCtl ctl{};
     for (int attempt = 0;; ++attempt) {
-        st = bounded ? launch_bounded<W, true>(r, L.keys_i, a.n_i, emission_split(k, a.n_i), 0, s) : launch_relative<W, true>(r, L.keys_i, a.n_i, s);
+        st = bounded ? launch_bounded<W, true>(r, keys_i, a.n_i, emission_split(k, a.n_i), 0, s)
+                     : launch_relative<W, true>(r, keys_i, a.n_i, s);
         if (st != QMBX_OK) return st;
         ++g_find_stats.walks;
+        unsigned int* bins = reinterpret_cast<unsigned int*>(L.hist);  // cleared by choose_emit_kernel
+        {
+            int64_t n_i = a.n_i, want = k, places = cap;
+            const double2* psi = r.psi;
+            void* args[] = {&L.emit_rank, &L.emit_keys, &places, &r.off, &r.diag, &psi, &n_i, &order_shift,
+                            &key_bits_total, &want, &L.ctl, &bins, &L.sel_keys};
+            QMBX_KERNEL(kGroupSelect, s, QMBX_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)find_select_kernel<W>, dim3(sms), dim3(kTailThreads), args, 0, s)));
+        }
+        {
+            int bytes = nq;
+            uint8_t* out = a.out;
+            void* args[] = {&L.sel_keys, &L.sort_keys, &L.sort_counts, &L.ctl, &bytes, &out};
+            const int64_t blocks = sort_blocks_for(k) < sms ? sort_blocks_for(k) : sms;
+            QMBX_KERNEL(kGroupSort, s, QMBX_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)find_sort_kernel<W>, dim3((unsigned)blocks), dim3(kTailThreads), args, 0, s)));
+        }
         QMBX_CUDA_TRY(cudaMemcpyAsync(&ctl, L.ctl, sizeof(FindCtl), cudaMemcpyDeviceToHost, s));
         QMBX_CUDA_TRY(cudaStreamSynchronize(s));
         if (ctl.overflow || (int64_t)ctl.n_emit > cap) {
@@ -837,54 +994,23 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
         if (attempt > 0) return fail(QMBX_ERR_DEVICE, "find_relative threshold did not settle");
         // the exact threshold from the counts of every record
         QMBX_KERNEL(kGroupOther, s, zero_u64_kernel<<<grid_for(kBuckets, kThreads), kThreads, 0, s>>>(L.hist, kBuckets));
-        if ((st = launch_relative<W, false>(r, L.keys_i, a.n_i, s)) != QMBX_OK) return st;
+        if ((st = launch_relative<W, false>(r, keys_i, a.n_i, s)) != QMBX_OK) return st;
         ++g_find_stats.walks;
         QMBX_CUDA_TRY(cudaMemsetAsync(L.ctl, 0, sizeof(FindCtl), s));
         QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, 1.0, (double)k, L.ctl));
         QMBX_LAUNCH_CHECK("choose_emit_kernel");
     }
-    g_find_stats.records = (int64_t)ctl.n_emit;
-    if (ctl.n_emit == 0) return QMBX_OK;
-    const int64_t e = (int64_t)ctl.n_emit;
-    // bytes of the visiting order (term index * n_i + row < n_terms * n_i)
-    int order_bytes = 1;
-    {
-        const double span = (double)(h->n_terms > 0 ? h->n_terms : 1) * (double)a.n_i;
-        while (order_bytes < 8 && span > std::ldexp(1.0, 8 * order_bytes)) ++order_bytes;
-    }
-    const int order_shift = 64 - 8 * order_bytes;
-    const int key_bits_total = 64 + 8 * order_bytes;
-    QMBX_KERNEL(kGroupSelect, s, rank_records_kernel<<<grid_for(e, kThreads), kThreads, 0, s>>>(L.emit_rank, e, r.off, r.diag, r.psi, a.n_i, order_shift, &L.ctl->n_zero));
-    QMBX_LAUNCH_CHECK("rank_records_kernel");
-    // radix select of the k smallest rank keys (zero-weight records rank last and are never taken)
-    QMBX_KERNEL(kGroupSelect, s, select_init_kernel<<<1, 256, 0, s>>>(L.ctl, (long long)k, (long long)e, L.bins));
-    const int levels = (key_bits_total + kSelectBits - 1) / kSelectBits;
-    const unsigned sel_grid = grid_for(e, kThreads) < 2u * 152u ? grid_for(e, kThreads) : 2u * 152u;
-    for (int level = 0; level < levels; ++level) {
-        QMBX_KERNEL(kGroupSelect, s, select_hist_kernel<<<sel_grid, kThreads, 0, s>>>(L.emit_rank, e, key_bits_total, L.ctl, L.bins));
-        QMBX_KERNEL(kGroupSelect, s, select_choose_kernel<<<1, kChooseThreads, 0, s>>>(key_bits_total, L.ctl, L.bins));
-    }
-    QMBX_KERNEL(kGroupSelect, s, select_compact_kernel<W><<<grid_for(e, kThreads), kThreads, 0, s>>>(L.emit_rank, L.emit_keys, e, L.ctl, L.sel_keys));
-    QMBX_LAUNCH_CHECK("find_relative selection");
-    unsigned long long n_sel = 0;
-    QMBX_CUDA_TRY(cudaMemcpyAsync(&n_sel, &L.ctl->n_sel, sizeof(n_sel), cudaMemcpyDeviceToHost, s));
-    QMBX_CUDA_TRY(cudaStreamSynchronize(s));
-    const int64_t keep = (int64_t)n_sel;
-    if (keep == 0) return QMBX_OK;
+    const int64_t keep = (int64_t)ctl.n_sel;
     if (keep > k) return fail(QMBX_ERR_DEVICE, "find_relative selected %lld records for %lld places", (long long)keep, (long long)k);
-    // sort and de-duplicate the selected rows, then unpack the distinct ones
+    g_find_stats.records = (int64_t)ctl.n_emit;
     g_find_stats.selected = keep;
-    g_find_stats.sort_passes = nq;
-    // per pass: the selected keys (8W bytes) and their 4-byte index, read and written
-    g_find_stats.sort_bytes = (int64_t)nq * 2 * keep * (8 * W + 4);
-    L.final_set.n = keep;
-    if ((st = sort_unique_keys<W>(L.sel_keys, nq, L.final_set, s)) != QMBX_OK) return st;
-    if ((st = unpack_rows<W>(L.final_set.keys, L.final_set.count, keep, nq, a.out, s)) != QMBX_OK) return st;
-    int n_unique = 0;
-    QMBX_CUDA_TRY(cudaMemcpyAsync(&n_unique, L.final_set.count, sizeof(int), cudaMemcpyDeviceToHost, s));
-    QMBX_CUDA_TRY(cudaStreamSynchronize(s));
-    *a.n_out = n_unique;
-    g_find_stats.rows_out = n_unique;
+    if (keep > 0) {
+        // per pass: the selected keys read and written
+        g_find_stats.sort_passes = nq;
+        g_find_stats.sort_bytes = (int64_t)nq * 2 * keep * 8 * W;
+    }
+    *a.n_out = (int64_t)ctl.n_unique;
+    g_find_stats.rows_out = (int64_t)ctl.n_unique;
     return QMBX_OK;
 }
 
