@@ -1045,6 +1045,7 @@ struct SingleVisitor : VisitorBase {
     const int32_t* orig;
     uint8_t* out;
     int nq;
+    const int32_t* rows;  // walked rows (NULL: every row)
     struct Acc {
         double key;
         int32_t term;
@@ -1097,9 +1098,158 @@ struct SingleVisitor : VisitorBase {
         }
     }
     __device__ __forceinline__ void finish(Acc& a, int64_t row, const Key<W>&) const {
-        uint8_t* r = out + row * nq;
+        uint8_t* r = out + (rows != nullptr ? (int64_t)__ldg(rows + row) : row) * nq;
         for (int b = 0; b < nq; ++b) r[b] = (uint8_t)(a.best.w[b >> 3] >> (8 * (7 - (b & 7))));
     }
+};
+
+// ---------------------------------------------------------------------------
+// single_relative by the terms in key order.  A term's key is the same for
+// every row, so a row's neighbour is given by the first term, in descending
+// key order, that applies and leads outside the input.  Terms apply to a few
+// per cent of the rows, so a row finds it among the first hundred or so: the
+// best couple of thousand terms are gathered and sorted once, and a warp takes a
+// row through them 32 at a time.  Rows that find none there are walked.
+//   20,000 rows under 55,371 terms: walk 648 us; bins, gather, sort and rows 26 us
+// ---------------------------------------------------------------------------
+
+constexpr int kBestTerms = 2048;
+constexpr int kKeyBins = 1 << 14;  // exponent and three mantissa bits of |key|: bins of a ratio of at most 1.125
+
+struct BestTerm {
+    unsigned long long key;  // |key| as ordered bits: the smallest is the best
+    int32_t orig, slot;      // input order breaks ties
+};
+
+struct SingleCtl {
+    int gathered;   // terms in the list
+    int unresolved; // rows to walk
+};
+
+__device__ __forceinline__ unsigned long long single_key(double kf) {
+    return (unsigned long long)__double_as_longlong(fabs(kf));  // keys are log(u) / |coef| <= 0
+}
+
+__global__ void single_bins_kernel(const double* __restrict__ kf, int64_t n, int* __restrict__ bins) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int bin = i < n ? (int)(single_key(kf[i]) >> 49) : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, bin);
+    if (bin >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(bins + bin, __popc(peers));
+}
+
+// The terms of the lowest bins that together hold at most kBestTerms.  Every
+// block finds the last such bin for itself.
+__global__ void __launch_bounds__(kTailThreads) single_gather_kernel(const double* __restrict__ kf,
+                                                                     const int32_t* __restrict__ orig, int64_t n,
+                                                                     const int* __restrict__ bins,
+                                                                     BestTerm* __restrict__ best,
+                                                                     SingleCtl* __restrict__ ctl) {
+    __shared__ int s_warp[32];
+    __shared__ int s_end;  // first bin left out
+    constexpr int kPer = kKeyBins / kTailThreads;
+    if (threadIdx.x == 0) s_end = kKeyBins;
+    int mine[kPer];
+    int sum = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; k += 4) {
+        const int4 v = __ldg(reinterpret_cast<const int4*>(bins + kPer * threadIdx.x + k));
+        mine[k] = v.x;
+        mine[k + 1] = v.y;
+        mine[k + 2] = v.z;
+        mine[k + 3] = v.w;
+        sum += v.x + v.y + v.z + v.w;
+    }
+    const int run = block_inclusive_scan(sum, s_warp);
+    if (run > kBestTerms && run - sum <= kBestTerms) {
+        int upto = run - sum, end = kPer * threadIdx.x;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            upto += mine[k];
+            if (upto <= kBestTerms) end = kPer * threadIdx.x + k + 1;
+        }
+        s_end = end;
+    }
+    __syncthreads();
+    const int end = s_end;
+    for (int64_t i = (int64_t)blockIdx.x * kTailThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kTailThreads) {
+        const unsigned long long key = single_key(kf[i]);
+        if ((int)(key >> 49) >= end) continue;
+        BestTerm t;
+        t.key = key;
+        t.orig = __ldg(orig + i);
+        t.slot = (int32_t)i;
+        best[atomicAdd(&ctl->gathered, 1)] = t;
+    }
+}
+
+// Sort the gathered terms by (key, input order), which no two share: a warp
+// counts the terms ahead of one.  (A bitonic sort of 4,096 terms in one block
+// took 112 us; the counts of 2,048 take a few.)
+__global__ void __launch_bounds__(kThreads) single_sort_kernel(const BestTerm* __restrict__ best,
+                                                               const SingleCtl* __restrict__ ctl,
+                                                               BestTerm* __restrict__ sorted) {
+    __shared__ unsigned long long s_key[kBestTerms];
+    __shared__ int32_t s_orig[kBestTerms];
+    const int n = ctl->gathered;
+    if ((int)blockIdx.x * kWarpsPerBlock >= n) return;
+    for (int i = threadIdx.x; i < n; i += kThreads) {
+        s_key[i] = best[i].key;
+        s_orig[i] = best[i].orig;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int me = (int)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    if (me >= n) return;
+    const unsigned long long key = s_key[me];
+    const int32_t orig = s_orig[me];
+    unsigned ahead = 0;
+    for (int i = lane; i < n; i += 32) ahead += s_key[i] < key || (s_key[i] == key && s_orig[i] < orig) ? 1u : 0u;
+    ahead = __reduce_add_sync(0xffffffffu, ahead);
+    if (lane == 0) sorted[ahead] = best[me];
+}
+
+template <int W>
+__global__ void __launch_bounds__(kThreads) single_first_kernel(const uint64_t* __restrict__ keys, int64_t n, HashView set,
+                                                                PartView off, const BestTerm* __restrict__ best,
+                                                                SingleCtl* __restrict__ ctl,
+                                                                int32_t* __restrict__ unresolved, int nq,
+                                                                uint8_t* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    if (row >= n) return;
+    const int terms = ctl->gathered;
+    const Key<W> c = load_key<W>(keys, row);
+    for (int base = 0; base < terms; base += 32) {
+        bool on = false;
+        Key<W> img{};
+        if (base + lane < terms) {
+            const int32_t slot = __ldg(&best[base + lane].slot);
+            TermRec<W> rec;
+            load_test<W>(rec, off, slot);
+            if (rec.applies(c)) {
+                load_apply<W>(rec, off, slot);
+                rec.image(c, img);
+                on = hash_find<W>(set, img) < 0;
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (m != 0) {
+            if (lane == __ffs(m) - 1) {
+                uint8_t* r = out + row * nq;
+                for (int b = 0; b < nq; ++b) r[b] = (uint8_t)(img.w[b >> 3] >> (8 * (7 - (b & 7))));
+            }
+            return;
+        }
+    }
+    if (lane == 0) unresolved[atomicAdd(&ctl->unresolved, 1)] = (int32_t)row;
+}
+
+// The rows of a list.
+template <int W>
+struct ListedRows {
+    const uint64_t* keys;
+    const int32_t* rows;
+    __device__ __forceinline__ Key<W> get(int64_t i) const { return load_key<W>(keys, __ldg(rows + i)); }
 };
 
 template <int W>
@@ -1107,6 +1257,34 @@ struct SingleLayout {
     HashRows set;
     double* kf;
 };
+
+// Behind it, for calls by the terms in key order.
+struct SingleOrder {
+    SingleCtl* ctl;  // followed by the bins, cleared together
+    int* bins;
+    BestTerm* best;
+    BestTerm* sorted;
+    int32_t* unresolved;
+};
+
+SingleOrder take_single_order(Arena& ws, int64_t n) {
+    SingleOrder o;
+    o.ctl = ws.take<SingleCtl>(1);
+    o.bins = ws.take<int>(kKeyBins);
+    o.best = ws.take<BestTerm>(kBestTerms);
+    o.sorted = ws.take<BestTerm>(kBestTerms);
+    o.unresolved = ws.take<int32_t>((uint64_t)(n > 0 ? n : 1));
+    return o;
+}
+
+// Whether rows are taken through the terms in key order: where the walks would
+// visit enough terms to outweigh ordering them.
+bool single_ordered(const PartView& off, int64_t n) {
+    const char* e = getenv("QMBX_WALK");
+    const char f = e != nullptr ? e[0] : 0;
+    if (f == 't' || f == 'g' || f == 'p') return false;
+    return off.n >= kGroupedMinTerms && (double)n * (double)off.n > 2e7;
+}
 
 template <int W>
 SingleLayout<W> take_single(Arena& ws, int64_t n, int64_t n_off) {
@@ -1126,14 +1304,31 @@ int single_impl(const void* table_host, const void* table_dev, const uint8_t* co
     if (!ws.fits()) return fail(QMBX_ERR_WORKSPACE, "single_relative needs %llu bytes of workspace", (unsigned long long)ws.used);
     if (n == 0) return QMBX_OK;
     int st;
-    if ((st = build_hashrows<W>(configs, h->n_qubytes, L.set, s)) != QMBX_OK) return st;
+    // the set is only looked up: no first rows, no list of distinct ones
+    if ((st = build_hashset<W>(configs, h->n_qubytes, L.set, s)) != QMBX_OK) return st;
     if (off.n > 0) {
         QMBX_KERNEL(kGroupOther, s, es_factor_kernel<<<grid_for(off.n, kThreads), kThreads, 0, s>>>(off.coef, off.orig, off.n, seed, L.kf));
         QMBX_LAUNCH_CHECK("es_factor_kernel");
     }
     PartView none = off;
     none.n = 0;
-    SingleVisitor<W> v{{}, L.set.hash(), L.kf, off.orig, out, h->n_qubytes};
+    SingleVisitor<W> v{{}, L.set.hash(), L.kf, off.orig, out, h->n_qubytes, nullptr};
+    Arena behind = ws;
+    const SingleOrder o = take_single_order(behind, n);
+    if (single_ordered(off, n) && behind.fits()) {
+        QMBX_CUDA_TRY(cudaMemsetAsync(o.ctl, 0, (size_t)(reinterpret_cast<char*>(o.bins + kKeyBins) - reinterpret_cast<char*>(o.ctl)), s));
+        const unsigned blocks = grid_for(off.n, kTailThreads) < 152u ? grid_for(off.n, kTailThreads) : 152u;
+        QMBX_KERNEL(kGroupSelect, s, single_bins_kernel<<<grid_for(off.n, kThreads), kThreads, 0, s>>>(L.kf, off.n, o.bins));
+        QMBX_KERNEL(kGroupSelect, s, single_gather_kernel<<<blocks, kTailThreads, 0, s>>>(L.kf, off.orig, off.n, o.bins, o.best, o.ctl));
+        QMBX_KERNEL(kGroupSort, s, single_sort_kernel<<<kBestTerms / kWarpsPerBlock, kThreads, 0, s>>>(o.best, o.ctl, o.sorted));
+        QMBX_KERNEL(kGroupEnumerate, s, single_first_kernel<W><<<grid_for(n, kWarpsPerBlock), kThreads, 0, s>>>(L.set.keys, n, L.set.hash(), off, o.sorted, o.ctl, o.unresolved, h->n_qubytes, out));
+        // rows that none of these terms serves: the walk over all terms
+        v.rows = o.unresolved;
+        ListedRows<W> rest{L.set.keys, o.unresolved};
+        QMBX_KERNEL(kGroupOther, s, grouped_kernel<W><<<grouped_grid(n), kThreads, 0, s>>>(v, rest, &o.ctl->unresolved, n, off, none));
+        QMBX_LAUNCH_CHECK("single_relative by terms in key order");
+        return QMBX_OK;
+    }
     KeyRows<W> src{L.set.keys};
     if (choose_walk(off, n, false) == Walk::kGrouped) {
         QMBX_KERNEL(kGroupEnumerate, s, grouped_kernel<W><<<grouped_grid(n), kThreads, 0, s>>>(v, src, nullptr, n, off, none));
@@ -1234,6 +1429,7 @@ extern "C" int qmbx_single_relative_workspace(const void* table_host, int64_t n,
         case 4: take_single<4>(probe, n, n_off); break;
         default: return fail(QMBX_ERR_ARGUMENT, "unsupported word count");
     }
+    take_single_order(probe, n);
     *bytes = probe.used;
     return QMBX_OK;
 }
