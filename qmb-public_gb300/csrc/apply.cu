@@ -87,7 +87,7 @@ __device__ __forceinline__ void comp_diag_add(CompSum& dre, CompSum& dim, float4
     const float sg = parity ? -1.f : 1.f;
     const float ih = CONJ ? -cf.z : cf.z, il = CONJ ? -cf.w : cf.w;
     dre.add2(sg * cf.x, sg * cf.y);
-    dim.add2(sg * ih, sg * il);
+    if (ih != 0.f || il != 0.f) dim.add2(sg * ih, sg * il);
 }
 
 // coef (hi/lo split, sign already folded) times psi, added to (re, im) with
@@ -302,11 +302,16 @@ struct DiagonalF64 : VisitorBase {
     __device__ __forceinline__ void visit_diag(Acc& a, const Key<W>&, int parity, int64_t slot) const {
         double2 cf = __ldg(dcoef + slot);
         a.re += parity ? -cf.x : cf.x;
-        a.im += parity ? -cf.y : cf.y;
+        if (cf.y != 0.0) a.im += parity ? -cf.y : cf.y;  // real operators: no second FP64 add
     }
     __device__ __forceinline__ void reduce(Acc& a) const {
         a.re = warp_sum(a.re);
         a.im = warp_sum(a.im);
+    }
+    template <int L>
+    __device__ __forceinline__ void reduce_lanes(Acc& a) const {
+        a.re = lanes_sum<L>(a.re);
+        a.im = lanes_sum<L>(a.im);
     }
     __device__ __forceinline__ void finish(Acc& a, int64_t row, const Key<W>&) const {
         out[row] = make_double2(a.re, a.im);
@@ -530,7 +535,7 @@ struct DiagAdd : VisitorBase {
             const double2 cf = __ldg(dcoef + slot);
             const double ci = CONJ ? -cf.y : cf.y;
             a.dre += parity ? -cf.x : cf.x;
-            a.dim += parity ? -ci : ci;
+            if (ci != 0.0) a.dim += parity ? -ci : ci;  // real operators: no second FP64 add
         }
     }
     __device__ __forceinline__ void reduce(Acc& a) const {
@@ -548,11 +553,8 @@ struct DiagAdd : VisitorBase {
             a.fre.template group_reduce<L>();
             a.fim.template group_reduce<L>();
         } else {
-#pragma unroll
-            for (int d = L / 2; d > 0; d >>= 1) {
-                a.dre += __shfl_xor_sync(0xffffffffu, a.dre, d);
-                a.dim += __shfl_xor_sync(0xffffffffu, a.dim, d);
-            }
+            a.dre = lanes_sum<L>(a.dre);
+            a.dim = lanes_sum<L>(a.dim);
         }
     }
     __device__ __forceinline__ void finish(Acc& a, int64_t u, const Key<W>& c) const {
@@ -737,26 +739,12 @@ int launch_walk(const V& v, const HashRows& walk, const PartView& part, const Pa
     return QMBX_OK;
 }
 
-// Pass over the diagonal terms of every walked row (adds into res): grouped
-// or tiled, as choose_walk says.
+// Pass over the diagonal terms of every walked row (adds into res).
 template <int W, class D>
-int launch_diag(const D& dv, const HashRows& walk, const PartView& part, const PartView& diag, cudaStream_t s,
-                int group = kGroupDiagonal) {
+int launch_diag(const D& dv, const HashRows& walk, const PartView& diag, cudaStream_t s, int group = kGroupDiagonal) {
     if (diag.n == 0) return QMBX_OK;
     UniqueRows<W> src{walk.keys, walk.unique};
-    PartView none = part;
-    none.n = 0;
-    if (choose_walk(diag, walk.n, false) == Walk::kGrouped) {
-        QMBX_KERNEL(group, s, grouped_kernel<W><<<grouped_grid(walk.n), kThreads, 0, s>>>(dv, src, walk.count, walk.n, none, diag));
-    } else {
-        if (diag_lanes(walk.n) == 8) {
-            QMBX_KERNEL(group, s, diag_split_kernel<W, 8><<<grid_for(walk.n * 8, kThreads), kThreads, 0, s>>>(dv, src, walk.count, walk.n, diag));
-        } else {
-            QMBX_KERNEL(group, s, enumerate_kernel<W><<<grid_for(walk.n, kThreads), kThreads, 0, s>>>(dv, src, walk.count, walk.n, none, diag));
-        }
-    }
-    QMBX_LAUNCH_CHECK("apply_within diagonal pass");
-    return QMBX_OK;
+    return launch_diagonal<W>(dv, src, walk.count, walk.n, diag, s, group);
 }
 
 // Pivot-major walk of the changing terms (results added into res by the
@@ -767,7 +755,7 @@ int launch_pivot(const V& v, const D& dv, const HashRows& walk, const PartView& 
     UniqueRows<W> src{walk.keys, walk.unique};
     QMBX_KERNEL(group, s, pivot_kernel<W><<<pivot_grid(), kThreads, 0, s>>>(v, src, walk.count, walk.n, part));
     QMBX_LAUNCH_CHECK("apply_within pivot walk");
-    return launch_diag<W>(dv, walk, part, diag, s, diag_group);
+    return launch_diag<W>(dv, walk, diag, s, diag_group);
 }
 
 // Whether apply_within walks its input side (scatter) or its output side:
@@ -883,7 +871,7 @@ int walk_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_s
 #define QMBX_DIAG_CASE(CONJ, F32, SCATTER)                                              \
     {                                                                                   \
         DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res}; dv.log = a.log;  \
-        st = launch_diag<W>(dv, walk, part, diag, s, diag_group);                                   \
+        st = launch_diag<W>(dv, walk, diag, s, diag_group);                                   \
     }
         if (scatter) {
             if (a.adjoint) {
@@ -935,7 +923,7 @@ int pair_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_s
 #define QMBX_DIAG_CASE(CONJ, F32, SCATTER)                                                                      \
     {                                                                                                           \
         DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res, a.log};      \
-        st = launch_diag<W>(dv, walk, fwd, diag, s, diag_group);                                                \
+        st = launch_diag<W>(dv, walk, diag, s, diag_group);                                                \
     }
     if (scatter) {
         if (a.adjoint) {
@@ -1102,18 +1090,10 @@ template <int W>
 int diagonal_impl(const void* table_host, const void* table_dev, const uint8_t* configs, int64_t n, double2* out,
                   cudaStream_t s) {
     const qmbx_table_header* h = header_of(table_host);
-    PartView none = part_view(table_host, table_dev, QMBX_PART_DIAG);
-    none.n = 0;
-    PartView diag = part_view(table_host, table_dev, QMBX_PART_DIAG);
+    const PartView diag = part_view(table_host, table_dev, QMBX_PART_DIAG);
     DiagonalF64<W> v{{}, diag.coef, out};
     ByteRows<W> src{configs, h->n_qubytes};
-    if (choose_walk(diag, n, false) == Walk::kGrouped) {
-        QMBX_KERNEL(kGroupEnumerate, s, grouped_kernel<W><<<grouped_grid(n), kThreads, 0, s>>>(v, src, nullptr, n, none, diag));
-    } else {
-        QMBX_KERNEL(kGroupEnumerate, s, enumerate_kernel<W><<<grid_for(n, kThreads), kThreads, 0, s>>>(v, src, nullptr, n, none, diag));
-    }
-    QMBX_LAUNCH_CHECK("diagonal_term enumeration");
-    return QMBX_OK;
+    return launch_diagonal<W>(v, src, nullptr, n, diag, s, kGroupEnumerate);
 }
 
 }  // namespace

@@ -107,6 +107,9 @@ struct qmbx_table_header {
     int64_t n_class_list;
     uint64_t off_bound[QMBX_PARTS]; // float[n] of the forward and the diagonal part: the largest norm from a term to
                                     // the end of its pivot group (0: none)
+    int32_t diag_bare;              // 1: every diagonal term is a product of at most two occupations: it applies to
+                                    // every row that reaches its pivot group, with no parity
+    int32_t reserved;
 };
 
 #ifdef __cplusplus

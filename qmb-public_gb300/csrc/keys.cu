@@ -321,6 +321,11 @@ int row_split(int64_t n_rows) {
     return (int)(k < 16 ? k : 16);
 }
 
+bool walk_forced() {
+    const char* e = getenv("QMBX_WALK");
+    return e != nullptr && (e[0] == 't' || e[0] == 'g' || e[0] == 'p');
+}
+
 Walk choose_walk(const PartView& part, int64_t n_rows, bool pivot_ok) {
     const char* e = getenv("QMBX_WALK");
     const char f = e != nullptr ? e[0] : 0;

@@ -139,11 +139,16 @@ struct MatrixDiagonal : VisitorBase {
     __device__ __forceinline__ void visit_diag(Acc& a, const Key<W>&, int parity, int64_t slot) const {
         const double2 cf = __ldg(dcoef + slot);
         a.re += parity ? -cf.x : cf.x;
-        a.im += parity ? -cf.y : cf.y;
+        if (cf.y != 0.0) a.im += parity ? -cf.y : cf.y;
     }
     __device__ __forceinline__ void reduce(Acc& a) const {
         a.re = warp_sum(a.re);
         a.im = warp_sum(a.im);
+    }
+    template <int L>
+    __device__ __forceinline__ void reduce_lanes(Acc& a) const {
+        a.re = lanes_sum<L>(a.re);
+        a.im = lanes_sum<L>(a.im);
     }
     __device__ __forceinline__ void finish(Acc& a, int64_t u, const Key<W>&) const {
         const int32_t row = __ldg(unique + u);
@@ -318,13 +323,8 @@ int matrix_walk(const void* table_host, const void* table_dev, const MatrixLayou
     }
     if (FILL) {
         MatrixDiagonal<W> dv{{}, diag.coef, L.rows.unique, row_ptr, col, val};
-        PartView nd = diag;
-        if (choose_walk(diag, n, false) == Walk::kGrouped) {
-            QMBX_KERNEL(kGroupDiagonal, s, grouped_kernel<W><<<grouped_grid(n), kThreads, 0, s>>>(dv, src, L.rows.count, n, none, nd));
-        } else {
-            QMBX_KERNEL(kGroupDiagonal, s, enumerate_kernel<W><<<grid_for(n, kThreads), kThreads, 0, s>>>(dv, src, L.rows.count, n, none, nd));
-        }
-        QMBX_LAUNCH_CHECK("matrix diagonal pass");
+        int st = launch_diagonal<W>(dv, src, L.rows.count, n, diag, s, kGroupDiagonal);
+        if (st != QMBX_OK) return st;
     }
     return QMBX_OK;
 }

@@ -511,6 +511,21 @@ extern "C" int qmbx_table_build(const int16_t* site, const uint8_t* kind, const 
             ++k_off;
         }
     }
+    {
+        const qmbx_table_part& p = h.part[QMBX_PART_DIAG];
+        const uint64_t* test = reinterpret_cast<const uint64_t*>(out + p.off_test);
+        const uint64_t* apply = reinterpret_cast<const uint64_t*>(out + p.off_apply);
+        h.diag_bare = 1;
+        for (int64_t t = 0; t < p.n; ++t) {
+            int sites = 0;
+            for (int w = 0; w < words; ++w) {
+                const uint64_t at = ((uint64_t)w * (uint64_t)p.n + (uint64_t)t) * 2;
+                sites += __builtin_popcountll(test[at]);
+                if (test[at] != test[at + 1] || apply[at + 1] != 0) h.diag_bare = 0;
+            }
+            if (sites > 2) h.diag_bare = 0;
+        }
+    }
     build_classes(out, h);
     build_bounds(out, h, QMBX_PART_FWD);
     build_bounds(out, h, QMBX_PART_DIAG);
