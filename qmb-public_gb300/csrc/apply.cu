@@ -126,6 +126,7 @@ __device__ __forceinline__ void comp_cmul_add(CompSum& re, CompSum& im, float4 c
 template <int W, bool CONJ>
 struct GatherF64 : VisitorBase {
     static constexpr bool kTiledDense = true;
+    static constexpr bool kWordFilter = true;
     HashView lookup;         // hash set over the unique keys of the looked-up row set
     const double2* val;      // one amplitude per unique looked-up key
     const double2* coef;     // coefficients of the walked part
@@ -133,6 +134,8 @@ struct GatherF64 : VisitorBase {
     const int32_t* unique;   // walk index -> first row of the walked key
     double2* res;            // result per first row of the walked side
     HitLog log;              // optional record of the hits (for the adjoint without a walk)
+    const uint8_t* reach;    // words to share, per walk index (NULL: every term is looked up)
+    int self;                // the walked set is the looked-up set: a row finds itself
     struct Acc {
         double re, im, dre, dim;
         int row;
@@ -192,7 +195,7 @@ struct GatherF64 : VisitorBase {
     }
     __device__ __forceinline__ void finish(Acc& a, int64_t u, const Key<W>& c) const {
         if (a.dre != 0.0 || a.dim != 0.0) {
-            int64_t pos = hash_find<W>(lookup, c);
+            const int64_t pos = self ? (int64_t)a.row : hash_find<W>(lookup, c);
             if (pos >= 0) log_diag(log, u, a.row, pos, a.dre, CONJ ? -a.dim : a.dim);
             if (pos >= 0) {
                 double2 p = __ldg(val + pos);
@@ -214,6 +217,7 @@ struct GatherF64 : VisitorBase {
 template <int W, bool CONJ>
 struct GatherF32C : VisitorBase {
     static constexpr bool kTiledDense = true;
+    static constexpr bool kWordFilter = true;
     HashView lookup;
     const float2* val;
     const float4* coef32;
@@ -222,6 +226,8 @@ struct GatherF32C : VisitorBase {
     const int32_t* unique;
     double2* res;
     HitLog log;
+    const uint8_t* reach;    // words to share, per walk index (NULL: every term is looked up)
+    int self;                // the walked set is the looked-up set: a row finds itself
     struct Acc {
         CompSum re, im, dre, dim;
         int row;
@@ -272,7 +278,7 @@ struct GatherF32C : VisitorBase {
         double re = a.re.value(), im = a.im.value();
         const double dre = a.dre.value(), dim = a.dim.value();
         if (include_diag && (dre != 0.0 || dim != 0.0)) {
-            int64_t pos = hash_find<W>(lookup, c);
+            const int64_t pos = self ? (int64_t)a.row : hash_find<W>(lookup, c);
             if (pos >= 0) log_diag(log, u, a.row, pos, dre, CONJ ? -dim : dim);
             if (pos >= 0) {
                 float2 p = __ldg(val + pos);
@@ -324,6 +330,7 @@ struct DiagonalF64 : VisitorBase {
 template <int W, bool CONJ, bool F32>
 struct Scatter : VisitorBase {
     static constexpr bool kTiledDense = true;
+    static constexpr bool kWordFilter = true;
     HashView lookup;        // output-side row set
     const void* val;        // amplitude per first row of the walked side (double2, or float2 for F32)
     const int32_t* unique;  // walk index -> first row of the walked key
@@ -334,6 +341,7 @@ struct Scatter : VisitorBase {
     int include_diag;
     double2* acc;           // per unique output-side key
     HitLog log;
+    const uint8_t* reach;    // words to share, per walk index (NULL: every term is looked up)
     struct Acc {
         double2 p;
         double dre, dim;    // FP64 path
@@ -518,6 +526,7 @@ struct DiagAdd : VisitorBase {
     const float4* dcoef32;   // F32 path (hi/lo)
     double2* res;
     HitLog log;
+    int self;                // the walked set is the looked-up set: a row finds itself
     struct Acc {
         double dre, dim;     // FP64 path
         CompSum fre, fim;    // F32 path
@@ -563,7 +572,7 @@ struct DiagAdd : VisitorBase {
             a.dim = a.fim.value();
         }
         if (a.dre == 0.0 && a.dim == 0.0) return;
-        const int64_t pos = hash_find<W>(lookup, c);
+        const int64_t pos = self ? (int64_t)__ldg(unique + u) : hash_find<W>(lookup, c);
         if (pos < 0) return;
         log_diag(log, u, __ldg(unique + u), pos, a.dre, a.dim);
         const int64_t from = SCATTER ? (int64_t)__ldg(unique + u) : pos;
@@ -729,6 +738,13 @@ int launch_walk(const V& v, const HashRows& walk, const PartView& part, const Pa
     if (choose_walk(part, walk.n, false) == Walk::kGrouped) {
         QMBX_KERNEL(group, s, grouped_kernel<W><<<grouped_grid(walk.n), kThreads, 0, s>>>(v, src, walk.count, walk.n, part, diag));
     } else {
+        if constexpr (V::kWordFilter && W > 1) {
+            if (v.reach != nullptr) {
+                QMBX_KERNEL(group, s, enumerate_reach_kernel<W><<<grid_for(walk.n, kThreads), kThreads, 0, s>>>(v, src, walk.count, walk.n, part, diag));
+                QMBX_LAUNCH_CHECK("apply_within enumeration");
+                return QMBX_OK;
+            }
+        }
         if constexpr (V::kTiledDense && W <= 2) {
             QMBX_KERNEL(group, s, enumerate_dense_kernel<W><<<grid_for(walk.n, kThreads), kThreads, 0, s>>>(v, src, walk.count, walk.n, part, diag));
         } else {
@@ -776,10 +792,12 @@ PartView walk_part_of(const ApplyArgs& a, bool scatter) {
 // (gather walks assign their rows' sums; scatter and pivot walks add, so the
 // caller clears res for them).  rows_gate (device int, or NULL): the walked
 // rows are the first *rows_gate of the walked set, so a launch can be made
-// conditional on device state without a host round trip.
+// conditional on device state without a host round trip.  reach (or NULL):
+// the walked rows' flags for a tiled walk (enumerate_reach_kernel).
 template <int W>
 int walk_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_set, const void* val, double2* res,
-               const int* rows_gate, cudaStream_t s, int group = kGroupEnumerate, int diag_group = kGroupDiagonal) {
+               const int* rows_gate, const uint8_t* reach, cudaStream_t s, int group = kGroupEnumerate,
+               int diag_group = kGroupDiagonal) {
     const int64_t n_in = a.adjoint ? a.n_j : a.n_i;
     const int64_t n_out = a.adjoint ? a.n_i : a.n_j;
     int st = QMBX_OK;
@@ -810,7 +828,7 @@ int walk_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_s
 #define QMBX_PIVOT_CASE(CONJ, F32, SCATTER)                                                                      \
     {                                                                                                            \
         PivotHits<W, CONJ, F32, SCATTER> v{{}, look, val, walk.unique, part.coef, part.coef32, res}; v.log = a.log;             \
-        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res}; dv.log = a.log;                           \
+        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res}; dv.log = a.log; dv.self = a.same;                           \
         st = launch_pivot<W>(v, dv, walk, part, diag, s, group, diag_group);                                                        \
     }
         const bool f32 = a.prec == Prec::F32C;
@@ -831,36 +849,36 @@ int walk_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_s
     } else if (scatter) {
         if (a.prec == Prec::F64) {
             if (a.adjoint) {
-                Scatter<W, true, false> v{{}, look, val, walk.unique, part.coef, part.coef32, diag.coef, diag.coef32, 1, res}; v.log = a.log;
+                Scatter<W, true, false> v{{}, look, val, walk.unique, part.coef, part.coef32, diag.coef, diag.coef32, 1, res}; v.log = a.log; v.reach = reach;
                 st = launch_walk<W>(v, walk, part, walk_diag, s, group);
             } else {
-                Scatter<W, false, false> v{{}, look, val, walk.unique, part.coef, part.coef32, diag.coef, diag.coef32, 1, res}; v.log = a.log;
+                Scatter<W, false, false> v{{}, look, val, walk.unique, part.coef, part.coef32, diag.coef, diag.coef32, 1, res}; v.log = a.log; v.reach = reach;
                 st = launch_walk<W>(v, walk, part, walk_diag, s, group);
             }
         } else {
             if (a.adjoint) {
-                Scatter<W, true, true> v{{}, look, val, walk.unique, part.coef, part.coef32, diag.coef, diag.coef32, include_diag, res}; v.log = a.log;
+                Scatter<W, true, true> v{{}, look, val, walk.unique, part.coef, part.coef32, diag.coef, diag.coef32, include_diag, res}; v.log = a.log; v.reach = reach;
                 st = launch_walk<W>(v, walk, part, walk_diag, s, group);
             } else {
-                Scatter<W, false, true> v{{}, look, val, walk.unique, part.coef, part.coef32, diag.coef, diag.coef32, include_diag, res}; v.log = a.log;
+                Scatter<W, false, true> v{{}, look, val, walk.unique, part.coef, part.coef32, diag.coef, diag.coef32, include_diag, res}; v.log = a.log; v.reach = reach;
                 st = launch_walk<W>(v, walk, part, walk_diag, s, group);
             }
         }
     } else {
         if (a.prec == Prec::F64) {
             if (a.adjoint) {
-                GatherF64<W, true> v{{}, look, (const double2*)val, part.coef, diag.coef, walk.unique, res}; v.log = a.log;
+                GatherF64<W, true> v{{}, look, (const double2*)val, part.coef, diag.coef, walk.unique, res}; v.log = a.log; v.reach = reach; v.self = a.same;
                 st = launch_walk<W>(v, walk, part, walk_diag, s, group);
             } else {
-                GatherF64<W, false> v{{}, look, (const double2*)val, part.coef, diag.coef, walk.unique, res}; v.log = a.log;
+                GatherF64<W, false> v{{}, look, (const double2*)val, part.coef, diag.coef, walk.unique, res}; v.log = a.log; v.reach = reach; v.self = a.same;
                 st = launch_walk<W>(v, walk, part, walk_diag, s, group);
             }
         } else {
             if (a.adjoint) {
-                GatherF32C<W, true> v{{}, look, (const float2*)val, part.coef32, diag.coef32, a.include_diag, walk.unique, res}; v.log = a.log;
+                GatherF32C<W, true> v{{}, look, (const float2*)val, part.coef32, diag.coef32, a.include_diag, walk.unique, res}; v.log = a.log; v.reach = reach; v.self = a.same;
                 st = launch_walk<W>(v, walk, part, walk_diag, s, group);
             } else {
-                GatherF32C<W, false> v{{}, look, (const float2*)val, part.coef32, diag.coef32, a.include_diag, walk.unique, res}; v.log = a.log;
+                GatherF32C<W, false> v{{}, look, (const float2*)val, part.coef32, diag.coef32, a.include_diag, walk.unique, res}; v.log = a.log; v.reach = reach; v.self = a.same;
                 st = launch_walk<W>(v, walk, part, walk_diag, s, group);
             }
         }
@@ -870,7 +888,7 @@ int walk_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_s
         const bool f32 = a.prec == Prec::F32C;
 #define QMBX_DIAG_CASE(CONJ, F32, SCATTER)                                              \
     {                                                                                   \
-        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res}; dv.log = a.log;  \
+        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res}; dv.log = a.log; dv.self = a.same;  \
         st = launch_diag<W>(dv, walk, diag, s, diag_group);                                   \
     }
         if (scatter) {
@@ -922,7 +940,7 @@ int pair_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_s
     const HashView look = scatter ? out_set.hash() : in_set.hash();
 #define QMBX_DIAG_CASE(CONJ, F32, SCATTER)                                                                      \
     {                                                                                                           \
-        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res, a.log};      \
+        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res, a.log, a.same};      \
         st = launch_diag<W>(dv, walk, diag, s, diag_group);                                                \
     }
     if (scatter) {
@@ -952,6 +970,13 @@ bool take_pairs_behind(const ApplyArgs& a, const Arena& ws, uint64_t base, PairW
     rest.used = base;
     pairs = take_pair_work<W>(rest, a.n_i, a.n_j, a.same, h->n_sites);
     return rest.fits();
+}
+
+// Whether a call has scratch for Reach: tables of few terms (their walks are
+// tiled) over enough rows to outweigh building it, 1,000,000 rows of two words
+// take 35 us, their walk 1.12 ms without and 0.31 ms with it.
+bool reach_scratch(const qmbx_table_header* h, int64_t n_i, int64_t n_j) {
+    return h->n_words > 1 && h->part[QMBX_PART_FWD].n < kGroupedMinTerms && n_i >= kFewWideRows && n_j >= kFewWideRows;
 }
 
 // Forward maps amplitudes on configs_i (input side) to configs_j (output
@@ -1012,10 +1037,24 @@ int apply_impl(const ApplyArgs& a, Arena& ws, cudaStream_t s) {
     const HashRows& walked = scatter ? in_set : out_set;
     PairWork pairs{};
     bool scan = pairs_wanted(h, a.n_i, a.n_j);
-    if (scan) {
-        uint64_t needed = 0, with_pairs = 0;
-        if ((st = apply_within_workspace_for(a.table_host, a.n_i, a.n_j, a.same, &needed, &with_pairs)) != QMBX_OK) return st;
-        scan = take_pairs_behind<W>(a, ws, needed, pairs);
+    const uint8_t* reach = nullptr;
+    const bool reaching = reach_scratch(h, a.n_i, a.n_j) && choose_walk(walk_part_of(a, scatter), walked.n, true) == Walk::kTiled;
+    if (scan || reaching) {
+        // optional scratch lies behind what every call needs: the pair scan's, then the reach of tiled walks
+        uint64_t needed = 0, most = 0;
+        if ((st = apply_within_workspace_for(a.table_host, a.n_i, a.n_j, a.same, &needed, &most)) != QMBX_OK) return st;
+        if (scan) {
+            scan = take_pairs_behind<W>(a, ws, needed, pairs);
+        } else if (W > 1) {
+            Arena rest = ws;
+            rest.used = needed;
+            if (pairs_scratch(h, a.n_i, a.n_j)) take_pair_work<W>(rest, a.n_i, a.n_j, a.same, h->n_sites);
+            const Reach r = take_reach<W>(rest, walked.n, scatter ? out_set.n : in_set.n);
+            if (rest.fits()) {
+                if ((st = build_reach<W>(walked, scatter ? out_set : in_set, a.same, r, s)) != QMBX_OK) return st;
+                reach = r.flags;
+            }
+        }
     }
     if (scan && ((st = build_pairs<W>(rs_i, rs_j, h->n_sites, pairs, s)) != QMBX_OK ||
                  (st = choose_pairs<W>(pairs, walked, s)) != QMBX_OK)) {
@@ -1033,7 +1072,7 @@ int apply_impl(const ApplyArgs& a, Arena& ws, cudaStream_t s) {
     }
     // the device chooses one of the two; the other finds no rows
     if (scan && (st = pair_apply<W>(a, in_set, out_set, pairs, val, res, pairs.gate, s)) != QMBX_OK) return st;
-    if ((st = walk_apply<W>(a, in_set, out_set, val, res, scan ? pairs.gate + 1 : nullptr, s,
+    if ((st = walk_apply<W>(a, in_set, out_set, val, res, scan ? pairs.gate + 1 : nullptr, reach, s,
                             scan ? kGroupOther : kGroupEnumerate, scan ? kGroupOther : kGroupDiagonal)) != QMBX_OK) {
         return st;
     }
@@ -1106,9 +1145,9 @@ namespace qmbx {
 // Workspace of an apply_within call on n_i x n_j rows, for one value of
 // same_configs (one row set instead of two when it is set): the largest of
 // the forward / adjoint, FP64 / FP32 layouts (they differ by one value array),
-// and the same with the pair scan's scratch behind it.
+// and the same with the optional scratch behind it.
 int apply_within_workspace_for(const void* table_host, int64_t n_i, int64_t n_j, bool same, uint64_t* needed,
-                               uint64_t* with_pairs) {
+                               uint64_t* most) {
     const qmbx_table_header* h = header_of(table_host);
     if (h == nullptr || h->magic != QMBX_MAGIC) return fail(QMBX_ERR_ARGUMENT, "not a compiled qmbx table");
     ApplyArgs a{};
@@ -1117,25 +1156,36 @@ int apply_within_workspace_for(const void* table_host, int64_t n_i, int64_t n_j,
     a.n_j = same ? n_i : n_j;
     a.same = same;
     a.prec = Prec::F64;
-    uint64_t most = 0;
+    uint64_t base = 0;
     for (int adj = 0; adj < 2; ++adj) {
         a.adjoint = adj != 0;
         Arena probe(nullptr, 0);
         int st = dispatch_apply(a, probe, nullptr);
         if (st != QMBX_OK) return st;
-        if (probe.used > most) most = probe.used;
+        if (probe.used > base) base = probe.used;
     }
-    *needed = *with_pairs = most;
+    *needed = *most = base;
     if (pairs_scratch(h, a.n_i, a.n_j)) {
         Arena rest(nullptr, 0);
-        rest.used = most;
+        rest.used = base;
         switch (h->n_words) {
             case 1: take_pair_work<1>(rest, a.n_i, a.n_j, same, h->n_sites); break;
             case 2: take_pair_work<2>(rest, a.n_i, a.n_j, same, h->n_sites); break;
             case 3: take_pair_work<3>(rest, a.n_i, a.n_j, same, h->n_sites); break;
             default: take_pair_work<4>(rest, a.n_i, a.n_j, same, h->n_sites); break;
         }
-        *with_pairs = rest.used;
+        *most = rest.used;
+    }
+    if (reach_scratch(h, a.n_i, a.n_j)) {
+        Arena rest(nullptr, 0);
+        rest.used = *most;
+        const int64_t rows = a.n_i > a.n_j ? a.n_i : a.n_j;
+        switch (h->n_words) {
+            case 2: take_reach<2>(rest, rows, rows); break;
+            case 3: take_reach<3>(rest, rows, rows); break;
+            default: take_reach<4>(rest, rows, rows); break;
+        }
+        *most = rest.used;
     }
     return QMBX_OK;
 }
@@ -1537,7 +1587,7 @@ int adjoint_from_log_impl(const void* table_host, const void* table_dev, char* b
     }
     QMBX_LAUNCH_CHECK("adjoint from log");
     // an incomplete record: the adjoint walk (its walked rows gated by the device count; 0 otherwise)
-    int st = walk_apply<W>(a, rs_j, rs_i, g, res, &gate->rows, s, kGroupSpmv, kGroupSpmv);
+    int st = walk_apply<W>(a, rs_j, rs_i, g, res, &gate->rows, nullptr, s, kGroupSpmv, kGroupSpmv);
     if (st != QMBX_OK) return st;
     // or the scan again, over the prepared rows the forward left in the buffer
     if (scan) {

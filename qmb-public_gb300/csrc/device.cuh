@@ -264,10 +264,10 @@ inline PartView part_view(const void* table_host, const void* table_dev, int whi
 int check_table(const void* table_host, const void* table_dev);
 
 // Workspace of an apply_within call for one value of same_configs (apply.cu): the part every call
-// needs, and with the pair scan's scratch behind it where the sizes give it one (calls with less
-// workspace walk the terms instead).
+// needs, and with the scratch of the pair scan and of reach-bounded walks behind it where the sizes
+// give them one (calls with less workspace walk the terms without).
 int apply_within_workspace_for(const void* table_host, int64_t n_i, int64_t n_j, bool same, uint64_t* needed,
-                               uint64_t* with_pairs);
+                               uint64_t* most);
 
 // ---------------------------------------------------------------------------
 // the enumeration kernel: every (configuration, term) pair of one or two
@@ -321,6 +321,60 @@ __device__ __forceinline__ int term_image(const uint64_t* t, const Key<W>& c, Ke
         par += __popcll(c.w[q] & t[4 * q + 3]);
     }
     return par & 1;
+}
+
+// One term record in registers (loaded with 16-byte vector loads).
+template <int W>
+struct TermRec {
+    uint64_t m[4 * W];
+    __device__ __forceinline__ bool applies(const Key<W>& c) const {
+        uint64_t bad = 0;
+#pragma unroll
+        for (int q = 0; q < W; ++q) bad |= (c.w[q] ^ m[4 * q + 1]) & m[4 * q];
+        return bad == 0;
+    }
+    __device__ __forceinline__ int image(const Key<W>& c, Key<W>& img) const {
+        int par = 0;
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+            img.w[q] = c.w[q] ^ m[4 * q + 2];
+            par += __popcll(c.w[q] & m[4 * q + 3]);
+        }
+        return par & 1;
+    }
+};
+
+// The test pair of every word of term t (into m[4q], m[4q + 1]).
+template <int W>
+__device__ __forceinline__ void load_test(TermRec<W>& r, const PartView& pv, int64_t t) {
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+        const ulonglong2 v = __ldg(pv.test + (int64_t)q * pv.stride + t);
+        r.m[4 * q] = v.x;
+        r.m[4 * q + 1] = v.y;
+    }
+}
+
+// The apply pair of every word of term t (into m[4q + 2], m[4q + 3]).
+template <int W>
+__device__ __forceinline__ void load_apply(TermRec<W>& r, const PartView& pv, int64_t t) {
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+        const ulonglong2 v = __ldg(pv.apply + (int64_t)q * pv.stride + t);
+        r.m[4 * q + 2] = v.x;
+        r.m[4 * q + 3] = v.y;
+    }
+}
+
+// The whole record of term t from its narrow form (one 16-byte load; the
+// part must have one: W == 1 and pv.narrow set).
+template <int W>
+__device__ __forceinline__ void load_narrow(TermRec<W>& r, const PartView& pv, int64_t t) {
+    const uint4 q = __ldg(pv.narrow + t);
+    r.m[0] = (uint64_t)q.x << 32;
+    r.m[1] = (uint64_t)q.y << 32;
+    r.m[2] = (uint64_t)q.z << 32;
+    r.m[3] = (uint64_t)q.w << 32;
 }
 
 // Row sources of the enumeration kernel: packed keys, or raw rows packed on the fly.
@@ -422,6 +476,7 @@ struct VisitorBase {
     __device__ __forceinline__ void flush(Acc&, int64_t, const K&) const {}
     static constexpr int kShared = 0;
     static constexpr bool kTiledDense = false;  // tiled walks may run as enumerate_dense_kernel (W <= 2)
+    static constexpr bool kWordFilter = false;  // has `reach` (walks of looked-up images only): see enumerate_reach_kernel
     static constexpr bool kBatched = false;  // hits are queued and processed by apply_hit with full lanes
     static constexpr bool kStateless = false; // pivot walks: hits carry their row and need no per-row state
     template <class Acc>
@@ -517,6 +572,100 @@ __global__ void __launch_bounds__(kThreads, 5) enumerate_dense_kernel(V v, Src s
     enumerate_rows<W>(v, src, n_rows, n_max, off, diag);
 }
 
+// The tiled walk with terms left out that cannot lead to a looked-up row.  A
+// term that changes one key word only leaves the others as they are, so its
+// image can be in the looked-up set only if a row there has the same other
+// words; v.reach holds, per walked row, a bit for every word of which that is
+// so (build_reach).  A block stages only the terms that one of its rows
+// needs, and a row looks up only those it needs.  On a lattice of 128 sites
+// over two words, random rows share no half, and only the hops between the
+// halves (32 of 448) are left to test and to look up.
+// (Visitors with kWordFilter and keys of two words or more.)
+template <int W, class V, class Src>
+__global__ void __launch_bounds__(kThreads) enumerate_reach_kernel(V v, Src src, const int* __restrict__ n_rows,
+                                                                   int64_t n_max, PartView off, PartView diag) {
+    __shared__ __align__(16) uint64_t s_term[kThreads][4 * W];  // a thread stages a term
+    __shared__ int s_slot[kThreads];
+    __shared__ uint8_t s_bit[kThreads];  // the word bit a staged term asks for (0: none)
+    __shared__ unsigned s_need;
+    __shared__ int s_count[kThreads / 32];
+    const int64_t n = n_rows ? (int64_t)*n_rows : n_max;
+    if ((int64_t)blockIdx.x * blockDim.x >= n) return;
+    const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = row < n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Key<W> c;
+    unsigned need = 0;
+    typename V::Acc acc;
+    if (live) {
+        c = src.get(row);
+        need = __ldg(v.reach + row);
+        v.init(acc, row, c, nullptr);
+    } else {
+#pragma unroll
+        for (int q = 0; q < W; ++q) c.w[q] = 0;
+    }
+    if (threadIdx.x == 0) s_need = 0;
+    __syncthreads();
+    const unsigned any = __reduce_or_sync(0xffffffffu, need);
+    if (lane == 0 && any != 0) atomicOr(&s_need, any);
+    __syncthreads();
+    const unsigned block_need = s_need;
+    for (int part = 0; part < 2; ++part) {
+        const PartView& pv = part == 0 ? off : diag;
+        for (int64_t t0 = 0; t0 < pv.n; t0 += kThreads) {
+            const int64_t t = t0 + threadIdx.x;
+            const bool in = t < pv.n;
+            TermRec<W> rec;
+            unsigned changed = 0;
+            if (in) {
+                load_test<W>(rec, pv, t);
+                load_apply<W>(rec, pv, t);
+#pragma unroll
+                for (int q = 0; q < W; ++q) changed |= rec.m[4 * q + 2] != 0 ? 1u << q : 0u;
+            }
+            const unsigned bit = (changed & (changed - 1)) == 0 ? changed : 0u;
+            const bool keep = in && (bit == 0 || (bit & block_need) != 0);
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            __syncthreads();  // the last tile has been read
+            if (lane == 0) s_count[warp] = __popc(m);
+            __syncthreads();
+            int count = 0, before = 0;
+#pragma unroll
+            for (int w = 0; w < kThreads / 32; ++w) {
+                if (w < warp) before += s_count[w];
+                count += s_count[w];
+            }
+            if (keep) {
+                const int at = before + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+                for (int q = 0; q < 4 * W; ++q) s_term[at][q] = rec.m[q];
+                s_slot[at] = (int)t;
+                s_bit[at] = (uint8_t)bit;
+            }
+            __syncthreads();
+            if (!live) continue;
+            for (int k0 = 0; k0 < count; k0 += 32) {
+                uint32_t hit = 0;
+                for (int b = 0; b < 32 && k0 + b < count; ++b) hit |= (uint32_t)term_applies<W>(s_term[k0 + b], c) << b;
+                while (hit) {
+                    const int k = k0 + __ffs(hit) - 1;
+                    hit &= hit - 1;
+                    if (s_bit[k] != 0 && (s_bit[k] & need) == 0) continue;
+                    Key<W> img;
+                    const int parity = term_image<W>(s_term[k], c, img);
+                    if (part == 0) {
+                        v.visit(acc, c, img, parity, s_slot[k]);
+                    } else {
+                        v.visit_diag(acc, c, parity, s_slot[k]);
+                    }
+                }
+            }
+        }
+    }
+    if (live) v.finish(acc, row, c);
+}
+
 // The tiled walk of a diagonal part with each row shared by L lanes (lane
 // group g = threadIdx.x / L of the block): lane s of a group tests terms s,
 // s + L, ... of every staged tile, the group's sums are combined with
@@ -580,60 +729,6 @@ constexpr int kWarpsPerBlock = kThreads / 32;
 
 // Parts with at least this many terms are walked by grouped_kernel.
 constexpr int64_t kGroupedMinTerms = 2048;
-
-// One term record in registers (loaded with 16-byte vector loads).
-template <int W>
-struct TermRec {
-    uint64_t m[4 * W];
-    __device__ __forceinline__ bool applies(const Key<W>& c) const {
-        uint64_t bad = 0;
-#pragma unroll
-        for (int q = 0; q < W; ++q) bad |= (c.w[q] ^ m[4 * q + 1]) & m[4 * q];
-        return bad == 0;
-    }
-    __device__ __forceinline__ int image(const Key<W>& c, Key<W>& img) const {
-        int par = 0;
-#pragma unroll
-        for (int q = 0; q < W; ++q) {
-            img.w[q] = c.w[q] ^ m[4 * q + 2];
-            par += __popcll(c.w[q] & m[4 * q + 3]);
-        }
-        return par & 1;
-    }
-};
-
-// The test pair of every word of term t (into m[4q], m[4q + 1]).
-template <int W>
-__device__ __forceinline__ void load_test(TermRec<W>& r, const PartView& pv, int64_t t) {
-#pragma unroll
-    for (int q = 0; q < W; ++q) {
-        const ulonglong2 v = __ldg(pv.test + (int64_t)q * pv.stride + t);
-        r.m[4 * q] = v.x;
-        r.m[4 * q + 1] = v.y;
-    }
-}
-
-// The apply pair of every word of term t (into m[4q + 2], m[4q + 3]).
-template <int W>
-__device__ __forceinline__ void load_apply(TermRec<W>& r, const PartView& pv, int64_t t) {
-#pragma unroll
-    for (int q = 0; q < W; ++q) {
-        const ulonglong2 v = __ldg(pv.apply + (int64_t)q * pv.stride + t);
-        r.m[4 * q + 2] = v.x;
-        r.m[4 * q + 3] = v.y;
-    }
-}
-
-// The whole record of term t from its narrow form (one 16-byte load; the
-// part must have one: W == 1 and pv.narrow set).
-template <int W>
-__device__ __forceinline__ void load_narrow(TermRec<W>& r, const PartView& pv, int64_t t) {
-    const uint4 q = __ldg(pv.narrow + t);
-    r.m[0] = (uint64_t)q.x << 32;
-    r.m[1] = (uint64_t)q.y << 32;
-    r.m[2] = (uint64_t)q.z << 32;
-    r.m[3] = (uint64_t)q.w << 32;
-}
 
 // Hits of batched visitors wait in a per-warp shared queue until 32 have
 // gathered, then every lane processes one: the floating-point work of a hit
@@ -1356,6 +1451,26 @@ int build_hashrows(const uint8_t* rows, int n_qubytes, HashRows& out, cudaStream
 // are only looked up (hash()).
 template <int W>
 int build_hashset(const uint8_t* rows, int n_qubytes, HashRows& out, cudaStream_t s);
+
+// For walks of few terms over many rows of two or more key words
+// (enumerate_reach_kernel): which words a walked row shares with the looked-up
+// rows but for one.  Blocked Bloom filters over the rows with one word left
+// out, four bits in one of 64 and 32 filter bits a row: a row that shares
+// nothing is taken for one that does with a probability of about 3e-4, which
+// costs lookups only.
+struct Reach {
+    unsigned long long* once;   // [W][words]: rows of the looked-up set
+    unsigned long long* twice;  // [W][words]: rows that found all their bits set
+    uint8_t* flags;             // per walk index: a bit for every word
+    uint64_t words;             // a power of two
+};
+
+template <int W>
+Reach take_reach(Arena& ws, int64_t n_walk, int64_t n_look);
+
+// same: the walked set is the looked-up set (a row shares with another one)
+template <int W>
+int build_reach(const HashRows& walk, const HashRows& look, bool same, const Reach& r, cudaStream_t s);
 
 // Rows of a HashRows set visited by the enumeration kernels: walk index u
 // is the u-th unique row.

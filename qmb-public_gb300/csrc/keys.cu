@@ -285,9 +285,79 @@ int build_hashrows(const uint8_t* rows, int nq, HashRows& out, cudaStream_t s) {
     return QMBX_OK;
 }
 
+// ---------------------------------------------------------------------------
+// rows that share all key words but one (Reach)
+// ---------------------------------------------------------------------------
+
+template <int W>
+__device__ __forceinline__ void reach_place(Key<W> k, int left_out, uint64_t words, uint64_t& at, unsigned long long& bits) {
+#pragma unroll
+    for (int q = 0; q < W; ++q) k.w[q] = q == left_out ? (uint64_t)(q + 1) : k.w[q];
+    const uint64_t f = bloom_mix(key_hash<W>(k));
+    at = (f >> 40) & (words - 1);
+    bits = (1ull << ((f >> 8) & 63)) | (1ull << ((f >> 14) & 63)) | (1ull << ((f >> 20) & 63)) | (1ull << ((f >> 26) & 63));
+}
+
+template <int W>
+__global__ void reach_insert_kernel(const uint64_t* __restrict__ keys, const int32_t* __restrict__ unique,
+                                    const int* __restrict__ count, Reach r) {
+    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= *count) return;
+    const Key<W> k = load_key<W>(keys, __ldg(unique + u));
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+        uint64_t at;
+        unsigned long long bits;
+        reach_place<W>(k, w, r.words, at, bits);
+        const unsigned long long old = atomicOr(r.once + w * r.words + at, bits);
+        if ((old & bits) == bits) atomicOr(r.twice + w * r.words + at, bits);
+    }
+}
+
+template <int W>
+__global__ void reach_flags_kernel(const uint64_t* __restrict__ keys, const int32_t* __restrict__ unique,
+                                   const int* __restrict__ count, int same, Reach r) {
+    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= *count) return;
+    const Key<W> k = load_key<W>(keys, __ldg(unique + u));
+    unsigned flags = 0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+        uint64_t at;
+        unsigned long long bits;
+        reach_place<W>(k, w, r.words, at, bits);
+        const unsigned long long have = __ldg((same ? r.twice : r.once) + w * r.words + at);
+        if ((have & bits) == bits) flags |= 1u << w;
+    }
+    r.flags[u] = (uint8_t)flags;
+}
+
+template <int W>
+Reach take_reach(Arena& ws, int64_t n_walk, int64_t n_look) {
+    Reach r{};
+    r.words = 1024;
+    while (r.words * 2 < (uint64_t)(n_look > 0 ? n_look : 1) && r.words < (1ull << 24)) r.words <<= 1;
+    r.once = ws.take<unsigned long long>(r.words * W);
+    r.twice = ws.take<unsigned long long>(r.words * W);
+    r.flags = ws.take<uint8_t>((uint64_t)(n_walk > 0 ? n_walk : 1));
+    return r;
+}
+
+template <int W>
+int build_reach(const HashRows& walk, const HashRows& look, bool same, const Reach& r, cudaStream_t s) {
+    QMBX_CUDA_TRY(cudaMemsetAsync(r.once, 0, (size_t)r.words * W * sizeof(unsigned long long), s));
+    QMBX_CUDA_TRY(cudaMemsetAsync(r.twice, 0, (size_t)r.words * W * sizeof(unsigned long long), s));
+    QMBX_KERNEL(kGroupKeys, s, reach_insert_kernel<W><<<grid_for(look.n, kThreads), kThreads, 0, s>>>(look.keys, look.unique, look.count, r));
+    QMBX_KERNEL(kGroupKeys, s, reach_flags_kernel<W><<<grid_for(walk.n, kThreads), kThreads, 0, s>>>(walk.keys, walk.unique, walk.count, same ? 1 : 0, r));
+    QMBX_LAUNCH_CHECK("build_reach");
+    return QMBX_OK;
+}
+
 #define QMBX_INSTANTIATE_KEYS(W)                                                          \
     template int pack_rows<W>(const uint8_t*, int64_t, int, uint64_t*, cudaStream_t);     \
     template HashRows take_hashrows<W>(Arena&, int64_t);                                  \
+    template Reach take_reach<W>(Arena&, int64_t, int64_t);                               \
+    template int build_reach<W>(const HashRows&, const HashRows&, bool, const Reach&, cudaStream_t); \
     template int build_hashset<W>(const uint8_t*, int, HashRows&, cudaStream_t);          \
     template int build_hashrows<W>(const uint8_t*, int, HashRows&, cudaStream_t);
 

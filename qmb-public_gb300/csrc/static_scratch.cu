@@ -73,8 +73,8 @@ extern "C" int qmbx_apply_within_static(const void* table_host, const void* tabl
                                         const double* psi_i, int64_t n_i, const uint8_t* configs_j, int64_t n_j,
                                         int32_t same_configs, double* psi_j, qmbx_stream_t stream) {
     qmbx::clear_error();
-    uint64_t need = 0, with_pairs = 0;
-    int st = qmbx::apply_within_workspace_for(table_host, n_i, n_j, same_configs != 0, &need, &with_pairs);
+    uint64_t need = 0, most = 0;
+    int st = qmbx::apply_within_workspace_for(table_host, n_i, n_j, same_configs != 0, &need, &most);
     if (st != QMBX_OK) return st;
     if (need > kStaticScratchBytes) {
         return qmbx::fail(QMBX_ERR_ARGUMENT,
