@@ -330,6 +330,16 @@ int qmbx_single_relative(const void* table_host, const void* table_dev, const ui
                          uint64_t seed, uint8_t* out, void* workspace, uint64_t workspace_bytes,
                          qmbx_stream_t stream);
 
+/* One iteration of the Lanczos recurrence on a matrix (qmb/rldiag.py:19-52),
+ * with its scalars on the device: w = A v, *alpha = Re<w, v>, w -= *alpha v +
+ * *beta_prev v_prev (v_prev and beta_prev NULL in the first iteration),
+ * *beta = |w|, v_next = w / *beta.  All vectors are complex double [n], the
+ * scalars device doubles; scratch holds 16 n + 40960 bytes, 256-byte aligned.
+ * Nothing waits for the device. */
+int qmbx_lanczos_step(int64_t n, const int64_t* row_ptr, const int32_t* col, const double* val, const double* v_prev,
+                      const double* beta_prev, const double* v, double* v_next, double* alpha, double* beta,
+                      void* scratch, uint64_t scratch_bytes, qmbx_stream_t stream);
+
 /* ---------------------------------------------------------------------------
  * The elementwise parts of the autoregressive network of qmb/mlp.py:60-314
  * (WaveFunctionElectronUpDown, the caller that samples the configurations

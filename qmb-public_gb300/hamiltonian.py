@@ -551,6 +551,14 @@ class HamiltonianMatrix:
                          self.val.data_ptr(), x.data_ptr(), y.data_ptr(), _stream(x.device))
         return y
 
+    def lanczos_step(self, v_prev: torch.Tensor | None, beta_prev: torch.Tensor | None, v: torch.Tensor,
+                     v_next: torch.Tensor, alpha: torch.Tensor, beta: torch.Tensor, scratch: torch.Tensor) -> None:
+        """One Lanczos iteration into v_next, alpha and beta (qmbx_lanczos_step), without waiting for the device."""
+        with torch.cuda.device(v.device):
+            _native.call("qmbx_lanczos_step", self.n, self.row_ptr.data_ptr(), self.col.data_ptr(), self.val.data_ptr(),
+                         _ptr(v_prev), _ptr(beta_prev), v.data_ptr(), v_next.data_ptr(), alpha.data_ptr(),
+                         beta.data_ptr(), scratch.data_ptr(), scratch.numel(), _stream(v.device))
+
     def to_dense(self) -> torch.Tensor:
         """The dense matrix (for checks on small row sets)."""
         rows = torch.repeat_interleave(torch.arange(self.n, device=self.val.device),

@@ -22,9 +22,11 @@ from __future__ import annotations
 
 import functools
 
+import numpy as np
 import scipy.linalg
 import torch
 
+from . import _native
 from .hamiltonian import Hamiltonian
 
 __all__ = ["lanczos_energy", "pt2_energy"]
@@ -49,8 +51,14 @@ def lanczos_energy(ham: Hamiltonian, configs: torch.Tensor, step: int, threshold
         start = torch.randn([configs.size(0)], dtype=torch.complex128, device=configs.device, generator=generator)
     apply = functools.partial(ham.apply_within, configs, configs_j=configs)
     if materialize and configs.is_cuda and configs.size(0) > 0:
-        mat = ham.matrix(configs, max_entries=_matrix_budget(configs.device)) \
-            if torch.unique(configs, dim=0).shape[0] == configs.shape[0] else None
+        try:
+            mat = ham.matrix(configs, max_entries=_matrix_budget(configs.device))
+        except _native.QmbxError as error:
+            if "must be distinct" not in str(error):
+                raise
+            mat = None  # repeated rows: every iteration walks the terms
+        if mat is not None and step >= 0:
+            return _lanczos_on_matrix(mat, start, step, threshold)
         if mat is not None:
             apply = mat.apply
     v = [start.to(torch.complex128) / torch.linalg.norm(start)]
@@ -74,10 +82,59 @@ def lanczos_energy(ham: Hamiltonian, configs: torch.Tensor, step: int, threshold
         i += 1
     if len(beta) == 0:
         return alpha[0].item(), v[0]
-    vals, vecs = scipy.linalg.eigh_tridiagonal(torch.stack(alpha).cpu().numpy(), torch.stack(beta).cpu().numpy(),
-                                               lapack_driver="stebz", select="i", select_range=(0, 0))
-    result = functools.reduce(torch.add, (float(weight[0]) * vector for weight, vector in zip(vecs, v)))
-    return float(vals[0]), result
+    value, weights = _lowest(torch.stack(alpha).cpu().numpy(), torch.stack(beta).cpu().numpy())
+    return value, functools.reduce(torch.add, (float(weight) * vector for weight, vector in zip(weights, v)))
+
+
+def _lowest(alpha, beta):
+    """Lowest eigenvalue and eigenvector of the tridiagonal matrix."""
+    vals, vecs = scipy.linalg.eigh_tridiagonal(alpha, beta, lapack_driver="stebz", select="i", select_range=(0, 0))
+    return float(vals[0]), vecs[:, 0]
+
+
+# iterations between two looks at beta on the host
+_LOOK_EVERY = 16
+
+
+def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
+    """The recurrence on a stored matrix: its scalars stay on the device, and the host looks for a norm
+    below the threshold once per block of iterations (what ran past it is dropped)."""
+    n, device = mat.n, start.device
+    if start.shape != (n,) or device != mat.val.device:
+        raise RuntimeError(f"start must have shape [{n}] and be on the matrix's device.")
+    scalars = torch.empty((2, step + 2), dtype=torch.float64, device=device)
+    alpha, beta = scalars[0], scalars[1]
+    scratch = torch.empty(16 * n + 40960, dtype=torch.uint8, device=device)
+    first = start.to(torch.complex128) / torch.linalg.norm(torch.view_as_real(start.to(torch.complex128)))
+    blocks = [first.reshape(1, n).contiguous()]
+    seen = []
+    v, v_prev, done, stop = blocks[0][0], None, 0, None
+    # iteration k forms alpha[k], beta[k] and vector k + 1; the last one's beta and vector are not used
+    while done < step + 2 and stop is None:
+        count = min(_LOOK_EVERY, step + 2 - done)
+        block = torch.empty((count, n), dtype=torch.complex128, device=device)
+        for k in range(done, done + count):
+            mat.lanczos_step(v_prev, beta[k - 1] if k else None, v, block[k - done], alpha[k], beta[k], scratch)
+            v_prev, v = v, block[k - done]
+        blocks.append(block)
+        host = scalars[:, done:done + count].cpu().numpy()
+        seen.append(host)
+        small = [k for k in range(done, done + count) if k < step + 1 and host[1, k - done] < threshold]
+        stop = small[0] if small else None
+        done += count
+    used = (step + 1 if stop is None else stop) + 1  # vectors 0 .. used - 1
+    host = np.concatenate(seen, axis=1)[:, :used]
+    if used == 1:
+        return float(host[0, 0]), blocks[0][0]
+    value, weights = _lowest(host[0], host[1, :used - 1])
+    result, at = torch.zeros(n, dtype=torch.complex128, device=device), 0
+    for block in blocks:
+        part = block[:max(0, used - at)]
+        if part.shape[0]:
+            weight = torch.from_numpy(weights[at:at + part.shape[0]].astype(np.complex128)).to(device)
+            result += weight @ part
+        at += block.shape[0]
+    return value, result
 
 
 def pt2_energy(ham: Hamiltonian, configs: torch.Tensor, psi: torch.Tensor, count_selected: int, *,
