@@ -62,6 +62,11 @@ struct CompSum {
         two_sum(s, hi, s, e);
         c = __fadd_rn(c, __fadd_rn(e, lo));
     }
+    __device__ __forceinline__ void merge(const CompSum& b) {
+        float e;
+        two_sum(s, b.s, s, e);
+        c = __fadd_rn(c, __fadd_rn(b.c, e));
+    }
     __device__ __forceinline__ double value() const { return (double)s + (double)c; }
     // Combine the lanes' pairs: two-sum of the leading parts, plain sum of the tails.
     __device__ __forceinline__ void warp_reduce() { group_reduce<32>(); }
@@ -193,6 +198,13 @@ struct GatherF64 : VisitorBase {
         a.dre = warp_sum(a.dre);
         a.dim = warp_sum(a.dim);
     }
+    static constexpr bool kMerges = true;
+    __device__ __forceinline__ void merge(Acc& a, const Acc& b) const {
+        a.re += b.re;
+        a.im += b.im;
+        a.dre += b.dre;
+        a.dim += b.dim;
+    }
     __device__ __forceinline__ void finish(Acc& a, int64_t u, const Key<W>& c) const {
         if (a.dre != 0.0 || a.dim != 0.0) {
             const int64_t pos = self ? (int64_t)a.row : hash_find<W>(lookup, c);
@@ -273,6 +285,13 @@ struct GatherF32C : VisitorBase {
         a.im.warp_reduce();
         a.dre.warp_reduce();
         a.dim.warp_reduce();
+    }
+    static constexpr bool kMerges = true;
+    __device__ __forceinline__ void merge(Acc& a, const Acc& b) const {
+        a.re.merge(b.re);
+        a.im.merge(b.im);
+        a.dre.merge(b.dre);
+        a.dim.merge(b.dim);
     }
     __device__ __forceinline__ void finish(Acc& a, int64_t u, const Key<W>& c) const {
         double re = a.re.value(), im = a.im.value();
@@ -433,6 +452,13 @@ struct Scatter : VisitorBase {
             a.dre = warp_sum(a.dre);
             a.dim = warp_sum(a.dim);
         }
+    }
+    static constexpr bool kMerges = true;
+    __device__ __forceinline__ void merge(Acc& a, const Acc& b) const {
+        a.dre += b.dre;
+        a.dim += b.dim;
+        a.fre.merge(b.fre);
+        a.fim.merge(b.fim);
     }
     __device__ __forceinline__ void finish(Acc& a, int64_t w, const Key<W>& c) const {
         const double dre = F32 ? a.fre.value() : a.dre, dim = F32 ? a.fim.value() : a.dim;
@@ -603,14 +629,18 @@ struct PairHits {
     const float4* coef32;
     double2* res;           // per first row of the output side
     HitLog log;
+    __device__ __forceinline__ bool recording() const { return log.hits != nullptr; }
+    // n (any number) hits about to be applied: one place in the record for all of them, since every
+    // warp's atomic meets the same counter
     __device__ __forceinline__ void record(const int4* q, int n, int lane) const {
         if (log.hits == nullptr || n <= 0) return;
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(log.count, (unsigned long long)n);
         base = __shfl_sync(0xffffffffu, base, 0);
-        if (lane < n && base + lane < (unsigned long long)log.cap) {
-            const int4 h = q[lane];
-            log.hits[base + lane] = make_int4(h.y, h.z, h.x, 0);
+        for (int k = lane; k < n; k += 32) {
+            if (base + k >= (unsigned long long)log.cap) break;
+            const int4 h = q[k];
+            log.hits[base + k] = make_int4(h.y, h.z, h.x, 0);
         }
     }
     __device__ __forceinline__ void apply(int4 h) const {
@@ -736,7 +766,17 @@ int launch_walk(const V& v, const HashRows& walk, const PartView& part, const Pa
                 int group = kGroupEnumerate) {
     UniqueRows<W> src{walk.keys, walk.unique};
     if (choose_walk(part, walk.n, false) == Walk::kGrouped) {
-        QMBX_KERNEL(group, s, grouped_kernel<W><<<grouped_grid(walk.n), kThreads, 0, s>>>(v, src, walk.count, walk.n, part, diag));
+        // (parts of small groups deal them 32 at a time to the lanes: a team of two took 43 us for 25)
+        const int team = V::kMerges && diag.n == 0 && part.wide ? team_size(walk.n) : 1;
+        if (team == 8) {
+            QMBX_KERNEL(group, s, grouped_team_kernel<W, 8><<<grid_for(walk.n, 1), kThreads, 0, s>>>(v, src, walk.count, walk.n, part));
+        } else if (team == 4) {
+            QMBX_KERNEL(group, s, grouped_team_kernel<W, 4><<<grid_for(walk.n, 2), kThreads, 0, s>>>(v, src, walk.count, walk.n, part));
+        } else if (team == 2) {
+            QMBX_KERNEL(group, s, grouped_team_kernel<W, 2><<<grid_for(walk.n, 4), kThreads, 0, s>>>(v, src, walk.count, walk.n, part));
+        } else {
+            QMBX_KERNEL(group, s, grouped_kernel<W><<<grouped_grid(walk.n), kThreads, 0, s>>>(v, src, walk.count, walk.n, part, diag));
+        }
     } else {
         if constexpr (V::kWordFilter && W > 1) {
             if (v.reach != nullptr) {

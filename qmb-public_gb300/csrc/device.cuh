@@ -477,6 +477,7 @@ struct VisitorBase {
     static constexpr int kShared = 0;
     static constexpr bool kTiledDense = false;  // tiled walks may run as enumerate_dense_kernel (W <= 2)
     static constexpr bool kWordFilter = false;  // has `reach` (walks of looked-up images only): see enumerate_reach_kernel
+    static constexpr bool kMerges = false;   // has merge(Acc&, const Acc&): grouped walks may share a row among warps
     static constexpr bool kBatched = false;  // hits are queued and processed by apply_hit with full lanes
     static constexpr bool kStateless = false; // pivot walks: hits carry their row and need no per-row state
     template <class Acc>
@@ -1088,6 +1089,46 @@ __global__ void __launch_bounds__(kThreads) grouped_kernel(V v, Src src, const i
     __syncthreads();
     v.block_flush(sh);
 }
+
+// The grouped walk with a row shared by a team of T warps of its block, for
+// batched visitors over too few rows to fill the GPU with a warp each: the
+// groups go to the warps in turn, and the team's first warp adds up the others'
+// sums (the visitor's merge) in a fixed order.  A warp's groups are a chain of
+// dependent reads: 400 rows under 1,819 terms 26.7 -> 18.4 us.
+template <int W, int T, class V, class Src>
+__global__ void __launch_bounds__(kThreads) grouped_team_kernel(V v, Src src, const int* __restrict__ n_rows,
+                                                                int64_t n_max, PartView off) {
+    static_assert(V::kBatched && V::kShared == 0, "teams serve batched visitors");
+    __shared__ int2 hitq[kWarpsPerBlock][64];
+    __shared__ uint64_t candkey[kWarpsPerBlock][cand_ring(W) * W];
+    __shared__ int candmeta[kWarpsPerBlock][cand_ring(W)];
+    __shared__ typename V::Acc team[kWarpsPerBlock];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t n = n_rows ? (int64_t)*n_rows : n_max;
+    const int64_t row = (int64_t)blockIdx.x * (kWarpsPerBlock / T) + warp / T;
+    const bool live = row < n;
+    Key<W> c{};
+    typename V::Acc acc;
+    if (live) {
+        c = src.get(row);
+        v.init(acc, row, c, nullptr);
+        HitQueue hq{hitq[warp], 0, candkey[warp], candmeta[warp], 0, 0};
+        walk_part<W, false>(v, acc, c, off, lane, hq, warp % T, T);
+        if (hq.ccount > 0) candidates_flush<W>(v, acc, hq, lane, hq.ccount);
+        queue_drain(v, acc, hq, lane, true);
+        v.reduce(acc);
+        if (lane == 0) team[warp] = acc;
+    }
+    __syncthreads();
+    if (live && warp % T == 0 && lane == 0) {
+        for (int k = 1; k < T; ++k) v.merge(acc, team[warp + k]);
+        v.finish(acc, row, c);
+    }
+}
+
+// Warps of a team for n rows: rows of a warp each fill the GPU from about
+// 5,000 on (152 SMs of 32 resident warps of this kernel).
+inline int team_size(int64_t n_rows) { return n_rows < 1216 ? 8 : n_rows < 2432 ? 4 : n_rows < 4864 ? 2 : 1; }
 
 // The grouped walk with each row's groups shared by `split` warps (warp
 // item u walks row u / split, every split-th group from the (u % split)-th):

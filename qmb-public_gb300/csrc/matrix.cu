@@ -110,6 +110,7 @@ struct MatrixPairs {
     int64_t* cursor;
     int32_t* col;
     double2* val;
+    __device__ __forceinline__ bool recording() const { return false; }
     __device__ __forceinline__ void record(const int4*, int, int) const {}
     __device__ __forceinline__ void apply(int4 h) const {
         if (!FILL) {

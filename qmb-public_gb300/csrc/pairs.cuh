@@ -80,9 +80,13 @@ constexpr int kPairBlocks = 608;
 template <int W>
 PairSet take_pair_set(Arena& ws, int64_t n, int sites);
 
-// Hits waiting for all lanes to have one: up to 31, while a lookup adds one a lane.
+// Hits waiting to be applied: one a lane, or four where they are recorded,
+// since every drain's atomic meets the same counter (3.6M recorded FP32 hits:
+// lookups 151 us with one, 128 us with four; unrecorded FP64 99 and 107 us).
+// Fewer than a drain wait while a lookup adds one a lane.
+constexpr int kPairDrain = 128;
 struct PairQueue {
-    int4 hits[64];  // (slot | parity << 31, from row, to row, 0)
+    int4 hits[kPairDrain + 32];  // (slot | parity << 31, from row, to row, 0)
 };
 
 template <int W>
@@ -221,9 +225,9 @@ struct PairWorker {
 
     __device__ __forceinline__ void drain(int n) {
         x.h.record(q.hits, n, lane);
-        if (lane < n) x.h.apply(q.hits[lane]);
+        for (int k = lane; k < n; k += 32) x.h.apply(q.hits[k]);
         __syncwarp();
-        if (lane < hcount - n) q.hits[lane] = q.hits[n + lane];
+        if (lane < hcount - n) q.hits[lane] = q.hits[n + lane];  // fewer than 32
         __syncwarp();
         hcount -= n;
     }
@@ -233,7 +237,8 @@ struct PairWorker {
         if (hit) q.hits[hcount + __popc(m & ((1u << lane) - 1u))] = v;
         hcount += __popc(m);
         __syncwarp();
-        if (hcount >= 32) drain(32);
+        const int full = x.h.recording() ? kPairDrain : 32;
+        if (hcount >= full) drain(full);
     }
     __device__ __forceinline__ uint32_t parity_of(const Key<W>& c, int64_t slot) const {
         int par = 0;
@@ -465,17 +470,46 @@ constexpr int kNotOrAnd = 0x07;     // ~(a | (b & c))
 template <int V>
 struct EmptyCount {
     uint32_t ones[V], twos[V], more[V];
-    // add a list of `pairs` pairs of positions
-    __device__ __forceinline__ void add(const uint32_t* planes, const uint16_t* list, int pairs, int lane) {
+    // count a list of `pairs` pairs of positions; more starts as `absent`
+    __device__ __forceinline__ void count(const uint32_t* planes, const uint16_t* list, int pairs, int lane,
+                                          const uint32_t (&absent)[V]) {
         int k = 0;
-#pragma unroll 1
-        for (; k + 2 <= pairs; k += 2) {
-            const uint2 at = *reinterpret_cast<const uint2*>(list + 2 * k);
+        if (pairs & 1) {
+            // an odd pair first: nothing is counted yet
+            const uint32_t at = *reinterpret_cast<const uint32_t*>(list + 2 * (pairs - 1));
+            uint32_t p0[V], p1[V];
+            PlaneWords<V>::get(planes + ((at & 0xffffu) + lane) * V, p0);
+            PlaneWords<V>::get(planes + ((at >> 16) + lane) * V, p1);
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                ones[v] = p0[v] ^ p1[v];
+                twos[v] = ~(p0[v] | p1[v]);
+                more[v] = absent[v];
+            }
+        } else if (pairs != 0) {
             uint32_t p0[V], p1[V], p2[V], p3[V];
-            PlaneWords<V>::get(planes + ((at.x & 0xffffu) + lane) * V, p0);
-            PlaneWords<V>::get(planes + ((at.x >> 16) + lane) * V, p1);
-            PlaneWords<V>::get(planes + ((at.y & 0xffffu) + lane) * V, p2);
-            PlaneWords<V>::get(planes + ((at.y >> 16) + lane) * V, p3);
+            four(planes, list, lane, p0, p1, p2, p3);
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const uint32_t c0 = ~(p0[v] | p1[v]);
+                const uint32_t s0 = p0[v] ^ p1[v];
+                const uint32_t c1 = logic3<kMajorityNot>(s0, p2[v], p3[v]);
+                ones[v] = logic3<kXor3>(s0, p2[v], p3[v]);
+                more[v] = logic3<kOrAnd>(absent[v], c0, c1);
+                twos[v] = c0 ^ c1;
+            }
+            k = 2;
+        } else {
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                ones[v] = twos[v] = 0u;
+                more[v] = absent[v];
+            }
+        }
+#pragma unroll 2
+        for (; k + 2 <= pairs; k += 2) {
+            uint32_t p0[V], p1[V], p2[V], p3[V];
+            four(planes, list + 2 * k, lane, p0, p1, p2, p3);
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 const uint32_t c0 = logic3<kMajorityNot>(ones[v], p0[v], p1[v]);
@@ -486,19 +520,14 @@ struct EmptyCount {
                 twos[v] = logic3<kXor3>(twos[v], c0, c1);
             }
         }
-        if (k < pairs) {
-            const uint32_t at = *reinterpret_cast<const uint32_t*>(list + 2 * k);
-            uint32_t p0[V], p1[V];
-            PlaneWords<V>::get(planes + ((at & 0xffffu) + lane) * V, p0);
-            PlaneWords<V>::get(planes + ((at >> 16) + lane) * V, p1);
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                const uint32_t c0 = logic3<kMajorityNot>(ones[v], p0[v], p1[v]);
-                ones[v] = logic3<kXor3>(ones[v], p0[v], p1[v]);
-                more[v] = logic3<kOrAnd>(more[v], twos[v], c0);
-                twos[v] ^= c0;
-            }
-        }
+    }
+    static __device__ __forceinline__ void four(const uint32_t* planes, const uint16_t* list, int lane, uint32_t (&p0)[V],
+                                                uint32_t (&p1)[V], uint32_t (&p2)[V], uint32_t (&p3)[V]) {
+        const uint2 at = *reinterpret_cast<const uint2*>(list);
+        PlaneWords<V>::get(planes + ((at.x & 0xffffu) + lane) * V, p0);
+        PlaneWords<V>::get(planes + ((at.x >> 16) + lane) * V, p1);
+        PlaneWords<V>::get(planes + ((at.y & 0xffffu) + lane) * V, p2);
+        PlaneWords<V>::get(planes + ((at.y >> 16) + lane) * V, p3);
     }
 };
 
@@ -586,12 +615,7 @@ __global__ void __launch_bounds__(kThreads, 3)
             for (; todo != 0; todo &= todo - 1) {
                 const int r = __ffs(todo) - 1;
                 EmptyCount<V> c;
-#pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    c.ones[v] = c.twos[v] = 0u;
-                    c.more[v] = absent[v];
-                }
-                c.add(s_planes, s_list + r * sites, __shfl_sync(0xffffffffu, twos, r), lane);
+                c.count(s_planes, s_list + r * sites, __shfl_sync(0xffffffffu, twos, r), lane, absent);
                 uint32_t near[V], any = 0;
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
