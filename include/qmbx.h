@@ -340,6 +340,18 @@ int qmbx_lanczos_step(int64_t n, const int64_t* row_ptr, const int32_t* col, con
                       const double* beta_prev, const double* v, double* v_next, double* alpha, double* beta,
                       void* scratch, uint64_t scratch_bytes, qmbx_stream_t stream);
 
+/* The energy of psi from H psi on the same rows (qmb/vmc.py:111-114) and its
+ * gradient for Hermitian H: sums[0] = Re<psi|H psi> / <psi|psi>, sums[1] =
+ * <psi|psi>; out = 2 *grad (H psi - sums[0] psi) / sums[1].  psi and out are
+ * complex float when single is set, else complex double; hpsi is complex
+ * double [n]; sums (2), grad (1) and scratch (1024) are device doubles.
+ * Everything is formed in FP64, in a fixed order. */
+int qmbx_energy(int64_t n, int32_t single, const void* psi, const double* hpsi, double* sums, double* scratch,
+                qmbx_stream_t stream);
+
+int qmbx_energy_grad(int64_t n, int32_t single, const void* psi, const double* hpsi, const double* sums,
+                     const double* grad, void* out, qmbx_stream_t stream);
+
 /* ---------------------------------------------------------------------------
  * The elementwise parts of the autoregressive network of qmb/mlp.py:60-314
  * (WaveFunctionElectronUpDown, the caller that samples the configurations

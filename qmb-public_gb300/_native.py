@@ -56,6 +56,8 @@ SIGNATURES: dict[str, tuple] = {
     "qmbx_matrix_count": (ctypes.c_int, [_P, _P, _P, _I64, _P, _PI64, _P, _U64, _P]),
     "qmbx_matrix_fill": (ctypes.c_int, [_P, _P, _P, _I64, _P, _P, _P, _P, _U64, _P]),
     "qmbx_matrix_apply": (ctypes.c_int, [_I64, _P, _P, _P, _P, _P, _P]),
+    "qmbx_energy": (ctypes.c_int, [_I64, _I32, _P, _P, _P, _P, _P]),
+    "qmbx_energy_grad": (ctypes.c_int, [_I64, _I32, _P, _P, _P, _P, _P, _P]),
     "qmbx_lanczos_step": (ctypes.c_int, [_I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _U64, _P]),
     "qmbx_matrix_apply_many": (ctypes.c_int, [_I64, _I64, _I32, _P, _P, _P, _P, _P, _P]),
     "qmbx_find_relative_workspace": (ctypes.c_int, [_P, _I64, _I64, _I64, _PU64]),

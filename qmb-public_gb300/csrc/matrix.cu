@@ -390,6 +390,65 @@ __global__ void __launch_bounds__(kThreads) spmm_kernel(int64_t n, int m, const 
     }
 }
 
+// ---------------------------------------------------------------------------
+// E = Re<psi|H psi> / <psi|psi> and its gradient 2 g (H psi - E psi) / <psi|psi>
+// in FP64, for psi in FP64 or FP32: one pass and a sum instead of nine library
+// calls (65,536 rows: 60 us of kernels), one pass instead of six.
+// ---------------------------------------------------------------------------
+
+template <bool F32>
+__device__ __forceinline__ double2 amplitude_at(const void* psi, int64_t i) {
+    if (F32) {
+        const float2 p = __ldg(static_cast<const float2*>(psi) + i);
+        return make_double2((double)p.x, (double)p.y);
+    }
+    return __ldg(static_cast<const double2*>(psi) + i);
+}
+
+template <bool F32>
+__global__ void __launch_bounds__(kThreads) energy_parts_kernel(int64_t n, const void* __restrict__ psi,
+                                                                const double2* __restrict__ hpsi,
+                                                                double* __restrict__ parts) {
+    __shared__ double s_warp[kWarpsPerBlock];
+    double num = 0.0, norm = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kThreads) {
+        const double2 p = amplitude_at<F32>(psi, i), h = __ldg(hpsi + i);
+        num += p.x * h.x + p.y * h.y;
+        norm += p.x * p.x + p.y * p.y;
+    }
+    store_part(num, parts, s_warp);
+    __syncthreads();
+    store_part(norm, parts + kLanczosBlocks, s_warp);
+}
+
+// out[0] = E, out[1] = <psi|psi>
+__global__ void __launch_bounds__(kThreads) energy_sum_kernel(const double* __restrict__ parts, int n_parts,
+                                                              double* __restrict__ out) {
+    __shared__ double s_warp[kWarpsPerBlock];
+    const double num = sum_parts(parts, n_parts, s_warp);
+    const double norm = sum_parts(parts + kLanczosBlocks, n_parts, s_warp);
+    if (threadIdx.x == 0) {
+        out[0] = num / norm;
+        out[1] = norm;
+    }
+}
+
+template <bool F32>
+__global__ void energy_grad_kernel(int64_t n, const void* __restrict__ psi, const double2* __restrict__ hpsi,
+                                   const double* __restrict__ sums, const double* __restrict__ grad,
+                                   void* __restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double e = sums[0], norm = sums[1], g = grad[0] * 2.0;
+    const double2 p = amplitude_at<F32>(psi, i), h = __ldg(hpsi + i);
+    const double re = g * (h.x - e * p.x) / norm, im = g * (h.y - e * p.y) / norm;
+    if (F32) {
+        static_cast<float2*>(out)[i] = make_float2((float)re, (float)im);
+    } else {
+        static_cast<double2*>(out)[i] = make_double2(re, im);
+    }
+}
+
 struct MatrixLayout {
     HashRows rows;
     int32_t* count;
@@ -663,5 +722,44 @@ extern "C" int qmbx_lanczos_step(int64_t n, const int64_t* row_ptr, const int32_
     QMBX_KERNEL(kGroupOther, s, lanczos_update_kernel<<<blocks, kThreads, 0, s>>>(n, parts, products, reinterpret_cast<const double2*>(v_prev), beta_prev, vv, w, alpha, norms));
     QMBX_KERNEL(kGroupOther, s, lanczos_scale_kernel<<<blocks, kThreads, 0, s>>>(n, norms, blocks, w, reinterpret_cast<double2*>(v_next), beta));
     QMBX_LAUNCH_CHECK("Lanczos step");
+    return QMBX_OK;
+}
+
+extern "C" int qmbx_energy(int64_t n, int32_t single, const void* psi, const double* hpsi, double* sums, double* scratch,
+                           qmbx_stream_t stream) {
+    clear_error();
+    if (n < 0 || n >= (int64_t(1) << 31)) return fail(QMBX_ERR_ARGUMENT, "row count out of range");
+    if ((n > 0 && (psi == nullptr || hpsi == nullptr)) || sums == nullptr || scratch == nullptr) {
+        return fail(QMBX_ERR_ARGUMENT, "pointers must not be NULL");
+    }
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    const double2* h = reinterpret_cast<const double2*>(hpsi);
+    const int blocks = grid_for(n, kThreads) < (unsigned)kLanczosBlocks ? (int)grid_for(n, kThreads) : kLanczosBlocks;
+    if (single) {
+        QMBX_KERNEL(kGroupOther, s, energy_parts_kernel<true><<<blocks, kThreads, 0, s>>>(n, psi, h, scratch));
+    } else {
+        QMBX_KERNEL(kGroupOther, s, energy_parts_kernel<false><<<blocks, kThreads, 0, s>>>(n, psi, h, scratch));
+    }
+    QMBX_KERNEL(kGroupOther, s, energy_sum_kernel<<<1, kThreads, 0, s>>>(scratch, blocks, sums));
+    QMBX_LAUNCH_CHECK("energy");
+    return QMBX_OK;
+}
+
+extern "C" int qmbx_energy_grad(int64_t n, int32_t single, const void* psi, const double* hpsi, const double* sums,
+                                const double* grad, void* out, qmbx_stream_t stream) {
+    clear_error();
+    if (n < 0 || n >= (int64_t(1) << 31)) return fail(QMBX_ERR_ARGUMENT, "row count out of range");
+    if (n == 0) return QMBX_OK;
+    if (psi == nullptr || hpsi == nullptr || sums == nullptr || grad == nullptr || out == nullptr) {
+        return fail(QMBX_ERR_ARGUMENT, "pointers must not be NULL");
+    }
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    const double2* h = reinterpret_cast<const double2*>(hpsi);
+    if (single) {
+        QMBX_KERNEL(kGroupOther, s, energy_grad_kernel<true><<<grid_for(n, kThreads), kThreads, 0, s>>>(n, psi, h, sums, grad, out));
+    } else {
+        QMBX_KERNEL(kGroupOther, s, energy_grad_kernel<false><<<grid_for(n, kThreads), kThreads, 0, s>>>(n, psi, h, sums, grad, out));
+    }
+    QMBX_LAUNCH_CHECK("energy gradient");
     return QMBX_OK;
 }

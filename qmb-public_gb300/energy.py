@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import torch
 
+from . import _native
 from .hamiltonian import Hamiltonian
 
 __all__ = ["variational_energy"]
@@ -25,23 +26,33 @@ class _HermitianEnergy(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, ham: Hamiltonian, configs, psi):
+        psi = psi.detach().resolve_conj().contiguous()
         if psi.dtype == torch.complex64:
-            hpsi = ham.apply_within_compensated(configs, psi.detach(), configs)
+            hpsi = ham.apply_within_compensated(configs, psi, configs)
         else:
-            hpsi = ham.apply_within(configs, psi.detach(), configs)
-        psi64 = psi.detach().to(torch.complex128)
-        norm = torch.sum(psi64.conj() * psi64).real
-        energy = torch.sum(psi64.conj() * hpsi).real / norm
-        ctx.in_dtype = psi.dtype
-        ctx.save_for_backward(hpsi, psi64, energy, norm)
-        return energy
+            hpsi = ham.apply_within(configs, psi, configs)
+        sums = torch.empty(2, dtype=torch.float64, device=psi.device)
+        with torch.cuda.device(psi.device):
+            scratch = torch.empty(1024, dtype=torch.float64, device=psi.device)
+            _native.call("qmbx_energy", psi.shape[0], int(psi.dtype == torch.complex64), psi.data_ptr(), hpsi.data_ptr(),
+                         sums.data_ptr(), scratch.data_ptr(), torch.cuda.current_stream(psi.device).cuda_stream)
+        ctx.save_for_backward(hpsi, psi, sums)
+        return sums[0].clone()
 
     @staticmethod
     def backward(ctx, grad):
-        hpsi, psi64, energy, norm = ctx.saved_tensors
+        hpsi, psi, sums = ctx.saved_tensors
         # torch's gradient of a real loss in a complex input is 2 dL/dpsi*
-        g = grad * 2.0 * (hpsi - energy * psi64) / norm
-        return None, None, g.to(ctx.in_dtype)
+        if torch.is_grad_enabled():  # a graph of the gradient was asked for: it is linear in grad
+            g = grad * 2.0 * (hpsi - sums[0] * psi.to(torch.complex128)) / sums[1]
+            return None, None, g.to(psi.dtype)
+        grad = grad.to(torch.float64).contiguous()
+        g = torch.empty_like(psi)
+        with torch.cuda.device(psi.device):
+            _native.call("qmbx_energy_grad", psi.shape[0], int(psi.dtype == torch.complex64), psi.data_ptr(),
+                         hpsi.data_ptr(), sums.data_ptr(), grad.data_ptr(), g.data_ptr(),
+                         torch.cuda.current_stream(psi.device).cuda_stream)
+        return None, None, g
 
 
 def variational_energy(ham: Hamiltonian, configs: torch.Tensor, psi: torch.Tensor, *,
