@@ -13,12 +13,13 @@ whose backward replays them.  The metric is term applications per second
 counted as the reference counts them: T * (N_i + N_j) per step (the
 reference's thread grid is T * N_i for a forward application, T * N_j for
 the same kernel run on the daggered table from configs_j).  The engine
-visits fewer pairs (one walk over the 20,000 configs_i rows);
-``walked_pairs_per_s`` reports that count.  The same
+visits no such pair where it compares rows with rows, so the rate is a work
+equivalent, not a count of what ran; ``walked_pairs_per_s`` is the same for
+one walk over the 20,000 configs_i rows.  The same
 line reports the FP64 path, the reference's own CUDA apply_within run from
 its cubin (``ref_cuda_fp64``), find_relative (top 50,000 excluding
 configs_i), the energy error of the FP32 path, the end-to-end rate through
-the public API with host buffers, the rooflines of the term walk, and the
+the public API with host buffers, the rooflines of the enumeration, and the
 CPU oracle's rate on the host cores.
 
 ``--impl reference`` times the reference's CPU algorithm (the oracle port in
@@ -604,7 +605,7 @@ def run_ours(args, wl, rank: int, world: int) -> dict | None:
     except (RuntimeError, OSError) as exc:  # a missing driver entry point or cubin load failure
         ref_cuda = {"unavailable": f"{type(exc).__name__}: {exc}"}
 
-    # roofline of the term walk: algorithmic bytes per launch
+    # roofline of the enumeration (the pair scan): algorithmic bytes per launch
     # forward: targets N_j (key + FP64 result), sources N_i (key + FP32 amplitude), terms T (28 B)
     # adjoint: the same with the two sets swapped
     # (a step walks once, the forward, when its backward replays the hit log; twice without it)
@@ -632,7 +633,7 @@ def run_ours(args, wl, rank: int, world: int) -> dict | None:
         "dtype": "f32",
         "data": "synthetic",
         "config": workload_config(args, wl),
-        "roofline": hbm_roofline(alg, per_launch_ms, "term walk (grouped_kernel)", figs),
+        "roofline": hbm_roofline(alg, per_launch_ms, "pair scan (pair_scan_kernel; its lookups are not in this time)", figs),
         "issue_roofline": issue_roofline(figs, per_launch_ms, device, clocks.summary()),
         "cpu_baseline": cpu,
         "e2e": {"value": world * units / (ms_e2e / args.steps * 1e-3), "unit": "term-applications/s",
@@ -648,8 +649,8 @@ def run_ours(args, wl, rank: int, world: int) -> dict | None:
                                                     launches_per_step=n_replay / args.steps)},
         "walked_pairs_per_s": {"value": world * walks_per_step * T * n_i / (ms_step32 * 1e-3),
                                "walks_per_step": walks_per_step,
-                               "what": "(term, row) pairs the term walks visit: each walk covers configs_i's "
-                                       f"{n_i} rows (T * N_i = {T * n_i:.3e}); the forward walk records its hits "
+                               "what": "(term, row) pairs that a term walk would visit, not pairs that the scan visits: configs_i's "
+                                       f"{n_i} rows (T * N_i = {T * n_i:.3e}); the forward records its hits "
                                        "and the adjoint replays them"},
         "fp64": {"value": world * units / (ms64 / args.steps * 1e-3), "ms_per_step": ms64 / args.steps},
         "speedup_fp32c_vs_fp64": ms64 / ms32,
@@ -658,7 +659,7 @@ def run_ours(args, wl, rank: int, world: int) -> dict | None:
                           "kernel_groups_ms": {g: prof_rel["groups"][g][1] / reps for g in prof_rel["groups"]},
                           "stats": stats_rel,
                           "sort_roofline": hbm_roofline(sort_bytes, ms_sort / reps,
-                                                        "radix sort of the selected rows (radix_hist/scatter + scans)",
+                                                        "sort and output of the selected rows (find_sort_kernel)",
                                                         None, launches_per_call=n_sort / reps) if ms_sort > 0 else None},
         "energy": {"fp64": e64, "fp32c": e32, "abs_error_ha": abs(e32 - e64)},
         "kernel_groups_ms_per_step": {g: prof["groups"][g][1] / args.steps for g in prof["groups"]},
@@ -802,7 +803,7 @@ def run_extra(args, wl) -> dict:
                      "energy_fp64": e64, "energy_fp32c": e32, "energy_abs_error_ha": abs(e32 - e64),
                      "hermitian": ham._table(device, nq).hermitian,
                      "walks_per_step": prof["groups"]["enumerate"][0],
-                     "roofline": walk_roofline(prof, n, n, 8, "term walk (pivot_kernel)"),
+                     "roofline": walk_roofline(prof, n, n, 8, "pair scan (pair_scan_kernel)"),
                      "kernel_groups_ms_per_step": {g: v[1] for g, v in prof["groups"].items()}})
     elif args.workload in ("c1", "c4"):
         psi32 = torch.from_numpy(wl["psi"]).to(torch.complex64).to(device)
@@ -884,7 +885,8 @@ def run_extra(args, wl) -> dict:
                                "denominators, Epstein-Nesbet sum)", "value": ms, "unit": "ms", "ms_per_step": ms,
                      "higher_is_better": False, "dtype": "f64", "count_selected": K, "e0": result["e"][0],
                      "e2": result["e"][1],
-                     "roofline": walk_roofline(prof, n, n, 16, "term walk"),
+                     "roofline": walk_roofline(prof, n, n, 16,
+                                           "find_relative passes (relative_bounded_kernel) and pair scan"),
                      "kernel_groups_ms_per_run": {g: v[1] for g, v in prof["groups"].items()}})
     elif args.workload == "sampler":
         from oracle import sampler as oracle_sampler
@@ -934,8 +936,8 @@ def run_extra(args, wl) -> dict:
                      "ms_per_step": ms, "higher_is_better": False, "dtype": "f64", "count_selected": K,
                      "rows_out": int(rel.shape[0]), "term_applications_per_s": T * n / (ms * 1e-3),
                      "stats": stats,
-                     "roofline": walk_roofline(prof, n, ci.shape[0], 16, "term walk (pivot_kernel)"),
-                     "sort_roofline": hbm_roofline(stats["sort_bytes"], ms_sort, "radix sort of the selected rows",
+                     "roofline": walk_roofline(prof, n, ci.shape[0], 16, "find_relative passes (relative_bounded_kernel)"),
+                     "sort_roofline": hbm_roofline(stats["sort_bytes"], ms_sort, "sort and output of the selected rows",
                                                    None, launches_per_call=n_sort) if ms_sort > 0 else None,
                      "kernel_groups_ms_per_run": {g: v[1] for g, v in prof["groups"].items()}})
     line["clocks"] = clocks.summary()

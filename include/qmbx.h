@@ -105,7 +105,9 @@ int qmbx_table_hermitian(const void* table_host, int32_t* hermitian);
  * side is not much larger than the input side.  Otherwise the input side is
  * walked and contributions are added with FP64 atomics (as is every
  * pivot-major walk, taken for tables whose pivot groups hold hundreds of
- * terms), whose order varies from run to run in the last bits.
+ * terms, and every pair scan, taken for large row sets under operators that
+ * keep the particle number), whose order varies from run to run in the last
+ * bits.
  * QMBX_DETERMINISTIC=1 in the environment (read at every call) keeps every
  * call on the fixed-order walk.  Repeated rows of an input are summed with
  * atomics before the walk in any case.

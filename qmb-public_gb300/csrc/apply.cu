@@ -3,11 +3,11 @@
 //
 // The reference scatters: one thread per (term, source) pair, a byte-wise
 // binary search of the image among the sorted targets, and FP64 atomics
-// (qmb/_hamiltonian_cuda.cu:86-274).  Here the work is gathered instead: one
-// thread per distinct target row walks the daggered terms, finds the source
-// row among the sorted, de-duplicated sources and accumulates in registers,
-// so no atomics are needed and the summation order is fixed.  The adjoint
-// runs the same walk with the forward terms over the sources.
+// (qmb/_hamiltonian_cuda.cu:86-274).  Here operators that conserve the particle
+// number compare the two row sets (pairs.cuh); the rest, and small calls, walk
+// the terms of the smaller side's distinct rows and look the images up in a
+// hash set of the other side: gathered in registers over the output side, or
+// scattered with FP64 atomics from the input side.
 #include <cuda_runtime.h>
 
 #include "pairs.cuh"

@@ -25,9 +25,10 @@
 //   those 65,536 rows with themselves     13.2 ms walked, 0.20 ms scanned
 //   20,000 x 200,000 rows of 10 on 28     0.80 ms walked, 0.31 + 0.10 ms (2.8M pairs looked up)
 //   16,384 clustered rows (8.7M hits)     6.4 ms walked, 0.11 + 0.17 ms (matrix count)
-// The scan is bound by the ALU pipe (74 % of its issue rate with the first
-// shape: 64 lanes a clock and SM for the three-input logic, 1.75 of them per
-// position and word); shared memory is at 56 % and L2 idle.  Counting the head
+// No one unit of the scan is full: the first shape keeps the ALU pipe at 62 %
+// (64 lanes a clock and SM for the three-input logic, 1.75 of them per position
+// and word) and L1 with shared memory at 77 %, the second 59 % and 67 %, with
+// 36 % of the warps resident; DRAM and L2 are near idle.  Counting the head
 // that sorted neighbours share once per run of rows gained 1 % and is not done.
 // The lookups are bound by the latency of their L2 reads.
 #pragma once

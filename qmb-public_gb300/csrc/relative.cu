@@ -5,24 +5,22 @@
 // single_relative neighbours under per-row locks (:805-996).  Here neither
 // needs a lock or any device-side wait:
 //
-//   find_relative  pass 1 counts the candidate records per weight bucket (the
-//                  top 12 bits of an FP32 estimate |coef|^2 |psi|^2 of the
-//                  weight) over every 16th source row (every row of small
-//                  inputs); one warp on the device picks from the scaled
-//                  counts a bucket that should hold about twice
-//                  count_selected records above it; pass 2 enumerates every
-//                  row, counts all records per bucket and keeps those at or
-//                  above the bucket below the chosen one.  The exact counts
-//                  of pass 2 confirm that every record down to the
-//                  count_selected-th was kept (else pass 2 runs again with
-//                  the exact threshold) -- the one host round trip before
-//                  the result.  The kept records get the reference's exact
-//                  FP64 weight (:494-497) and a 128-bit rank key (weight,
-//                  visiting order); a radix select over 12-bit digits finds
-//                  the count_selected-th key, the records up to it are
-//                  compacted, and their rows are sorted and de-duplicated.
-//   single_relative  one thread per row keeps the best Efraimidis-Spirakis
-//                  key of its candidates in registers.
+//   find_relative  pass 1 counts records per weight bucket (the top 12 bits of
+//                  an FP32 estimate |coef|^2 |psi|^2 of the weight) over every
+//                  16th source row (every row of small inputs); one block
+//                  picks from the scaled counts a bucket that should hold
+//                  about twice count_selected records above it; pass 2 keeps
+//                  the records at or above the bucket below that one.  The
+//                  kept records get the reference's exact FP64 weight
+//                  (:494-497) and a 128-bit rank key (weight, visiting order);
+//                  a radix select finds the count_selected-th key, and the
+//                  rows up to it are sorted, de-duplicated and unpacked, all
+//                  from counts on the device.  The host reads once: if fewer
+//                  than count_selected records were kept, pass 2 and the rest
+//                  run again with an exact threshold.
+//   single_relative  the first term, in descending order of its
+//                  Efraimidis-Spirakis key, that leads outside the input; the
+//                  walks keep the best key of a row's candidates in registers.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

@@ -5,8 +5,9 @@ the loop of qmb/haar.py:107-183): repeated square applications of H on a
 fixed basis, the three-term recurrence on device in complex128, and the
 lowest Ritz pair from SciPy's ``eigh_tridiagonal`` ('stebz').  Unlike the
 reference, H is materialised once on the basis as a sparse matrix
-(``Hamiltonian.matrix``: two term walks) and every iteration is a sparse
-matrix-vector product, unless the matrix would not fit the memory budget, in
+(``Hamiltonian.matrix``) and every iteration is a sparse matrix-vector
+product and two vector passes, whose scalars stay on the device
+(``HamiltonianMatrix.lanczos_step``), unless the matrix would not fit the memory budget, in
 which case every iteration walks the terms (``apply_within``) as the
 reference does; the Krylov vectors stay in device memory (a GB300 holds
 ~280 GB), so no vector is copied to the host inside the loop.
