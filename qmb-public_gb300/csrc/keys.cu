@@ -314,19 +314,23 @@ __global__ void reach_insert_kernel(const uint64_t* __restrict__ keys, const int
     }
 }
 
+// A walked row that is itself in the looked-up set shares all its words with
+// its own copy, which no term that changes a row leads to: only places that
+// two rows or more took count for it.
 template <int W>
 __global__ void reach_flags_kernel(const uint64_t* __restrict__ keys, const int32_t* __restrict__ unique,
-                                   const int* __restrict__ count, int same, Reach r) {
+                                   const int* __restrict__ count, int same, HashView look, Reach r) {
     const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= *count) return;
     const Key<W> k = load_key<W>(keys, __ldg(unique + u));
     unsigned flags = 0;
+    const bool own = same || hash_find<W>(look, k) >= 0;
 #pragma unroll
     for (int w = 0; w < W; ++w) {
         uint64_t at;
         unsigned long long bits;
         reach_place<W>(k, w, r.words, at, bits);
-        const unsigned long long have = __ldg((same ? r.twice : r.once) + w * r.words + at);
+        const unsigned long long have = __ldg((own ? r.twice : r.once) + w * r.words + at);
         if ((have & bits) == bits) flags |= 1u << w;
     }
     r.flags[u] = (uint8_t)flags;
@@ -348,7 +352,7 @@ int build_reach(const HashRows& walk, const HashRows& look, bool same, const Rea
     QMBX_CUDA_TRY(cudaMemsetAsync(r.once, 0, (size_t)r.words * W * sizeof(unsigned long long), s));
     QMBX_CUDA_TRY(cudaMemsetAsync(r.twice, 0, (size_t)r.words * W * sizeof(unsigned long long), s));
     QMBX_KERNEL(kGroupKeys, s, reach_insert_kernel<W><<<grid_for(look.n, kThreads), kThreads, 0, s>>>(look.keys, look.unique, look.count, r));
-    QMBX_KERNEL(kGroupKeys, s, reach_flags_kernel<W><<<grid_for(walk.n, kThreads), kThreads, 0, s>>>(walk.keys, walk.unique, walk.count, same ? 1 : 0, r));
+    QMBX_KERNEL(kGroupKeys, s, reach_flags_kernel<W><<<grid_for(walk.n, kThreads), kThreads, 0, s>>>(walk.keys, walk.unique, walk.count, same ? 1 : 0, look.hash(), r));
     QMBX_LAUNCH_CHECK("build_reach");
     return QMBX_OK;
 }

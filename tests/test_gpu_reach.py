@@ -62,3 +62,26 @@ def test_reach_matches_the_oracle(n_qubytes, shift, kinds, cuda_device):
         assert np.all(np.abs(y.detach().cpu().numpy() - want) <= tol * scale)
         want = oracle.apply_within_adjoint(site, kind, coef, ci, cj, gj.astype(dtype).astype(np.complex128), 1)
         assert np.all(np.abs(back.cpu().numpy() - want) <= tol * scale)
+
+
+@pytest.mark.parametrize("kind", ["random", "halves", "chains"])
+@pytest.mark.parametrize("more", [0, 500])
+def test_reach_with_the_rows_copied(kind, more, cuda_device):
+    # the looked-up set holds a copy of every walked row, and `more` others
+    site, kinds, coef = (x.numpy() for x in terms.sort_terms(*terms.prepare(terms.hubbard_dict(6, 6, 1.0, 4.0))))
+    shift, n_qubytes = 4, 10
+    site = np.where(kinds == 2, site, site + shift).astype(np.int16)
+    ci = _rows(n_qubytes, 72, shift, kind, 61)
+    cj = ci if more == 0 else terms.unique_rows(np.concatenate([ci, _rows(n_qubytes, 72, shift, "random", 62)[:more]]))
+    ham = Hamiltonian((torch.from_numpy(site), torch.from_numpy(kinds), torch.from_numpy(coef)), kind="fermi")
+    di, dj = torch.from_numpy(ci).to(cuda_device), torch.from_numpy(cj.copy()).to(cuda_device)
+    psi, gj = terms.random_psi(ci.shape[0], seed=63), terms.random_psi(cj.shape[0], seed=64)
+    scale = np.abs(coef).sum() * max(np.abs(psi).max(), np.abs(gj).max())
+    for dtype, tol in ((np.complex128, 1e-12), (np.complex64, 2e-7)):
+        p = torch.from_numpy(psi.astype(dtype)).to(cuda_device).requires_grad_(True)
+        y = ham.apply_within(di, p, dj)
+        (back,) = torch.autograd.grad(y, p, grad_outputs=torch.from_numpy(gj.astype(dtype)).to(cuda_device))
+        want = oracle.apply_within(site, kinds, coef, ci, psi.astype(dtype).astype(np.complex128), cj, 1)
+        assert np.all(np.abs(y.detach().cpu().numpy() - want) <= tol * scale)
+        want = oracle.apply_within_adjoint(site, kinds, coef, ci, cj, gj.astype(dtype).astype(np.complex128), 1)
+        assert np.all(np.abs(back.cpu().numpy() - want) <= tol * scale)
