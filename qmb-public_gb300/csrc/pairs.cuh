@@ -67,7 +67,7 @@ struct PairSet {
 
 struct PairWork {
     PairSet i, j;          // j == i for the same rows on both sides
-    unsigned int* next;    // work items handed out, and pairs listed (two counters)
+    unsigned long long* next;  // work items handed out, and close pairs found (two counters)
     uint2* pairs;          // pairs that stay: scan positions of the list side and the plane side
     unsigned int cap;      // places in `pairs`; pairs past them are looked up by the scan itself,
     void* overflow;        // with a PairQueue per warp of the grid
@@ -96,7 +96,7 @@ PairWork take_pair_work(Arena& ws, int64_t n_i, int64_t n_j, bool same, int site
     p.same = same;
     p.i = take_pair_set<W>(ws, n_i, sites);
     p.j = same ? p.i : take_pair_set<W>(ws, n_j, sites);
-    p.next = ws.take<unsigned int>(2);
+    p.next = ws.take<unsigned long long>(2);
     // room for a few dozen pairs a row (C2's 220,000 rows list 2.8M pairs); a
     // looked-up pair costs about 35 ps in the list and ten times that in the scan
     const double all = (double)(n_i > 0 ? n_i : 1) * (double)(n_j > 0 ? n_j : 1);
@@ -324,10 +324,10 @@ __device__ __noinline__ void pair_overflow(const PairContext<W, H>* x, PairQueue
 template <int W, class H>
 __global__ void __launch_bounds__(kThreads) pair_lookup_kernel(const __grid_constant__ PairContext<W, H> context,
                                                                const uint2* __restrict__ pairs,
-                                                               const unsigned int* __restrict__ listed,
+                                                               const unsigned long long* __restrict__ listed,
                                                                unsigned int cap) {
     __shared__ PairQueue s_queue[kWarpsPerBlock];
-    const unsigned int n = *listed < cap ? *listed : cap;
+    const unsigned int n = *listed < cap ? (unsigned int)*listed : cap;
     const int lane = threadIdx.x & 31;
     PairWorker<W, H> work{context, s_queue[threadIdx.x >> 5], 0, lane};
     const uint64_t step = (uint64_t)gridDim.x * kThreads;
@@ -355,7 +355,7 @@ template <int W, class H>
 struct PairOut {
     const PairContext<W, H>* context;
     uint2* pairs;
-    unsigned int* listed;
+    unsigned long long* listed;  // counts on past the list's end; two sets can hold more than 2^32 close pairs
     unsigned int cap;
     PairQueue* overflow;
 };
@@ -364,13 +364,13 @@ struct PairOut {
 template <int W, class H>
 __device__ __forceinline__ void pair_list(const PairOut<W, H>& out, const PairFound<W>& f, int64_t a0, int64_t b0,
                                           int waiting, int n, int lane) {
-    unsigned int base = 0;
-    if (lane == 0) base = atomicAdd(out.listed, (unsigned int)n);
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(out.listed, (unsigned long long)n);
     base = __shfl_sync(0xffffffffu, base, 0);
     const uint32_t e = f.pairs[lane < n ? waiting - n + lane : 0];
     const uint32_t pa = (uint32_t)a0 + (e >> PairFound<W>::kTileBits);
     const uint32_t pb = (uint32_t)b0 + (e & ((1u << PairFound<W>::kTileBits) - 1u));
-    const bool late = lane < n && (uint64_t)base + lane >= out.cap;
+    const bool late = lane < n && base + lane >= out.cap;
     if (lane < n && !late) out.pairs[base + lane] = make_uint2(pa, pb);
     if (__any_sync(0xffffffffu, late)) {
         pair_overflow<W, H>(out.context, out.overflow + blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5), late, pa, pb);
@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     pair_scan_kernel(const __grid_constant__ PairContext<W, H> context, const uint32_t* __restrict__ planes,
                      const uint16_t* __restrict__ lists, const int* __restrict__ a_count,
                      const int* __restrict__ b_count, int sites, int chunk,
-                     unsigned int* __restrict__ next, uint2* __restrict__ pairs, unsigned int cap, PairQueue* overflow,
+                     unsigned long long* __restrict__ next, uint2* __restrict__ pairs, unsigned int cap, PairQueue* overflow,
                      const int* __restrict__ gate) {
     constexpr int V = pair_words<W>();
     constexpr int kWords = 32 * V;
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     extern __shared__ uint4 pair_sm[];
     uint32_t* s_planes = reinterpret_cast<uint32_t*>(pair_sm);
     __shared__ PairFound<W> s_found[kWarpsPerBlock];
-    __shared__ unsigned int s_item;
+    __shared__ unsigned long long s_item;
     if (gate != nullptr && *gate == 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
@@ -567,9 +567,9 @@ __global__ void __launch_bounds__(kThreads, 3)
     int rows = 0, single = 0;  // entries and pairs waiting in `found`
     for (;;) {
         __syncthreads();  // the last item's planes and number have been read
-        if (threadIdx.x == 0) s_item = atomicAdd(next, 1u);
+        if (threadIdx.x == 0) s_item = atomicAdd(next, 1ull);
         __syncthreads();
-        const int64_t item = s_item;
+        const int64_t item = (int64_t)s_item;
         if (item >= tiles * chunks) break;
         const int64_t tile = item / chunks;
         const int64_t first = (item - tile * chunks) * chunk;
@@ -660,7 +660,7 @@ int launch_pair_scan(const H& h, const PairWork& p, const void* table_host, cons
     QMBX_CUDA_TRY(cudaFuncSetAttribute(pair_scan_kernel<W, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
     const PairContext<W, H> context{h, class_view(table_host, table_dev), part_view(table_host, table_dev, QMBX_PART_FWD),
                                     a.keys, b.keys, a.row, b.row, p.same ? 1 : 0, swap ? 1 : 0};
-    QMBX_CUDA_TRY(cudaMemsetAsync(p.next, 0, 2 * sizeof(unsigned int), s));
+    QMBX_CUDA_TRY(cudaMemsetAsync(p.next, 0, 2 * sizeof(unsigned long long), s));
     const int grid = pivot_grid() < kPairBlocks ? pivot_grid() : kPairBlocks;
     QMBX_KERNEL(group, s, pair_scan_kernel<W, H><<<grid, kThreads, shared, s>>>(
         context, b.planes, a.list, a.count, b.count, sites, pair_chunk(a.n, b.n, pair_tile<W>()), p.next, p.pairs, p.cap,
