@@ -106,7 +106,8 @@ def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
     scalars = torch.empty((2, step + 2), dtype=torch.float64, device=device)
     alpha, beta = scalars[0], scalars[1]
     scratch = torch.empty(16 * n + 40960, dtype=torch.uint8, device=device)
-    first = start.to(torch.complex128) / torch.linalg.norm(torch.view_as_real(start.to(torch.complex128)))
+    start = start.to(torch.complex128).resolve_conj().resolve_neg()
+    first = start / torch.linalg.norm(torch.view_as_real(start))
     blocks = [first.reshape(1, n).contiguous()]
     seen = []
     v, v_prev, done, stop = blocks[0][0], None, 0, None

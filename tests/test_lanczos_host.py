@@ -1,0 +1,50 @@
+"""Host logic of the Lanczos recurrence on a stored matrix, on the CPU: a stand-in does the iteration's arithmetic."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from qmb_gb300 import solvers
+
+
+class DenseMatrix:
+    """HamiltonianMatrix.lanczos_step on a dense matrix; counts the iterations."""
+
+    def __init__(self, h: np.ndarray):
+        self.h = torch.from_numpy(h).to(torch.complex128)
+        self.val, self.n, self.steps = self.h, h.shape[0], 0
+
+    def lanczos_step(self, v_prev, beta_prev, v, v_next, alpha, beta, scratch):
+        self.steps += 1
+        w = self.h @ v
+        alpha.copy_((w.conj() @ v).real)
+        w = w - alpha * v - (beta_prev * v_prev if v_prev is not None else 0)
+        beta.copy_(torch.linalg.norm(w))
+        v_next.copy_(w / beta)
+
+
+def _matrix(n, seed):
+    rng = np.random.default_rng(seed)
+    h = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    return h + h.conj().T, rng.standard_normal(n) + 1j * rng.standard_normal(n)
+
+
+def _check(energy, vector, h):
+    v = vector.numpy()
+    assert abs(np.vdot(v, h @ v).real / np.vdot(v, v).real - energy) <= 1e-9 * np.abs(h).sum()
+
+
+@pytest.mark.parametrize("dtype", [torch.complex128, torch.complex64, torch.float64])
+def test_lazy_conjugates_and_other_types(dtype):
+    h, start = _matrix(40, 1)
+    x = torch.from_numpy(start)
+    x = x.to(dtype) if dtype.is_complex else x.real.contiguous().to(dtype)
+    plain, _ = solvers._lanczos_on_matrix(DenseMatrix(h), x.conj().resolve_conj().clone(), 8, 1e-12)
+    energy, vector = solvers._lanczos_on_matrix(DenseMatrix(h), x.conj(), 8, 1e-12)
+    assert abs(energy - plain) <= 1e-12 * abs(plain)
+    _check(energy, vector, h)
+    energy, _ = solvers._lanczos_on_matrix(DenseMatrix(h), torch._neg_view(x), 8, 1e-12)
+    want, _ = solvers._lanczos_on_matrix(DenseMatrix(h), -x, 8, 1e-12)
+    assert abs(energy - want) <= 1e-12 * abs(want)
