@@ -103,23 +103,22 @@ def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
     n, device = mat.n, start.device
     if start.shape != (n,) or device != mat.val.device:
         raise RuntimeError(f"start must have shape [{n}] and be on the matrix's device.")
-    scalars = torch.empty((2, step + 2), dtype=torch.float64, device=device)
-    alpha, beta = scalars[0], scalars[1]
     scratch = torch.empty(16 * n + 40960, dtype=torch.uint8, device=device)
     start = start.to(torch.complex128).resolve_conj().resolve_neg()
     first = start / torch.linalg.norm(torch.view_as_real(start))
     blocks = [first.reshape(1, n).contiguous()]
     seen = []
-    v, v_prev, done, stop = blocks[0][0], None, 0, None
+    v, v_prev, beta_prev, done, stop = blocks[0][0], None, None, 0, None
     # iteration k forms alpha[k], beta[k] and vector k + 1; the last one's beta and vector are not used
     while done < step + 2 and stop is None:
         count = min(_LOOK_EVERY, step + 2 - done)
         block = torch.empty((count, n), dtype=torch.complex128, device=device)
-        for k in range(done, done + count):
-            mat.lanczos_step(v_prev, beta[k - 1] if k else None, v, block[k - done], alpha[k], beta[k], scratch)
-            v_prev, v = v, block[k - done]
+        scalars = torch.empty((2, count), dtype=torch.float64, device=device)  # alpha and beta of the block
+        for k in range(count):
+            mat.lanczos_step(v_prev, beta_prev, v, block[k], scalars[0, k], scalars[1, k], scratch)
+            v_prev, v, beta_prev = v, block[k], scalars[1, k]
         blocks.append(block)
-        host = scalars[:, done:done + count].cpu().numpy()
+        host = scalars.cpu().numpy()
         seen.append(host)
         small = [k for k in range(done, done + count) if k < step + 1 and host[1, k - done] < threshold]
         stop = small[0] if small else None

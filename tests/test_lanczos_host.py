@@ -48,3 +48,11 @@ def test_lazy_conjugates_and_other_types(dtype):
     energy, _ = solvers._lanczos_on_matrix(DenseMatrix(h), torch._neg_view(x), 8, 1e-12)
     want, _ = solvers._lanczos_on_matrix(DenseMatrix(h), -x, 8, 1e-12)
     assert abs(energy - want) <= 1e-12 * abs(want)
+
+
+def test_more_steps_than_memory_has_places():
+    # "until the recurrence ends": nothing is reserved for steps that are never taken
+    h, start = _matrix(6, 2)
+    energy, vector = solvers._lanczos_on_matrix(DenseMatrix(h), torch.from_numpy(start), 10**15, 1e-9)
+    assert abs(energy - np.linalg.eigvalsh(h)[0]) <= 1e-8 * np.abs(h).sum()
+    _check(energy, vector, h)
