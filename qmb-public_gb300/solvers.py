@@ -93,13 +93,33 @@ def _lowest(alpha, beta):
     return float(vals[0]), vecs[:, 0]
 
 
-# iterations between two looks at beta on the host
-_LOOK_EVERY = 16
+# Iterations of a block at most.  The host looks at a block's norms while the next one runs, so that at most the
+# rest of a block and one more run past the end of the recurrence; with blocks of 16 and a look behind each, a
+# start that ends after two iterations cost 16 (1,000,000 rows of an entry each: 1.2 ms of products became 25).
+_LOOK_EVERY = 4
+
+
+class _Look:
+    """A copy of a small device tensor on its way to the host."""
+
+    def __init__(self, values: torch.Tensor):
+        if values.is_cuda:
+            self.host = torch.empty(values.shape, dtype=values.dtype, pin_memory=True)
+            self.host.copy_(values, non_blocking=True)
+            self.done = torch.cuda.Event()
+            self.done.record(torch.cuda.current_stream(values.device))
+        else:
+            self.host, self.done = values.clone(), None
+
+    def get(self) -> np.ndarray:
+        if self.done is not None:
+            self.done.synchronize()
+        return self.host.numpy()
 
 
 def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
     """The recurrence on a stored matrix: its scalars stay on the device, and the host looks for a norm
-    below the threshold once per block of iterations (what ran past it is dropped)."""
+    below the threshold one block of iterations behind (what ran past it is dropped)."""
     n, device = mat.n, start.device
     if start.shape != (n,) or device != mat.val.device:
         raise RuntimeError(f"start must have shape [{n}] and be on the matrix's device.")
@@ -107,22 +127,31 @@ def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
     start = start.to(torch.complex128).resolve_conj().resolve_neg()
     first = start / torch.linalg.norm(torch.view_as_real(start))
     blocks = [first.reshape(1, n).contiguous()]
-    seen = []
+    looks, seen = [], []
     v, v_prev, beta_prev, done, stop = blocks[0][0], None, None, 0, None
+
+    def look(behind: int) -> int | None:
+        """The first iteration whose norm ends the recurrence, in all blocks but the last `behind`."""
+        while len(seen) < len(looks) - behind:
+            at = sum(values.shape[1] for values in seen)
+            seen.append(looks[len(seen)].get())
+            small = np.nonzero(seen[-1][1] < threshold)[0]
+            if len(small) and at + small[0] < step + 1:
+                return int(at + small[0])
+        return None
+
     # iteration k forms alpha[k], beta[k] and vector k + 1; the last one's beta and vector are not used
     while done < step + 2 and stop is None:
-        count = min(_LOOK_EVERY, step + 2 - done)
+        count = min(_LOOK_EVERY, max(1, done // 2), step + 2 - done)
         block = torch.empty((count, n), dtype=torch.complex128, device=device)
         scalars = torch.empty((2, count), dtype=torch.float64, device=device)  # alpha and beta of the block
         for k in range(count):
             mat.lanczos_step(v_prev, beta_prev, v, block[k], scalars[0, k], scalars[1, k], scratch)
             v_prev, v, beta_prev = v, block[k], scalars[1, k]
         blocks.append(block)
-        host = scalars.cpu().numpy()
-        seen.append(host)
-        small = [k for k in range(done, done + count) if k < step + 1 and host[1, k - done] < threshold]
-        stop = small[0] if small else None
+        looks.append(_Look(scalars))
         done += count
+        stop = look(1 if done < step + 2 else 0)
     used = (step + 1 if stop is None else stop) + 1  # vectors 0 .. used - 1
     host = np.concatenate(seen, axis=1)[:, :used]
     if used == 1:

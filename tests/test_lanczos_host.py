@@ -56,3 +56,21 @@ def test_more_steps_than_memory_has_places():
     energy, vector = solvers._lanczos_on_matrix(DenseMatrix(h), torch.from_numpy(start), 10**15, 1e-9)
     assert abs(energy - np.linalg.eigvalsh(h)[0]) <= 1e-8 * np.abs(h).sum()
     _check(energy, vector, h)
+
+
+@pytest.mark.parametrize("ends", [1, 2, 3, 5, 9, 14])
+@pytest.mark.parametrize("step", [0, 1, 2, 7, 12, 13, 100])
+def test_few_iterations_run_past_the_end(ends, step):
+    # an invariant subspace of `ends` vectors; the norm that ends the recurrence is seen within eight iterations
+    h = np.zeros((20, 20), dtype=np.complex128)
+    h[:ends, :ends], start = _matrix(ends, 10 + ends)
+    v = np.zeros(20, dtype=np.complex128)
+    v[:ends] = start
+    mat = DenseMatrix(h)
+    energy, vector = solvers._lanczos_on_matrix(mat, torch.from_numpy(v), step, 1e-9)
+    assert mat.steps <= min(step + 2, ends + min(7, ends + 1))
+    basis = min(step + 2, ends)
+    q, _ = np.linalg.qr(np.stack([np.linalg.matrix_power(h[:ends, :ends] / 10, k) @ start for k in range(basis)], axis=1))
+    want = np.linalg.eigvalsh(q.conj().T @ h[:ends, :ends] @ q)[0]
+    assert abs(energy - want) <= 1e-6 * np.abs(h).sum()
+    _check(energy, vector, h)
