@@ -237,6 +237,23 @@ __device__ __forceinline__ double2 row_times(const int64_t* __restrict__ row_ptr
     return make_double2(warp_sum(re), warp_sum(im));
 }
 
+// Row j of A times x, one thread, entries in order: for rows whose mean is below kFewEntries.
+constexpr int64_t kFewEntries = 4;
+
+__device__ __forceinline__ double2 short_row_times(const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
+                                                   const double2* __restrict__ val, const double2* __restrict__ x,
+                                                   int64_t j) {
+    const int64_t b = __ldg(row_ptr + j), e = __ldg(row_ptr + j + 1);
+    double re = 0.0, im = 0.0;
+    for (int64_t k = b; k < e; ++k) {
+        const double2 v = __ldg(val + k);
+        const double2 p = __ldg(x + __ldg(col + k));
+        re += v.x * p.x - v.y * p.y;
+        im += v.x * p.y + v.y * p.x;
+    }
+    return make_double2(re, im);
+}
+
 // y = A x, a warp per row.
 __global__ void __launch_bounds__(kThreads) spmv_kernel(int64_t n, const int64_t* __restrict__ row_ptr,
                                                         const int32_t* __restrict__ col,
@@ -293,9 +310,19 @@ __global__ void __launch_bounds__(kThreads) lanczos_product_kernel(int64_t n, co
                                                                    const double2* __restrict__ v,
                                                                    double2* __restrict__ w, double* __restrict__ parts) {
     __shared__ double s_warp[kWarpsPerBlock];
+    double dot = 0.0;
+    if (__ldg(row_ptr + n) < kFewEntries * n) {
+        for (int64_t j = (int64_t)blockIdx.x * kThreads + threadIdx.x; j < n; j += (int64_t)gridDim.x * kThreads) {
+            const double2 r = short_row_times(row_ptr, col, val, v, j);
+            w[j] = r;
+            const double2 p = __ldg(v + j);
+            dot += r.x * p.x + r.y * p.y;
+        }
+        store_part(dot, parts, s_warp);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * kWarpsPerBlock;
-    double dot = 0.0;
     for (int64_t j = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); j < n; j += warps) {
         const double2 r = row_times(row_ptr, col, val, v, j, lane);
         if (lane == 0) {
@@ -353,18 +380,8 @@ __global__ void __launch_bounds__(kThreads) spmv_rows_kernel(int64_t n, const in
                                                              const double2* __restrict__ val,
                                                              const double2* __restrict__ x, double2* __restrict__ y) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const int64_t b = __ldg(row_ptr + j), e = __ldg(row_ptr + j + 1);
-    double re = 0.0, im = 0.0;
-    for (int64_t k = b; k < e; ++k) {
-        const double2 v = __ldg(val + k);
-        const double2 p = __ldg(x + __ldg(col + k));
-        re += v.x * p.x - v.y * p.y;
-        im += v.x * p.y + v.y * p.x;
-    }
-    y[j] = make_double2(re, im);
+    if (j < n) y[j] = short_row_times(row_ptr, col, val, x, j);
 }
-constexpr int64_t kFewEntries = 4;
 
 // Y = A X for m vectors (X, Y row-major [n][m]): one warp per row, lane l
 // owns vectors l, l + 32, ...; the row's entries are read once per 32
