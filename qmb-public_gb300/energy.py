@@ -26,7 +26,7 @@ class _HermitianEnergy(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, ham: Hamiltonian, configs, psi):
-        psi = psi.detach().resolve_conj().contiguous()
+        given, psi = psi, psi.detach().resolve_conj().resolve_neg().contiguous()
         if psi.dtype == torch.complex64:
             hpsi = ham.apply_within_compensated(configs, psi, configs)
         else:
@@ -36,6 +36,8 @@ class _HermitianEnergy(torch.autograd.Function):
             scratch = torch.empty(1024, dtype=torch.float64, device=psi.device)
             _native.call("qmbx_energy", psi.shape[0], int(psi.dtype == torch.complex64), psi.data_ptr(), hpsi.data_ptr(),
                          sums.data_ptr(), scratch.data_ptr(), torch.cuda.current_stream(psi.device).cuda_stream)
+        if psi.dtype == torch.complex64 and psi.data_ptr() == given.data_ptr():
+            psi = psi.clone()  # a caller may change complex64 amplitudes in place before the backward
         ctx.save_for_backward(hpsi, psi, sums)
         return sums[0].clone()
 
