@@ -45,14 +45,20 @@ class _HermitianEnergy(torch.autograd.Function):
     def backward(ctx, grad):
         hpsi, psi, sums = ctx.saved_tensors
         # torch's gradient of a real loss in a complex input is 2 dL/dpsi*
-        if torch.is_grad_enabled():  # a graph of the gradient was asked for: it is linear in grad
+        composed = torch.is_grad_enabled()  # a graph of the gradient was asked for: it is linear in grad
+        if not composed:
+            grad = grad.to(torch.float64).contiguous()
+            try:
+                grad_ptr = grad.data_ptr()
+            except RuntimeError:  # a batch of gradients (is_grads_batched) has no memory of its own
+                composed = True
+        if composed:
             g = grad * 2.0 * (hpsi - sums[0] * psi.to(torch.complex128)) / sums[1]
             return None, None, g.to(psi.dtype)
-        grad = grad.to(torch.float64).contiguous()
         g = torch.empty_like(psi)
         with torch.cuda.device(psi.device):
             _native.call("qmbx_energy_grad", psi.shape[0], int(psi.dtype == torch.complex64), psi.data_ptr(),
-                         hpsi.data_ptr(), sums.data_ptr(), grad.data_ptr(), g.data_ptr(),
+                         hpsi.data_ptr(), sums.data_ptr(), grad_ptr, g.data_ptr(),
                          torch.cuda.current_stream(psi.device).cuda_stream)
         return None, None, g
 

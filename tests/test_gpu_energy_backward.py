@@ -30,3 +30,15 @@ def test_complex64_changed_in_place(cuda_device):
         psi.mul_(0.5)
     (got,) = torch.autograd.grad(energy, psi)
     assert (got - want).abs().max().item() <= 1e-6 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("dtype", [torch.complex128, torch.complex64])
+def test_batched_gradients(dtype, cuda_device):
+    ham, rows, psi = _system(cuda_device, dtype)
+    energy = variational_energy(ham, rows, psi.requires_grad_(True))
+    weights = torch.tensor([1.0, -2.0, 0.25], dtype=torch.float64, device=cuda_device)
+    (got,) = torch.autograd.grad(energy, psi, grad_outputs=weights, is_grads_batched=True, retain_graph=True)
+    tol = 1e-13 if dtype == torch.complex128 else 1e-6
+    for k in range(3):
+        (want,) = torch.autograd.grad(energy, psi, grad_outputs=weights[k], retain_graph=True)
+        assert (got[k] - want).abs().max().item() <= tol * want.abs().max().item()
