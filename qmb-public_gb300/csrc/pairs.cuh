@@ -656,8 +656,11 @@ int launch_pair_scan(const H& h, const PairWork& p, const void* table_host, cons
     const PairSet& a = swap ? p.j : p.i;
     const PairSet& b = swap ? p.i : p.j;
     const int shared = pair_shared_bytes<W>(sites);
-    // beside the static queues the planes of more than about 40 positions pass the default limit
-    QMBX_CUDA_TRY(cudaFuncSetAttribute(pair_scan_kernel<W, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
+    // Beside the static queues the planes of more than about 40 positions pass the default limit.  The limit is the
+    // kernel's, not the call's: every call sets what the longest rows of W words need, so that no thread lowers it
+    // between another's setting and launch.
+    QMBX_CUDA_TRY(cudaFuncSetAttribute(pair_scan_kernel<W, H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       pair_shared_bytes<W>(64 * W)));
     const PairContext<W, H> context{h, class_view(table_host, table_dev), part_view(table_host, table_dev, QMBX_PART_FWD),
                                     a.keys, b.keys, a.row, b.row, p.same ? 1 : 0, swap ? 1 : 0};
     QMBX_CUDA_TRY(cudaMemsetAsync(p.next, 0, 2 * sizeof(unsigned long long), s));
