@@ -566,8 +566,8 @@ __global__ void __launch_bounds__(kTailThreads)
                        PartView diag, const double2* __restrict__ psi, int64_t n_i, int order_shift,
                        int key_bits_total, int64_t k, FindCtl* ctl, unsigned int* bins, uint64_t* __restrict__ out) {
     __shared__ unsigned int s_bins[kSelectBins];
-    __shared__ int s_warp[32];
-    __shared__ int s_pick[3];  // digit, records below it, records at it
+    __shared__ long long s_warp[32];
+    __shared__ long long s_pick[3];  // digit, records below it, records at it
     const cg::grid_group grid = cg::this_grid();
     const int64_t e = (int64_t)ctl->n_emit;
     if (ctl->overflow || e > cap || e == 0 || (ctl->emit_from > 0 && e < k)) return;  // (the same for every block)
@@ -613,11 +613,11 @@ __global__ void __launch_bounds__(kTailThreads)
             if (v) atomicAdd(mine + b, v);
         }
         grid.sync();
-        // the digit where the remaining count is reached: two bins a thread (records number less than 2^31)
+        // the digit where the remaining count is reached: two bins a thread (2^31 records and more are summed)
         static_assert(kSelectBins == 2 * kTailThreads, "two bins a thread");
-        const int c0 = (int)((volatile unsigned int*)mine)[2 * threadIdx.x], c1 = (int)((volatile unsigned int*)mine)[2 * threadIdx.x + 1];
-        const int run = block_inclusive_scan(c0 + c1, s_warp);
-        const int before = run - c0 - c1;
+        const long long c0 = ((volatile unsigned int*)mine)[2 * threadIdx.x], c1 = ((volatile unsigned int*)mine)[2 * threadIdx.x + 1];
+        const long long run = block_inclusive_scan(c0 + c1, s_warp);
+        const long long before = run - c0 - c1;
         if (run >= need && before < need) {
             const bool second = before + c0 < need;
             s_pick[0] = 2 * threadIdx.x + (second ? 1 : 0);
