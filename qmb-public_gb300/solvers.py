@@ -93,9 +93,9 @@ def _lowest(alpha, beta):
     return float(vals[0]), vecs[:, 0]
 
 
-# Iterations of a block at most.  The host looks at a block's norms while the next one runs, so that at most the
-# rest of a block and one more run past the end of the recurrence; with blocks of 16 and a look behind each, a
-# start that ends after two iterations cost 16 (1,000,000 rows of an entry each: 1.2 ms of products became 25).
+# Iterations between two looks at most.  The host looks at the norms of some iterations while the next ones run,
+# so that at most seven run past the end of the recurrence; with 16 iterations and then a look, a start that ends
+# after two of them cost 16 (1,000,000 rows of an entry each: 1.2 ms of products became 25).
 _LOOK_EVERY = 4
 
 
@@ -141,14 +141,17 @@ def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
         return None
 
     # iteration k forms alpha[k], beta[k] and vector k + 1; the last one's beta and vector are not used
+    room = 0  # vectors that the last of `blocks` still has room for
     while done < step + 2 and stop is None:
         count = min(_LOOK_EVERY, max(1, done // 2), step + 2 - done)
-        block = torch.empty((count, n), dtype=torch.complex128, device=device)
-        scalars = torch.empty((2, count), dtype=torch.float64, device=device)  # alpha and beta of the block
+        scalars = torch.empty((2, count), dtype=torch.float64, device=device)  # alpha and beta of the iterations
         for k in range(count):
-            mat.lanczos_step(v_prev, beta_prev, v, block[k], scalars[0, k], scalars[1, k], scratch)
-            v_prev, v, beta_prev = v, block[k], scalars[1, k]
-        blocks.append(block)
+            if room == 0:
+                room = min(16, max(1, done + k))
+                blocks.append(torch.empty((room, n), dtype=torch.complex128, device=device))
+            v_next = blocks[-1][-room]
+            mat.lanczos_step(v_prev, beta_prev, v, v_next, scalars[0, k], scalars[1, k], scratch)
+            v_prev, v, beta_prev, room = v, v_next, scalars[1, k], room - 1
         looks.append(_Look(scalars))
         done += count
         stop = look(1 if done < step + 2 else 0)
@@ -157,12 +160,12 @@ def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
     if used == 1:
         return float(host[0, 0]), blocks[0][0]
     value, weights = _lowest(host[0], host[1, :used - 1])
+    weights = torch.from_numpy(weights.astype(np.complex128)).to(device)
     result, at = torch.zeros(n, dtype=torch.complex128, device=device), 0
     for block in blocks:
         part = block[:max(0, used - at)]
         if part.shape[0]:
-            weight = torch.from_numpy(weights[at:at + part.shape[0]].astype(np.complex128)).to(device)
-            result += weight @ part
+            result += weights[at:at + part.shape[0]] @ part
         at += block.shape[0]
     return value, result
 
