@@ -55,7 +55,7 @@ def lanczos_energy(ham: Hamiltonian, configs: torch.Tensor, step: int, threshold
         try:
             mat = ham.matrix(configs, max_entries=_matrix_budget(configs.device))
         except _native.QmbxError as error:
-            if "must be distinct" not in str(error):
+            if error.status != _native.QMBX_ERR_ARGUMENT or torch.unique(configs, dim=0).shape[0] == configs.shape[0]:
                 raise
             mat = None  # repeated rows: every iteration walks the terms
         if mat is not None and step >= 0:

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 import torch
 
+from qmb_gb300 import Hamiltonian, _native, lanczos_energy, terms
 from qmb_gb300.hamiltonian import HamiltonianMatrix
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +41,28 @@ def test_step(n, entries, cuda_device):
         whole = size + abs(a) * np.abs(v) + np.abs(prev)
         assert abs(b - np.linalg.norm(w)) <= (n + 16) * eps * np.linalg.norm(whole)
         assert np.all(np.abs(out.cpu().numpy() * b - w) <= 64 * eps * whole)
+
+
+def test_repeated_rows_whatever_the_message(cuda_device, monkeypatch):
+    table = terms.integral_hamiltonian_tables(5, seed=71)
+    rows = torch.from_numpy(terms.all_determinants(5, 2, 2)).to(cuda_device)
+    start = torch.from_numpy(terms.random_psi(2 * rows.shape[0], seed=72)).to(cuda_device)
+
+    class Reworded(Hamiltonian):
+        def matrix(self, configs, **options):
+            try:
+                return super().matrix(configs, **options)
+            except _native.QmbxError as error:
+                raise _native.QmbxError(error.status, "some other words") from error
+
+    twice = torch.cat([rows, rows])
+    want, _ = lanczos_energy(Hamiltonian(table, kind="fermi"), twice, 6, start=start, materialize=False)
+    got, _ = lanczos_energy(Reworded(table, kind="fermi"), twice, 6, start=start)
+    assert abs(got - want) <= 1e-10 * abs(want)
+
+    class Failing(Hamiltonian):
+        def matrix(self, configs, **options):
+            raise _native.QmbxError(_native.QMBX_ERR_ARGUMENT, "some other fault")
+
+    with pytest.raises(_native.QmbxError, match="other fault"):
+        lanczos_energy(Failing(table, kind="fermi"), rows, 6, start=start[:rows.shape[0]].contiguous())
