@@ -1096,8 +1096,8 @@ int apply_impl(const ApplyArgs& a, Arena& ws, cudaStream_t s) {
             }
         }
     }
-    if (scan && ((st = build_pairs<W>(rs_i, rs_j, h->n_sites, pairs, s)) != QMBX_OK ||
-                 (st = choose_pairs<W>(pairs, walked, s)) != QMBX_OK)) {
+    if (scan && ((st = choose_pairs<W>(pairs, rs_i, rs_j, walked, walk_part_of(a, scatter), s)) != QMBX_OK ||
+                 (st = build_pairs<W>(rs_i, rs_j, h->n_sites, pairs, s)) != QMBX_OK)) {
         return st;
     }
     if (scan || scatter || choose_walk(walk_part_of(a, scatter), walked.n, !deterministic_mode()) == Walk::kPivot) {
@@ -1633,6 +1633,7 @@ int adjoint_from_log_impl(const void* table_host, const void* table_dev, char* b
     if (scan) {
         pairs.i.count = rs_i.count;
         pairs.j.count = rs_j.count;
+        QMBX_CUDA_TRY(cudaMemsetAsync(pairs.next, 0, kPairCounters * sizeof(unsigned long long), s));
         if ((st = pair_apply<W>(a, rs_j, rs_i, pairs, g, res, &gate->pairs, s, kGroupSpmv, kGroupSpmv)) != QMBX_OK) return st;
     }
     QMBX_KERNEL(kGroupOther, s, apply_finalize_kernel<<<grid_for(n_i, kThreads), kThreads, 0, s>>>(res, rs_i.first, n_i, 1, out64, out32));

@@ -512,8 +512,8 @@ int matrix_walk(const void* table_host, const void* table_dev, const MatrixLayou
     const int* walk_rows = L.rows.count;
     if (adj.n > 0 && pairs != nullptr) {
         // the device chooses the scan or the walk below; the other finds no rows
-        int st = build_pairs<W>(L.rows, L.rows, header_of(table_host)->n_sites, *pairs, s);
-        if (st != QMBX_OK || (st = choose_pairs<W>(*pairs, L.rows, s)) != QMBX_OK) return st;
+        int st = choose_pairs<W>(*pairs, L.rows, L.rows, L.rows, adj, s);
+        if (st != QMBX_OK || (st = build_pairs<W>(L.rows, L.rows, header_of(table_host)->n_sites, *pairs, s)) != QMBX_OK) return st;
         walk_rows = pairs->gate + 1;
         const PartView fwd = part_view(table_host, table_dev, QMBX_PART_FWD);
         MatrixPairs<FILL> v{fwd.coef, L.count, L.cursor, col, val};

@@ -21,7 +21,9 @@ __device__ __forceinline__ int particles(const Key<W>& k) {
 // so a warp adds one count per number it sees.
 template <int W>
 __global__ void pair_count_kernel(const uint64_t* __restrict__ keys, const int32_t* __restrict__ unique,
-                                  const int* __restrict__ count, int* __restrict__ hist) {
+                                  const int* __restrict__ count, const int* __restrict__ gate,
+                                  int* __restrict__ hist) {
+    if (*gate == 0) return;
     const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = u < *count;
     const int p = live ? particles<W>(load_key<W>(keys, __ldg(unique + u))) : -1;
@@ -34,11 +36,13 @@ __global__ void pair_count_kernel(const uint64_t* __restrict__ keys, const int32
 template <int W>
 __global__ void __launch_bounds__(kThreads) pair_place_kernel(const uint64_t* __restrict__ keys,
                                                               const int32_t* __restrict__ unique,
-                                                              const int* __restrict__ count, int* __restrict__ hist,
+                                                              const int* __restrict__ count,
+                                                              const int* __restrict__ gate, int* __restrict__ hist,
                                                               uint64_t* __restrict__ out_keys,
                                                               int32_t* __restrict__ out_row) {
     constexpr int kNumbers = 64 * W + 1;
     __shared__ int s_base[kNumbers + 31];
+    if (*gate == 0) return;
     const int lane = threadIdx.x & 31;
     if (threadIdx.x < 32) {
         int before = 0;
@@ -80,8 +84,10 @@ __global__ void __launch_bounds__(kThreads) pair_place_kernel(const uint64_t* __
 // A warp forms one word of every plane: the ballot over its 32 rows.
 template <int W>
 __global__ void __launch_bounds__(kThreads) pair_planes_kernel(const uint64_t* __restrict__ keys,
-                                                               const int* __restrict__ count, int sites,
+                                                               const int* __restrict__ count,
+                                                               const int* __restrict__ gate, int sites,
                                                                uint32_t* __restrict__ planes) {
+    if (*gate == 0) return;
     constexpr int kWords = 32 * pair_words<W>();
     const int lane = threadIdx.x & 31;
     const int64_t word = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -108,8 +114,10 @@ __global__ void __launch_bounds__(kThreads) pair_planes_kernel(const uint64_t* _
 // The list of every row's occupied sites (PairSet::list), a thread per row.
 template <int W>
 __global__ void __launch_bounds__(kThreads) pair_list_kernel(const uint64_t* __restrict__ keys,
-                                                             const int* __restrict__ count, int sites,
+                                                             const int* __restrict__ count,
+                                                             const int* __restrict__ gate, int sites,
                                                              uint16_t* __restrict__ lists) {
+    if (*gate == 0) return;
     const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pos >= *count) return;
     const Key<W> k = load_key<W>(keys, pos);
@@ -126,11 +134,85 @@ __global__ void __launch_bounds__(kThreads) pair_list_kernel(const uint64_t* __r
     if (n & 1) list[n] = (uint16_t)(sites * 32);
 }
 
+// choose_pairs' sample: a warp takes a row a of the list side, 256 rows b of the other one from a place of its own,
+// and the sizes of a's pivot groups.  The last block to finish sums up.
+constexpr int kGateBlocks = 152;
+constexpr int kGateRows = 256;
+
 template <int W>
-__global__ void pair_gate_kernel(const uint64_t* __restrict__ keys, const int* __restrict__ count,
-                                 const int* __restrict__ walked, int* __restrict__ gate) {
-    const int64_t n = *count;
-    const bool scan = n > 0 && particles<W>(load_key<W>(keys, n - 1)) > 3;  // rows are ordered by number
+__global__ void __launch_bounds__(kThreads) pair_gate_kernel(UniqueRows<W> a, const int* __restrict__ a_count,
+                                                             UniqueRows<W> b, const int* __restrict__ b_count,
+                                                             const int2* __restrict__ groups, int same, int forced,
+                                                             const int* __restrict__ walked,
+                                                             unsigned long long* sums, int* __restrict__ gate) {
+    __shared__ uint8_t s_pos[kWarpsPerBlock][64 * W];
+    __shared__ unsigned int s_sum[3];  // close pairs, reached terms, particles
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int64_t na = *a_count, nb = *b_count;
+    if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+    if (na > 0 && nb > 0) {
+        const uint64_t w = (uint64_t)blockIdx.x * kWarpsPerBlock + warp;
+        const int64_t ia = (int64_t)(w * (uint64_t)na / (uint64_t)(kGateBlocks * kWarpsPerBlock));
+        const Key<W> c = a.get(ia);
+        const uint64_t start = ((w * 0x9E3779B97F4A7C15ull) >> 24) % (uint64_t)nb;
+        int close = 0, reach = 0, occ = 0;
+#pragma unroll
+        for (int u = 0; u < kGateRows / 32; ++u) {
+            int64_t ib = (int64_t)start + 32 * u + lane;
+            if (ib >= nb) ib %= nb;
+            const Key<W> k = b.get(ib);
+            int gone = 0, come = 0;
+#pragma unroll
+            for (int q = 0; q < W; ++q) {
+                gone += __popcll(c.w[q] & ~k.w[q]);
+                come += __popcll(k.w[q] & ~c.w[q]);
+            }
+            close += gone == come && gone <= 2 && !(same && ia == ib) ? 1 : 0;
+        }
+        uint8_t* pos = s_pos[warp];
+#pragma unroll
+        for (int h = 0; h < 2 * W; ++h) {
+            const uint32_t bits = (uint32_t)(c.w[h >> 1] >> (32 * (h & 1)));
+            if (bits >> lane & 1u) pos[occ + __popc(bits & lt)] = (uint8_t)(32 * h + lane);
+            occ += __popc(bits);
+        }
+        __syncwarp();
+        auto size = [&](int64_t g) {
+            const int2 se = __ldg(groups + g);
+            return se.y - se.x;
+        };
+        if (lane == 0) reach += size(0);
+        for (int i = lane; i < occ; i += 32) reach += size(qmbx_single_group(pos[i]));
+        for (int i = 0; i < occ; ++i) {
+            for (int k = i + 1 + lane; k < occ; k += 32) reach += size(qmbx_pair_group(W, pos[i], pos[k]));
+        }
+        close = (int)__reduce_add_sync(0xffffffffu, (unsigned)close);
+        const unsigned high = __reduce_add_sync(0xffffffffu, (unsigned)reach >> 16);
+        const unsigned low = __reduce_add_sync(0xffffffffu, (unsigned)reach & 0xffffu);
+        if (lane == 0) {
+            atomicAdd(&s_sum[0], (unsigned)close);
+            atomicAdd(&s_sum[2], (unsigned)occ);
+            atomicAdd(sums + 1, ((unsigned long long)high << 16) + low);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    atomicAdd(sums + 0, (unsigned long long)s_sum[0]);
+    atomicAdd(sums + 2, (unsigned long long)s_sum[2]);
+    __threadfence();
+    if (atomicAdd(sums + 3, 1ull) != gridDim.x - 1) return;
+    __threadfence();
+    constexpr double kWarps = (double)kGateBlocks * kWarpsPerBlock;
+    const double close = (double)*(volatile unsigned long long*)(sums + 0) / (kWarps * kGateRows);
+    const double reach = (double)*(volatile unsigned long long*)(sums + 1) / kWarps;
+    const double particles = (double)*(volatile unsigned long long*)(sums + 2) / kWarps;
+    const double pairs = (double)na * (double)nb * (same ? 0.5 : 1.0);
+    const double scan_ps = pairs * (0.0075 * particles + close * (same ? 80.0 : 40.0));
+    const double walk_ps = 5.0 * (double)*walked * reach;
+    // forced: still not for rows of three particles and fewer
+    const bool scan = na > 0 && nb > 0 && (forced ? particles > 3.0 : scan_ps < walk_ps);
     gate[0] = scan ? *walked : 0;
     gate[1] = scan ? 0 : *walked;
 }
@@ -138,9 +220,12 @@ __global__ void pair_gate_kernel(const uint64_t* __restrict__ keys, const int* _
 }  // namespace
 
 template <int W>
-int choose_pairs(const PairWork& p, const HashRows& walked, cudaStream_t s) {
-    const PairSet& a = pairs_swapped(p) ? p.j : p.i;
-    QMBX_KERNEL(kGroupOther, s, pair_gate_kernel<W><<<1, 1, 0, s>>>(a.keys, a.count, walked.count, p.gate));
+int choose_pairs(const PairWork& p, const HashRows& rows_i, const HashRows& rows_j, const HashRows& walked,
+                 const PartView& terms, cudaStream_t s) {
+    const HashRows& a = pairs_swapped(p) ? rows_j : rows_i;
+    const HashRows& b = pairs_swapped(p) ? rows_i : rows_j;
+    QMBX_CUDA_TRY(cudaMemsetAsync(p.next, 0, kPairCounters * sizeof(unsigned long long), s));
+    QMBX_KERNEL(kGroupOther, s, pair_gate_kernel<W><<<kGateBlocks, kThreads, 0, s>>>(UniqueRows<W>{a.keys, a.unique}, a.count, UniqueRows<W>{b.keys, b.unique}, b.count, terms.groups, p.same ? 1 : 0, pairs_forced() ? 1 : 0, walked.count, p.next + 2, p.gate));
     QMBX_LAUNCH_CHECK("pair_gate_kernel");
     return QMBX_OK;
 }
@@ -160,22 +245,22 @@ PairSet take_pair_set(Arena& ws, int64_t n, int sites) {
 }
 
 template <int W>
-int build_pair_set(const HashRows& rows, int sites, bool planes, bool lists, PairSet& out, cudaStream_t s) {
+int build_pair_set(const HashRows& rows, int sites, bool planes, bool lists, const int* gate, PairSet& out, cudaStream_t s) {
     out.count = rows.count;
     QMBX_CUDA_TRY(cudaMemsetAsync(out.hist, 0, 2 * (64 * W + 1) * sizeof(int), s));
     const int64_t words = (rows.n + pair_tile<W>() - 1) / pair_tile<W>() * 32 * pair_words<W>();
-    QMBX_KERNEL(kGroupKeys, s, pair_count_kernel<W><<<grid_for(rows.n, kThreads), kThreads, 0, s>>>(rows.keys, rows.unique, rows.count, out.hist));
-    QMBX_KERNEL(kGroupKeys, s, pair_place_kernel<W><<<grid_for(rows.n, kThreads), kThreads, 0, s>>>(rows.keys, rows.unique, rows.count, out.hist, out.keys, out.row));
-    if (lists) QMBX_KERNEL(kGroupKeys, s, pair_list_kernel<W><<<grid_for(rows.n, kThreads), kThreads, 0, s>>>(out.keys, rows.count, sites, out.list));
-    if (planes) QMBX_KERNEL(kGroupKeys, s, pair_planes_kernel<W><<<grid_for(words, kWarpsPerBlock), kThreads, 0, s>>>(out.keys, rows.count, sites, out.planes));
+    QMBX_KERNEL(kGroupKeys, s, pair_count_kernel<W><<<grid_for(rows.n, kThreads), kThreads, 0, s>>>(rows.keys, rows.unique, rows.count, gate, out.hist));
+    QMBX_KERNEL(kGroupKeys, s, pair_place_kernel<W><<<grid_for(rows.n, kThreads), kThreads, 0, s>>>(rows.keys, rows.unique, rows.count, gate, out.hist, out.keys, out.row));
+    if (lists) QMBX_KERNEL(kGroupKeys, s, pair_list_kernel<W><<<grid_for(rows.n, kThreads), kThreads, 0, s>>>(out.keys, rows.count, gate, sites, out.list));
+    if (planes) QMBX_KERNEL(kGroupKeys, s, pair_planes_kernel<W><<<grid_for(words, kWarpsPerBlock), kThreads, 0, s>>>(out.keys, rows.count, gate, sites, out.planes));
     QMBX_LAUNCH_CHECK("build_pair_set");
     return QMBX_OK;
 }
 
 #define QMBX_INSTANTIATE_PAIRS(W)                                     \
     template PairSet take_pair_set<W>(Arena&, int64_t, int);          \
-    template int choose_pairs<W>(const PairWork&, const HashRows&, cudaStream_t); \
-    template int build_pair_set<W>(const HashRows&, int, bool, bool, PairSet&, cudaStream_t);
+    template int choose_pairs<W>(const PairWork&, const HashRows&, const HashRows&, const HashRows&, const PartView&, cudaStream_t); \
+    template int build_pair_set<W>(const HashRows&, int, bool, bool, const int*, PairSet&, cudaStream_t);
 
 QMBX_INSTANTIATE_PAIRS(1)
 QMBX_INSTANTIATE_PAIRS(2)
@@ -210,12 +295,14 @@ bool pairs_scratch(const qmbx_table_header* h, int64_t n_i, int64_t n_j) {
     return pairs_possible(h) && n_i > 0 && n_j > 0 && (scan_pays(h, n_i, n_j) || n_i + n_j <= kPairsAlways);
 }
 
+bool pairs_forced() {
+    const char* e = getenv("QMBX_WALK");
+    return e != nullptr && e[0] == 's';
+}
+
 bool pairs_wanted(const qmbx_table_header* h, int64_t n_i, int64_t n_j) {
     if (!pairs_possible(h) || n_i <= 0 || n_j <= 0 || deterministic_mode()) return false;
-    const char* e = getenv("QMBX_WALK");
-    const char f = e != nullptr ? e[0] : 0;
-    if (f == 's') return true;
-    return f != 't' && f != 'g' && f != 'p' && scan_pays(h, n_i, n_j);
+    return pairs_forced() || (!walk_forced() && scan_pays(h, n_i, n_j));
 }
 
 int pair_chunk(int64_t n_list, int64_t n_planes, int tile) {

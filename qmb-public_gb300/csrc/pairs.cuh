@@ -67,7 +67,7 @@ struct PairSet {
 
 struct PairWork {
     PairSet i, j;          // j == i for the same rows on both sides
-    unsigned long long* next;  // work items handed out, and close pairs found (two counters)
+    unsigned long long* next;  // kPairCounters: work items handed out, close pairs found, then choose_pairs' sums
     uint2* pairs;          // pairs that stay: scan positions of the list side and the plane side
     unsigned int cap;      // places in `pairs`; pairs past them are looked up by the scan itself,
     void* overflow;        // with a PairQueue per warp of the grid
@@ -77,6 +77,7 @@ struct PairWork {
 
 // Blocks of the scan: four resident per SM on 152 SMs.
 constexpr int kPairBlocks = 608;
+constexpr int kPairCounters = 6;
 
 template <int W>
 PairSet take_pair_set(Arena& ws, int64_t n, int sites);
@@ -96,7 +97,7 @@ PairWork take_pair_work(Arena& ws, int64_t n_i, int64_t n_j, bool same, int site
     p.same = same;
     p.i = take_pair_set<W>(ws, n_i, sites);
     p.j = same ? p.i : take_pair_set<W>(ws, n_j, sites);
-    p.next = ws.take<unsigned long long>(2);
+    p.next = ws.take<unsigned long long>(kPairCounters);
     // room for a few dozen pairs a row (C2's 220,000 rows list 2.8M pairs); a
     // looked-up pair costs about 35 ps in the list and ten times that in the scan
     const double all = (double)(n_i > 0 ? n_i : 1) * (double)(n_j > 0 ? n_j : 1);
@@ -108,31 +109,39 @@ PairWork take_pair_work(Arena& ws, int64_t n_i, int64_t n_j, bool same, int site
     return p;
 }
 
-// Order the distinct rows of `rows`; form their planes, their position lists, or both.
+// Order the distinct rows of `rows`; form their planes, their position lists, or both (nothing when *gate is 0).
 template <int W>
-int build_pair_set(const HashRows& rows, int sites, bool planes, bool lists, PairSet& out, cudaStream_t s);
+int build_pair_set(const HashRows& rows, int sites, bool planes, bool lists, const int* gate, PairSet& out, cudaStream_t s);
 
-// p.gate from the prepared list side: the scan for rows of more than three
-// particles, else the walk (`walked`: its row set).  Rows of so few particles
-// reach few terms, and any two of them are likely to be close: 2,000 rows of
-// three among 60 sites take 222 us by the scan and 140 us by the walk, 2,000
-// of six 103 and 255 us.
-template <int W>
-int choose_pairs(const PairWork& p, const HashRows& walked, cudaStream_t s);
-
-// Prepare both sides.  The planes are made of the larger side, whose tiles
-// they fill better.
+// The planes are made of the larger side, whose tiles they fill better.
 inline bool pairs_swapped(const PairWork& p) { return !p.same && p.i.n > p.j.n; }
+
+// p.gate for the rows at hand, and cleared counters: the scan, or else the walk (`walked`: its row set; `terms`:
+// its part).  On the host only numbers of rows and terms are known; what the scan costs also depends on how many
+// pairs are close, and the walk on how many terms a row reaches, so a sample of both is taken on the device.
+// Costs, fitted to whole FP64 calls (times in ps, summed over the GPU): a pair of rows 0.0075 a particle; a close
+// pair 80 within one set (100 for its two lookups and hits, less 20 for the two hits a walk would find), 40 between
+// two; a reached term 5 in the walk.  (scan and walk, us)
+//   every determinant of 3 + 3 in 14 orbitals, 132,496 rows    11,934   4,093 (all of a row's 1,485 neighbours present)
+//   a random third of them, 40,000 rows                          1,184   1,016
+//   200,000 of the 4.0M of 5 + 5                                 2,783   7,914
+//   16,384 and 262,144 clustered rows of 7 + 7 in 26      515, 13,740   4,610, 70,543
+//   8,281 rows, all of 2 + 2 in 14                                  518     219
+template <int W>
+int choose_pairs(const PairWork& p, const HashRows& rows_i, const HashRows& rows_j, const HashRows& walked,
+                 const PartView& terms, cudaStream_t s);
+
+// Prepare both sides.
 template <int W>
 int build_pairs(const HashRows& rows_i, const HashRows& rows_j, int sites, PairWork& p, cudaStream_t s) {
     const bool swap = pairs_swapped(p);
-    int st = build_pair_set<W>(rows_i, sites, p.same || swap, p.same || !swap, p.i, s);
+    int st = build_pair_set<W>(rows_i, sites, p.same || swap, p.same || !swap, p.gate, p.i, s);
     if (st != QMBX_OK) return st;
     if (p.same) {
         p.j = p.i;
         return QMBX_OK;
     }
-    return build_pair_set<W>(rows_j, sites, !swap, swap, p.j, s);
+    return build_pair_set<W>(rows_j, sites, !swap, swap, p.gate, p.j, s);
 }
 
 // Whether the table can be scanned, whether a call on n_i x n_j rows has
@@ -140,6 +149,7 @@ int build_pairs(const HashRows& rows_i, const HashRows& rows_j, int sites, PairW
 bool pairs_possible(const qmbx_table_header* h);
 bool pairs_scratch(const qmbx_table_header* h, int64_t n_i, int64_t n_j);
 bool pairs_wanted(const qmbx_table_header* h, int64_t n_i, int64_t n_j);
+bool pairs_forced();  // QMBX_WALK names the scan
 
 // Rows of the list side per work item, for about 16 items per SM.
 int pair_chunk(int64_t n_list, int64_t n_planes, int tile);
@@ -647,7 +657,7 @@ __global__ void __launch_bounds__(kThreads, 3)
 }
 
 // Scan every pair of rows of i and j: hits of terms that lead from a row of i
-// to a row of j.
+// to a row of j.  The counters are cleared (choose_pairs).
 template <int W, class H>
 int launch_pair_scan(const H& h, const PairWork& p, const void* table_host, const void* table_dev, const int* gate,
                      cudaStream_t s, int group) {
@@ -663,7 +673,6 @@ int launch_pair_scan(const H& h, const PairWork& p, const void* table_host, cons
                                        pair_shared_bytes<W>(64 * W)));
     const PairContext<W, H> context{h, class_view(table_host, table_dev), part_view(table_host, table_dev, QMBX_PART_FWD),
                                     a.keys, b.keys, a.row, b.row, p.same ? 1 : 0, swap ? 1 : 0};
-    QMBX_CUDA_TRY(cudaMemsetAsync(p.next, 0, 2 * sizeof(unsigned long long), s));
     const int grid = pivot_grid() < kPairBlocks ? pivot_grid() : kPairBlocks;
     QMBX_KERNEL(group, s, pair_scan_kernel<W, H><<<grid, kThreads, shared, s>>>(
         context, b.planes, a.list, a.count, b.count, sites, pair_chunk(a.n, b.n, pair_tile<W>()), p.next, p.pairs, p.cap,

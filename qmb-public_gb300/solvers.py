@@ -100,9 +100,10 @@ _LOOK_EVERY = 4
 
 
 class _Look:
-    """A copy of a small device tensor on its way to the host."""
+    """A copy of the iterations' scalars on its way to the host."""
 
     def __init__(self, values: torch.Tensor):
+        self.count = values.shape[1]
         if values.is_cuda:
             self.host = torch.empty(values.shape, dtype=values.dtype, pin_memory=True)
             self.host.copy_(values, non_blocking=True)
@@ -119,7 +120,7 @@ class _Look:
 
 def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
     """The recurrence on a stored matrix: its scalars stay on the device, and the host looks for a norm
-    below the threshold one block of iterations behind (what ran past it is dropped)."""
+    below the threshold a few iterations behind (what ran past it is dropped)."""
     n, device = mat.n, start.device
     if start.shape != (n,) or device != mat.val.device:
         raise RuntimeError(f"start must have shape [{n}] and be on the matrix's device.")
@@ -127,19 +128,8 @@ def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
     start = start.to(torch.complex128).resolve_conj().resolve_neg()
     first = start / torch.linalg.norm(torch.view_as_real(start))
     blocks = [first.reshape(1, n).contiguous()]
-    looks, seen = [], []
+    looks, seen, at = [], [], 0
     v, v_prev, beta_prev, done, stop = blocks[0][0], None, None, 0, None
-
-    def look(behind: int) -> int | None:
-        """The first iteration whose norm ends the recurrence, in all blocks but the last `behind`."""
-        while len(seen) < len(looks) - behind:
-            at = sum(values.shape[1] for values in seen)
-            seen.append(looks[len(seen)].get())
-            small = np.nonzero(seen[-1][1] < threshold)[0]
-            if len(small) and at + small[0] < step + 1:
-                return int(at + small[0])
-        return None
-
     # iteration k forms alpha[k], beta[k] and vector k + 1; the last one's beta and vector are not used
     room = 0  # vectors that the last of `blocks` still has room for
     while done < step + 2 and stop is None:
@@ -154,7 +144,13 @@ def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
             v_prev, v, beta_prev, room = v, v_next, scalars[1, k], room - 1
         looks.append(_Look(scalars))
         done += count
-        stop = look(1 if done < step + 2 else 0)
+        # two iterations stay queued while the host looks at the ones before, so that the device does not wait
+        while stop is None and looks and (done == step + 2 or at + looks[0].count <= done - 2):
+            seen.append(looks.pop(0).get())
+            small = np.nonzero(seen[-1][1] < threshold)[0]
+            if len(small) and at + small[0] < step + 1:
+                stop = int(at + small[0])
+            at += seen[-1].shape[1]
     used = (step + 1 if stop is None else stop) + 1  # vectors 0 .. used - 1
     host = np.concatenate(seen, axis=1)[:, :used]
     if used == 1:
