@@ -804,14 +804,13 @@ int launch_diag(const D& dv, const HashRows& walk, const PartView& diag, cudaStr
 }
 
 // Pivot-major walk of the changing terms (results added into res by the
-// visitor's flush or hits) followed by a tiled pass over the diagonal terms.
-template <int W, class V, class D>
-int launch_pivot(const V& v, const D& dv, const HashRows& walk, const PartView& part, const PartView& diag,
-                 cudaStream_t s, int group = kGroupEnumerate, int diag_group = kGroupDiagonal) {
+// visitor's flush or hits).
+template <int W, class V>
+int launch_pivot(const V& v, const HashRows& walk, const PartView& part, cudaStream_t s, int group = kGroupEnumerate) {
     UniqueRows<W> src{walk.keys, walk.unique};
     QMBX_KERNEL(group, s, pivot_kernel<W><<<pivot_grid(), kThreads, 0, s>>>(v, src, walk.count, walk.n, part));
     QMBX_LAUNCH_CHECK("apply_within pivot walk");
-    return launch_diag<W>(dv, walk, diag, s, diag_group);
+    return QMBX_OK;
 }
 
 // Whether apply_within walks its input side (scatter) or its output side:
@@ -827,17 +826,50 @@ PartView walk_part_of(const ApplyArgs& a, bool scatter) {
                      scatter ? (a.adjoint ? QMBX_PART_ADJ : QMBX_PART_FWD) : (a.adjoint ? QMBX_PART_FWD : QMBX_PART_ADJ));
 }
 
+// The pass over the diagonal terms of the walked side's rows, added into res, where the walk or scan of the changing
+// terms leaves them out.  rows (device int, or NULL): its first *rows rows only.
+template <int W>
+int diag_pass(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_set, const void* val, double2* res,
+              const int* rows, cudaStream_t s, int group) {
+    const PartView diag = part_view(a.table_host, a.table_dev, QMBX_PART_DIAG);
+    const bool f32 = a.prec == Prec::F32C;
+    if (diag.n == 0 || (f32 && !a.include_diag)) return QMBX_OK;
+    const bool scatter = apply_scatter(a, in_set.n, out_set.n);
+    HashRows walk = scatter ? in_set : out_set;
+    if (rows != nullptr) walk.count = const_cast<int*>(rows);
+    const HashView look = scatter ? out_set.hash() : in_set.hash();
+#define QMBX_DIAG_CASE(CONJ, F32, SCATTER)                                                                                        \
+    return launch_diag<W>(DiagAdd<W, CONJ, F32, SCATTER>{{}, look, val, walk.unique, diag.coef, diag.coef32, res, a.log, a.same}, \
+                          walk, diag, s, group)
+    if (scatter) {
+        if (a.adjoint) {
+            if (f32) QMBX_DIAG_CASE(true, true, true);
+            QMBX_DIAG_CASE(true, false, true);
+        }
+        if (f32) QMBX_DIAG_CASE(false, true, true);
+        QMBX_DIAG_CASE(false, false, true);
+    }
+    if (a.adjoint) {
+        if (f32) QMBX_DIAG_CASE(true, true, false);
+        QMBX_DIAG_CASE(true, false, false);
+    }
+    if (f32) QMBX_DIAG_CASE(false, true, false);
+    QMBX_DIAG_CASE(false, false, false);
+#undef QMBX_DIAG_CASE
+}
+
 // The walks of apply_within over built row sets: amplitudes `val` per first
 // row of the input side, results into res per first row of the output side
 // (gather walks assign their rows' sums; scatter and pivot walks add, so the
 // caller clears res for them).  rows_gate (device int, or NULL): the walked
 // rows are the first *rows_gate of the walked set, so a launch can be made
-// conditional on device state without a host round trip.  reach (or NULL):
-// the walked rows' flags for a tiled walk (enumerate_reach_kernel).
+// conditional on device state without a host round trip.  diag_gate: the same
+// for a separate pass over the diagonal terms.  reach (or NULL): the walked
+// rows' flags for a tiled walk (enumerate_reach_kernel).
 template <int W>
 int walk_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_set, const void* val, double2* res,
-               const int* rows_gate, const uint8_t* reach, cudaStream_t s, int group = kGroupEnumerate,
-               int diag_group = kGroupDiagonal) {
+               const int* rows_gate, const int* diag_gate, const uint8_t* reach, cudaStream_t s,
+               int group = kGroupEnumerate, int diag_group = kGroupDiagonal) {
     const int64_t n_in = a.adjoint ? a.n_j : a.n_i;
     const int64_t n_out = a.adjoint ? a.n_i : a.n_j;
     int st = QMBX_OK;
@@ -868,8 +900,7 @@ int walk_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_s
 #define QMBX_PIVOT_CASE(CONJ, F32, SCATTER)                                                                      \
     {                                                                                                            \
         PivotHits<W, CONJ, F32, SCATTER> v{{}, look, val, walk.unique, part.coef, part.coef32, res}; v.log = a.log;             \
-        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res}; dv.log = a.log; dv.self = a.same;                           \
-        st = launch_pivot<W>(v, dv, walk, part, diag, s, group, diag_group);                                                        \
+        st = launch_pivot<W>(v, walk, part, s, group);                                                        \
     }
         const bool f32 = a.prec == Prec::F32C;
         if (scatter) {
@@ -923,81 +954,27 @@ int walk_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_s
             }
         }
     }
-    if (st != QMBX_OK) return st;
-    if (grouped && diag.n > 0) {
-        const bool f32 = a.prec == Prec::F32C;
-#define QMBX_DIAG_CASE(CONJ, F32, SCATTER)                                              \
-    {                                                                                   \
-        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res}; dv.log = a.log; dv.self = a.same;  \
-        st = launch_diag<W>(dv, walk, diag, s, diag_group);                                   \
-    }
-        if (scatter) {
-            if (a.adjoint) {
-                if (f32) QMBX_DIAG_CASE(true, true, true) else QMBX_DIAG_CASE(true, false, true)
-            } else {
-                if (f32) QMBX_DIAG_CASE(false, true, true) else QMBX_DIAG_CASE(false, false, true)
-            }
-        } else {
-            if (a.adjoint) {
-                if (f32) QMBX_DIAG_CASE(true, true, false) else QMBX_DIAG_CASE(true, false, false)
-            } else {
-                if (f32) QMBX_DIAG_CASE(false, true, false) else QMBX_DIAG_CASE(false, false, false)
-            }
-        }
-#undef QMBX_DIAG_CASE
-        if (st != QMBX_OK) return st;
-    }
-    return QMBX_OK;
+    if (st != QMBX_OK || !(pivot || grouped)) return st;
+    return diag_pass<W>(a, in_set, out_set, val, res, diag_gate, s, diag_group);
 }
 
-// apply_within by the pair scan: hits of the changing terms added into res
-// (cleared by the caller), then the diagonal terms over the side the walks
-// would take.  gate (device int): nothing is scanned when it is 0, and it is
-// the number of rows of the diagonal pass.
+// The changing terms of apply_within by the pair scan: hits added into res
+// (cleared by the caller).  gate (device int): nothing is scanned when it is 0.
 template <int W>
-int pair_apply(const ApplyArgs& a, const HashRows& in_set, const HashRows& out_set, const PairWork& pairs,
-               const void* val, double2* res, const int* gate, cudaStream_t s, int group = kGroupEnumerate,
-               int diag_group = kGroupDiagonal) {
+int pair_apply(const ApplyArgs& a, const PairWork& pairs, const void* val, double2* res, const int* gate,
+               cudaStream_t s, int group = kGroupEnumerate) {
     const PartView fwd = part_view(a.table_host, a.table_dev, QMBX_PART_FWD);
-    const PartView diag = part_view(a.table_host, a.table_dev, QMBX_PART_DIAG);
     const bool f32 = a.prec == Prec::F32C;
-    int st = QMBX_OK;
-#define QMBX_PAIR_CASE(CONJ, F32)                                                                        \
-    {                                                                                                    \
-        PairHits<W, CONJ, F32> v{val, fwd.coef, fwd.coef32, res, a.log};                                 \
-        st = launch_pair_scan<W>(v, pairs, a.table_host, a.table_dev, gate, s, group);                   \
-    }
+#define QMBX_PAIR_CASE(CONJ, F32)                                                                      \
+    return launch_pair_scan<W>(PairHits<W, CONJ, F32>{val, fwd.coef, fwd.coef32, res, a.log}, pairs,   \
+                               a.table_host, a.table_dev, gate, s, group)
     if (a.adjoint) {
-        if (f32) QMBX_PAIR_CASE(true, true) else QMBX_PAIR_CASE(true, false)
-    } else {
-        if (f32) QMBX_PAIR_CASE(false, true) else QMBX_PAIR_CASE(false, false)
+        if (f32) QMBX_PAIR_CASE(true, true);
+        QMBX_PAIR_CASE(true, false);
     }
+    if (f32) QMBX_PAIR_CASE(false, true);
+    QMBX_PAIR_CASE(false, false);
 #undef QMBX_PAIR_CASE
-    if (st != QMBX_OK || diag.n == 0 || !(a.prec == Prec::F64 || a.include_diag)) return st;
-    const bool scatter = apply_scatter(a, in_set.n, out_set.n);
-    HashRows walk = scatter ? in_set : out_set;
-    walk.count = const_cast<int*>(gate);
-    const HashView look = scatter ? out_set.hash() : in_set.hash();
-#define QMBX_DIAG_CASE(CONJ, F32, SCATTER)                                                                      \
-    {                                                                                                           \
-        DiagAdd<W, CONJ, F32, SCATTER> dv{{}, look, val, walk.unique, diag.coef, diag.coef32, res, a.log, a.same};      \
-        st = launch_diag<W>(dv, walk, diag, s, diag_group);                                                \
-    }
-    if (scatter) {
-        if (a.adjoint) {
-            if (f32) QMBX_DIAG_CASE(true, true, true) else QMBX_DIAG_CASE(true, false, true)
-        } else {
-            if (f32) QMBX_DIAG_CASE(false, true, true) else QMBX_DIAG_CASE(false, false, true)
-        }
-    } else {
-        if (a.adjoint) {
-            if (f32) QMBX_DIAG_CASE(true, true, false) else QMBX_DIAG_CASE(true, false, false)
-        } else {
-            if (f32) QMBX_DIAG_CASE(false, true, false) else QMBX_DIAG_CASE(false, false, false)
-        }
-    }
-#undef QMBX_DIAG_CASE
-    return st;
 }
 
 // The pair scan's scratch of a call behind the first `base` bytes of its
@@ -1110,11 +1087,15 @@ int apply_impl(const ApplyArgs& a, Arena& ws, cudaStream_t s) {
         QMBX_CUDA_TRY(cudaMemsetAsync(a.log.diag_rows, 0xff, (size_t)a.log_rows * sizeof(int2), s));
         QMBX_KERNEL(kGroupOther, s, log_head_kernel<<<1, 1, 0, s>>>(a.log_head, scatter ? 0 : 1, scan ? pairs.gate : nullptr, a.n_i, a.n_j, a.log.cap));
     }
-    // the device chooses one of the two; the other finds no rows
-    if (scan && (st = pair_apply<W>(a, in_set, out_set, pairs, val, res, pairs.gate, s)) != QMBX_OK) return st;
-    if ((st = walk_apply<W>(a, in_set, out_set, val, res, scan ? pairs.gate + 1 : nullptr, reach, s,
-                            scan ? kGroupOther : kGroupEnumerate, scan ? kGroupOther : kGroupDiagonal)) != QMBX_OK) {
-        return st;
+    if (!scan) {
+        if ((st = walk_apply<W>(a, in_set, out_set, val, res, nullptr, nullptr, reach, s)) != QMBX_OK) return st;
+    } else {
+        // the device chooses one of the two, the other finds no rows; the diagonal pass serves both, but a tiled walk
+        // has the diagonal terms within
+        const bool tiled = choose_walk(walk_part_of(a, scatter), walked.n, true) == Walk::kTiled;
+        if ((st = pair_apply<W>(a, pairs, val, res, pairs.gate, s)) != QMBX_OK) return st;
+        if (tiled && (st = diag_pass<W>(a, in_set, out_set, val, res, pairs.gate, s, kGroupDiagonal)) != QMBX_OK) return st;
+        if ((st = walk_apply<W>(a, in_set, out_set, val, res, pairs.gate + 1, nullptr, reach, s, kGroupOther)) != QMBX_OK) return st;
     }
     QMBX_KERNEL(kGroupOther, s, apply_finalize_kernel<<<grid_for(n_out, kThreads), kThreads, 0, s>>>(res, out_set.first, n_out, a.adjoint ? 1 : 0, a.out64, a.out32));
     QMBX_LAUNCH_CHECK("apply_finalize_kernel");
@@ -1627,14 +1608,17 @@ int adjoint_from_log_impl(const void* table_host, const void* table_dev, char* b
     }
     QMBX_LAUNCH_CHECK("adjoint from log");
     // an incomplete record: the adjoint walk (its walked rows gated by the device count; 0 otherwise)
-    int st = walk_apply<W>(a, rs_j, rs_i, g, res, &gate->rows, nullptr, s, kGroupSpmv, kGroupSpmv);
+    int st = walk_apply<W>(a, rs_j, rs_i, g, res, &gate->rows, &gate->rows, nullptr, s, kGroupSpmv, kGroupSpmv);
     if (st != QMBX_OK) return st;
     // or the scan again, over the prepared rows the forward left in the buffer
     if (scan) {
         pairs.i.count = rs_i.count;
         pairs.j.count = rs_j.count;
         QMBX_CUDA_TRY(cudaMemsetAsync(pairs.next, 0, kPairCounters * sizeof(unsigned long long), s));
-        if ((st = pair_apply<W>(a, rs_j, rs_i, pairs, g, res, &gate->pairs, s, kGroupSpmv, kGroupSpmv)) != QMBX_OK) return st;
+        if ((st = pair_apply<W>(a, pairs, g, res, &gate->pairs, s, kGroupSpmv)) != QMBX_OK ||
+            (st = diag_pass<W>(a, rs_j, rs_i, g, res, &gate->pairs, s, kGroupSpmv)) != QMBX_OK) {
+            return st;
+        }
     }
     QMBX_KERNEL(kGroupOther, s, apply_finalize_kernel<<<grid_for(n_i, kThreads), kThreads, 0, s>>>(res, rs_i.first, n_i, 1, out64, out32));
     QMBX_KERNEL(kGroupOther, s, log_poison_kernel<<<grid_for(n_i, kThreads), kThreads, 0, s>>>(gate, n_i, out64, out32));

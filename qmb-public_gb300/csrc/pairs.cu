@@ -81,12 +81,15 @@ __global__ void __launch_bounds__(kThreads) pair_place_kernel(const uint64_t* __
     }
 }
 
-// A warp forms one word of every plane: the ballot over its 32 rows.
+// The planes of the rows (a warp forms one word of every plane: the ballot
+// over its 32 rows), the list of every row's occupied sites (PairSet::list, a
+// thread per row), or both.
 template <int W>
-__global__ void __launch_bounds__(kThreads) pair_planes_kernel(const uint64_t* __restrict__ keys,
-                                                               const int* __restrict__ count,
-                                                               const int* __restrict__ gate, int sites,
-                                                               uint32_t* __restrict__ planes) {
+__global__ void __launch_bounds__(kThreads) pair_form_kernel(const uint64_t* __restrict__ keys,
+                                                             const int* __restrict__ count,
+                                                             const int* __restrict__ gate, int sites,
+                                                             uint32_t* __restrict__ planes,
+                                                             uint16_t* __restrict__ lists) {
     if (*gate == 0) return;
     constexpr int kWords = 32 * pair_words<W>();
     const int lane = threadIdx.x & 31;
@@ -97,41 +100,33 @@ __global__ void __launch_bounds__(kThreads) pair_planes_kernel(const uint64_t* _
     const int64_t pos = 32 * word + lane;
     Key<W> k{};
     if (pos < n) k = load_key<W>(keys, pos);
-    uint32_t* out = planes + word / kWords * sites * kWords + word % kWords;
+    if (planes != nullptr) {
+        uint32_t* out = planes + word / kWords * sites * kWords + word % kWords;
 #pragma unroll
-    for (int q = 0; q < 2 * W; ++q) {
-        uint32_t mine = 0;
+        for (int q = 0; q < 2 * W; ++q) {
+            uint32_t mine = 0;
 #pragma unroll
-        for (int b = 0; b < 32; ++b) {
-            const int bit = (32 * (q & 1) + b) ^ 56;  // site 32 q + b of the row
-            const uint32_t m = __ballot_sync(0xffffffffu, (k.w[q >> 1] >> bit) & 1ull);
-            if (lane == b) mine = m;
-        }
-        if (32 * q + lane < sites) out[(32 * q + lane) * kWords] = mine;
-    }
-}
-
-// The list of every row's occupied sites (PairSet::list), a thread per row.
-template <int W>
-__global__ void __launch_bounds__(kThreads) pair_list_kernel(const uint64_t* __restrict__ keys,
-                                                             const int* __restrict__ count,
-                                                             const int* __restrict__ gate, int sites,
-                                                             uint16_t* __restrict__ lists) {
-    if (*gate == 0) return;
-    const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos >= *count) return;
-    const Key<W> k = load_key<W>(keys, pos);
-    uint16_t* list = lists + pos * sites;
-    int n = 0;
-#pragma unroll
-    for (int q = 0; q < W; ++q) {
-        for (uint64_t m = k.w[q]; m != 0;) {
-            const int bit = 63 - __clzll((long long)m);
-            m ^= 1ull << bit;
-            list[n++] = (uint16_t)((64 * q + (bit ^ 56)) * 32);  // key bit to site (see format.h)
+            for (int b = 0; b < 32; ++b) {
+                const int bit = (32 * (q & 1) + b) ^ 56;  // site 32 q + b of the row
+                const uint32_t m = __ballot_sync(0xffffffffu, (k.w[q >> 1] >> bit) & 1ull);
+                if (lane == b) mine = m;
+            }
+            if (32 * q + lane < sites) out[(32 * q + lane) * kWords] = mine;
         }
     }
-    if (n & 1) list[n] = (uint16_t)(sites * 32);
+    if (lists != nullptr && pos < n) {
+        uint16_t* list = lists + pos * sites;
+        int at = 0;
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+            for (uint64_t m = k.w[q]; m != 0;) {
+                const int bit = 63 - __clzll((long long)m);
+                m ^= 1ull << bit;
+                list[at++] = (uint16_t)((64 * q + (bit ^ 56)) * 32);  // key bit to site (see format.h)
+            }
+        }
+        if (at & 1) list[at] = (uint16_t)(sites * 32);
+    }
 }
 
 // choose_pairs' sample: a warp takes a row a of the list side, 256 rows b of the other one from a place of its own,
@@ -224,14 +219,14 @@ int choose_pairs(const PairWork& p, const HashRows& rows_i, const HashRows& rows
                  const PartView& terms, cudaStream_t s) {
     const HashRows& a = pairs_swapped(p) ? rows_j : rows_i;
     const HashRows& b = pairs_swapped(p) ? rows_i : rows_j;
-    QMBX_CUDA_TRY(cudaMemsetAsync(p.next, 0, kPairCounters * sizeof(unsigned long long), s));
+    QMBX_CUDA_TRY(cudaMemsetAsync(p.next, 0, p.clear_bytes, s));
     QMBX_KERNEL(kGroupOther, s, pair_gate_kernel<W><<<kGateBlocks, kThreads, 0, s>>>(UniqueRows<W>{a.keys, a.unique}, a.count, UniqueRows<W>{b.keys, b.unique}, b.count, terms.groups, p.same ? 1 : 0, pairs_forced() ? 1 : 0, walked.count, p.next + 2, p.gate));
     QMBX_LAUNCH_CHECK("pair_gate_kernel");
     return QMBX_OK;
 }
 
 template <int W>
-PairSet take_pair_set(Arena& ws, int64_t n, int sites) {
+PairSet take_pair_set(Arena& ws, int64_t n, int sites, int* hist) {
     PairSet out{};
     const uint64_t cap = (uint64_t)(n > 0 ? n : 1);
     const uint64_t tiles = (cap + pair_tile<W>() - 1) / pair_tile<W>();
@@ -240,25 +235,23 @@ PairSet take_pair_set(Arena& ws, int64_t n, int sites) {
     out.row = ws.take<int32_t>(cap);
     out.planes = ws.take<uint32_t>(tiles * (uint64_t)sites * 32 * pair_words<W>());
     out.list = ws.take<uint16_t>((cap + kPairRun - 1) / kPairRun * kPairRun * (uint64_t)sites);
-    out.hist = ws.take<int>(2 * (64 * W + 1));
+    out.hist = hist;
     return out;
 }
 
 template <int W>
 int build_pair_set(const HashRows& rows, int sites, bool planes, bool lists, const int* gate, PairSet& out, cudaStream_t s) {
     out.count = rows.count;
-    QMBX_CUDA_TRY(cudaMemsetAsync(out.hist, 0, 2 * (64 * W + 1) * sizeof(int), s));
     const int64_t words = (rows.n + pair_tile<W>() - 1) / pair_tile<W>() * 32 * pair_words<W>();
     QMBX_KERNEL(kGroupKeys, s, pair_count_kernel<W><<<grid_for(rows.n, kThreads), kThreads, 0, s>>>(rows.keys, rows.unique, rows.count, gate, out.hist));
     QMBX_KERNEL(kGroupKeys, s, pair_place_kernel<W><<<grid_for(rows.n, kThreads), kThreads, 0, s>>>(rows.keys, rows.unique, rows.count, gate, out.hist, out.keys, out.row));
-    if (lists) QMBX_KERNEL(kGroupKeys, s, pair_list_kernel<W><<<grid_for(rows.n, kThreads), kThreads, 0, s>>>(out.keys, rows.count, gate, sites, out.list));
-    if (planes) QMBX_KERNEL(kGroupKeys, s, pair_planes_kernel<W><<<grid_for(words, kWarpsPerBlock), kThreads, 0, s>>>(out.keys, rows.count, gate, sites, out.planes));
+    QMBX_KERNEL(kGroupKeys, s, pair_form_kernel<W><<<grid_for(words, kWarpsPerBlock), kThreads, 0, s>>>(out.keys, rows.count, gate, sites, planes ? out.planes : nullptr, lists ? out.list : nullptr));
     QMBX_LAUNCH_CHECK("build_pair_set");
     return QMBX_OK;
 }
 
 #define QMBX_INSTANTIATE_PAIRS(W)                                     \
-    template PairSet take_pair_set<W>(Arena&, int64_t, int);          \
+    template PairSet take_pair_set<W>(Arena&, int64_t, int, int*);    \
     template int choose_pairs<W>(const PairWork&, const HashRows&, const HashRows&, const HashRows&, const PartView&, cudaStream_t); \
     template int build_pair_set<W>(const HashRows&, int, bool, bool, const int*, PairSet&, cudaStream_t);
 

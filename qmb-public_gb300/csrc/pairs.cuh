@@ -67,7 +67,9 @@ struct PairSet {
 
 struct PairWork {
     PairSet i, j;          // j == i for the same rows on both sides
-    unsigned long long* next;  // kPairCounters: work items handed out, close pairs found, then choose_pairs' sums
+    // work items handed out, close pairs found, choose_pairs' sums; then both sets' hist, all cleared at once
+    unsigned long long* next;
+    uint64_t clear_bytes;
     uint2* pairs;          // pairs that stay: scan positions of the list side and the plane side
     unsigned int cap;      // places in `pairs`; pairs past them are looked up by the scan itself,
     void* overflow;        // with a PairQueue per warp of the grid
@@ -78,9 +80,14 @@ struct PairWork {
 // Blocks of the scan: four resident per SM on 152 SMs.
 constexpr int kPairBlocks = 608;
 constexpr int kPairCounters = 6;
+// Words of 64 bits for a set's hist (a count for each of 0 .. 64 W particles, twice, as ints).
+template <int W>
+constexpr int pair_hist() {
+    return 64 * W + 1;
+}
 
 template <int W>
-PairSet take_pair_set(Arena& ws, int64_t n, int sites);
+PairSet take_pair_set(Arena& ws, int64_t n, int sites, int* hist);
 
 // Hits waiting to be applied: one a lane, or four where they are recorded,
 // since every drain's atomic meets the same counter (3.6M recorded FP32 hits:
@@ -95,9 +102,11 @@ template <int W>
 PairWork take_pair_work(Arena& ws, int64_t n_i, int64_t n_j, bool same, int sites) {
     PairWork p{};
     p.same = same;
-    p.i = take_pair_set<W>(ws, n_i, sites);
-    p.j = same ? p.i : take_pair_set<W>(ws, n_j, sites);
-    p.next = ws.take<unsigned long long>(kPairCounters);
+    p.clear_bytes = (kPairCounters + 2 * pair_hist<W>()) * sizeof(unsigned long long);
+    p.next = ws.take<unsigned long long>(kPairCounters + 2 * pair_hist<W>());
+    int* hist = p.next != nullptr ? reinterpret_cast<int*>(p.next + kPairCounters) : nullptr;
+    p.i = take_pair_set<W>(ws, n_i, sites, hist);
+    p.j = same ? p.i : take_pair_set<W>(ws, n_j, sites, hist != nullptr ? hist + 2 * pair_hist<W>() : nullptr);
     // room for a few dozen pairs a row (C2's 220,000 rows list 2.8M pairs); a
     // looked-up pair costs about 35 ps in the list and ten times that in the scan
     const double all = (double)(n_i > 0 ? n_i : 1) * (double)(n_j > 0 ? n_j : 1);
