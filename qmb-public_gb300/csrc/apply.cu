@@ -1347,7 +1347,7 @@ int attach_log(ApplyArgs& a, void* log, uint64_t log_bytes, int64_t cap, void** 
     LogLayout L;
     int st = log_layout(a.table_host, a.n_i, n_j, a.same, cap, L);
     if (st != QMBX_OK) return st;
-    if (log_bytes < L.total) {
+    if (log_bytes < L.ws + L.ws_needed) {
         return fail(QMBX_ERR_WORKSPACE, "a log of %lld hits on %lld x %lld rows needs %llu bytes", (long long)cap,
                     (long long)a.n_i, (long long)n_j, (unsigned long long)L.total);
     }
@@ -1360,7 +1360,7 @@ int attach_log(ApplyArgs& a, void* log, uint64_t log_bytes, int64_t cap, void** 
     a.log.diag_val = reinterpret_cast<double2*>(b + L.diag_val);
     a.log_rows = a.n_i > n_j ? a.n_i : n_j;
     *ws = b + L.ws;
-    *ws_bytes = L.ws_bytes;
+    *ws_bytes = log_bytes - L.ws;
     return QMBX_OK;
 }
 
@@ -1641,7 +1641,9 @@ int adjoint_from_log(const void* table_host, const void* table_dev, const void* 
     }
     LogLayout L;
     if ((st = log_layout(table_host, n_i, n_j, same, cap, L)) != QMBX_OK) return st;
-    if (log_bytes < L.total) return fail(QMBX_ERR_ARGUMENT, "log buffer smaller than its layout");
+    // (optional scratch may have been granted otherwise when the buffer was sized: its users look at L.ws_bytes)
+    if (log_bytes < L.ws + L.ws_needed) return fail(QMBX_ERR_ARGUMENT, "log buffer smaller than its layout");
+    L.ws_bytes = log_bytes - L.ws;
     if (n_i > 0 && out64 == nullptr && out32 == nullptr) return fail(QMBX_ERR_ARGUMENT, "no output given");
     if (n_j > 0 && g == nullptr) return fail(QMBX_ERR_ARGUMENT, "g_j must not be NULL");
     if (n_i == 0) return QMBX_OK;

@@ -279,18 +279,21 @@ bool scan_pays(const qmbx_table_header* h, int64_t n_i, int64_t n_j) {
     return other * sites < 250.0 * terms && walked * terms > 1e8 && terms > 0.01 * moves * moves;
 }
 
-// Small calls always have scratch for the scan, so that it can be forced on them.
-constexpr int64_t kPairsAlways = int64_t(1) << 17;
+// Calls on more rows have no scratch for a scan that QMBX_WALK forces on them.
+constexpr int64_t kPairsForced = int64_t(1) << 17;
 
 }  // namespace
-
-bool pairs_scratch(const qmbx_table_header* h, int64_t n_i, int64_t n_j) {
-    return pairs_possible(h) && n_i > 0 && n_j > 0 && (scan_pays(h, n_i, n_j) || n_i + n_j <= kPairsAlways);
-}
 
 bool pairs_forced() {
     const char* e = getenv("QMBX_WALK");
     return e != nullptr && e[0] == 's';
+}
+
+// Scratch is for the sizes that may be scanned, and for small calls while QMBX_WALK forces the scan on them: every
+// call compares what it was given with what its scan needs, and walks without.
+bool pairs_scratch(const qmbx_table_header* h, int64_t n_i, int64_t n_j) {
+    if (!pairs_possible(h) || n_i <= 0 || n_j <= 0) return false;
+    return scan_pays(h, n_i, n_j) || (pairs_forced() && n_i + n_j <= kPairsForced);
 }
 
 bool pairs_wanted(const qmbx_table_header* h, int64_t n_i, int64_t n_j) {

@@ -107,13 +107,15 @@ PairWork take_pair_work(Arena& ws, int64_t n_i, int64_t n_j, bool same, int site
     int* hist = p.next != nullptr ? reinterpret_cast<int*>(p.next + kPairCounters) : nullptr;
     p.i = take_pair_set<W>(ws, n_i, sites, hist);
     p.j = same ? p.i : take_pair_set<W>(ws, n_j, sites, hist != nullptr ? hist + 2 * pair_hist<W>() : nullptr);
-    // room for a few dozen pairs a row (C2's 220,000 rows list 2.8M pairs); a
-    // looked-up pair costs about 35 ps in the list and ten times that in the scan
-    const double all = (double)(n_i > 0 ? n_i : 1) * (double)(n_j > 0 ? n_j : 1);
+    // Room for a few dozen pairs a row (20,000 x 200,000 rows of 10 among 28 list 2.8M pairs).  A pair past it costs
+    // up to half again as much where most pairs connect (140 against 100 ps), more where few do.
+    const double rows_i = (double)(n_i > 0 ? n_i : 1), rows_j = (double)(n_j > 0 ? n_j : 1);
+    const double all = same ? 0.5 * rows_i * (rows_i - 1.0) + 1.0 : rows_i * rows_j;
     const double room = (double)(1 << 22) + 32.0 * ((double)n_i + (double)n_j);
     p.cap = (unsigned int)(all < room ? all : room < 4e9 ? room : 4e9);
     p.pairs = ws.take<uint2>(p.cap);
-    p.overflow = ws.take<PairQueue>((uint64_t)kPairBlocks * kWarpsPerBlock);
+    // a list with a place for every pair does not run over
+    p.overflow = (double)p.cap < all ? ws.take<PairQueue>((uint64_t)kPairBlocks * kWarpsPerBlock) : nullptr;
     p.gate = ws.take<int>(2);
     return p;
 }
@@ -154,7 +156,7 @@ int build_pairs(const HashRows& rows_i, const HashRows& rows_j, int sites, PairW
 }
 
 // Whether the table can be scanned, whether a call on n_i x n_j rows has
-// scratch for it, and whether it should be (pairs.cu).
+// scratch for it, and whether it may be (pairs.cu).
 bool pairs_possible(const qmbx_table_header* h);
 bool pairs_scratch(const qmbx_table_header* h, int64_t n_i, int64_t n_j);
 bool pairs_wanted(const qmbx_table_header* h, int64_t n_i, int64_t n_j);

@@ -57,3 +57,22 @@ def test_choice(orbits, alpha, beta, n, scanned, cuda_device, monkeypatch):
         size = bound.apply_within(rows, x.abs().to(torch.complex128), rows).abs()
     assert torch.equal(mat.row_ptr, other.row_ptr)
     assert torch.all((mat.apply(x) - other.apply(x)).abs() <= TOL * size)
+
+
+@pytest.mark.parametrize("first,then", [(None, "scan"), ("scan", None), ("scan", "grouped"), ("grouped", "scan")])
+@pytest.mark.parametrize("first_guess", [1 << 20, 16])
+def test_environment_changed_before_the_backward(first, then, first_guess, cuda_device, monkeypatch):
+    table = terms.integral_hamiltonian_tables(9, seed=106, complex_valued=True)
+    ham = Hamiltonian(table, kind="fermi")
+    ham._LOG_FIRST_GUESS = first_guess
+    rows = torch.from_numpy(terms.random_determinants(9, 4, 4, 900, seed=107)).to(cuda_device)
+    psi, g = _psi(900, 108, cuda_device).requires_grad_(True), _psi(900, 109, cuda_device)
+    set_to = lambda walk: monkeypatch.setenv("QMBX_WALK", walk) if walk else monkeypatch.delenv("QMBX_WALK", raising=False)
+    set_to(first)
+    y = ham.apply_within(rows, psi, rows)
+    set_to(then)
+    (back,) = torch.autograd.grad(y, psi, grad_outputs=g)
+    set_to("grouped")
+    want = ham.apply_within_adjoint(rows, g, rows)
+    size = _magnitudes(table).apply_within_adjoint(rows, g.abs().to(torch.complex128), rows).abs()
+    assert torch.all((back - want).abs() <= TOL * size)
