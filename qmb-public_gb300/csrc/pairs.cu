@@ -138,6 +138,7 @@ template <int W>
 __global__ void __launch_bounds__(kThreads) pair_gate_kernel(UniqueRows<W> a, const int* __restrict__ a_count,
                                                              UniqueRows<W> b, const int* __restrict__ b_count,
                                                              const int2* __restrict__ groups, int same, int forced,
+                                                             double fixed_ps,
                                                              const int* __restrict__ walked,
                                                              unsigned long long* sums, int* __restrict__ gate) {
     __shared__ uint8_t s_pos[kWarpsPerBlock][64 * W];
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(kThreads) pair_gate_kernel(UniqueRows<W> a, co
     const double reach = (double)*(volatile unsigned long long*)(sums + 1) / kWarps;
     const double particles = (double)*(volatile unsigned long long*)(sums + 2) / kWarps;
     const double pairs = (double)na * (double)nb * (same ? 0.5 : 1.0);
-    const double scan_ps = pairs * (0.0075 * particles + close * (same ? 80.0 : 40.0));
+    const double scan_ps = fixed_ps + pairs * (0.0075 * particles + close * (same ? 80.0 : 40.0));
     const double walk_ps = 5.0 * (double)*walked * reach;
     // forced: still not for rows of three particles and fewer
     const bool scan = na > 0 && nb > 0 && (forced ? particles > 3.0 : scan_ps < walk_ps);
@@ -220,7 +221,8 @@ int choose_pairs(const PairWork& p, const HashRows& rows_i, const HashRows& rows
     const HashRows& a = pairs_swapped(p) ? rows_j : rows_i;
     const HashRows& b = pairs_swapped(p) ? rows_i : rows_j;
     QMBX_CUDA_TRY(cudaMemsetAsync(p.next, 0, p.clear_bytes, s));
-    QMBX_KERNEL(kGroupOther, s, pair_gate_kernel<W><<<kGateBlocks, kThreads, 0, s>>>(UniqueRows<W>{a.keys, a.unique}, a.count, UniqueRows<W>{b.keys, b.unique}, b.count, terms.groups, p.same ? 1 : 0, pairs_forced() ? 1 : 0, walked.count, p.next + 2, p.gate));
+    const double fixed_ps = choose_walk(terms, walked.n, true) == Walk::kPivot ? 0.0 : 35e6;
+    QMBX_KERNEL(kGroupOther, s, pair_gate_kernel<W><<<kGateBlocks, kThreads, 0, s>>>(UniqueRows<W>{a.keys, a.unique}, a.count, UniqueRows<W>{b.keys, b.unique}, b.count, terms.groups, p.same ? 1 : 0, pairs_forced() ? 1 : 0, fixed_ps, walked.count, p.next + 2, p.gate));
     QMBX_LAUNCH_CHECK("pair_gate_kernel");
     return QMBX_OK;
 }
@@ -264,19 +266,23 @@ bool pairs_possible(const qmbx_table_header* h) { return h->n_class_buckets > 0;
 
 namespace {
 
-// The sizes at which the scan beats the term walks, measured on FP64 calls
-// (whole calls, scan against the faster walk).  A walk's work is its rows
-// times the terms they reach, the scan's its pairs of rows: 200,000 x 20,000
-// rows of 55,371 terms on 28 sites 0.62 against 0.94 ms, 65,536 rows of
-// 669,579 terms on 52 sites 0.44 against 13.4 ms.  Small calls are launches
-// (400 rows of 55,371 terms 138 against 109 us, 2,000 rows 113 against 165
-// us).  Operators that hold few of the possible transitions connect few of
-// the pairs that the scan looks up.
+// The sizes at which the scan can beat the term walks; choose_pairs then looks
+// at the rows.  (us, FP64 calls within one set, scan against the faster walk)
+//   terms x walked rows: small calls are launches, and a call that may scan
+//     and walks has 25 us of them for nothing.  3,792 rows under 55,371 terms
+//     (2.1e8) 111 against 208 with 5 + 5 electrons, 128 against 143 with 3 + 3
+//     and 151 (walked) against 122 with 2 + 2; 1,805 rows (1e8) 110 against
+//     148, 113 against 104 and, clustered, 196 against 117.
+//   other side x sites: in choose_pairs' costs a pair of rows may cost 0.0075
+//     N / (5 N^2 / S^2) of a reached term at N of S sites, so the walk is the
+//     cheaper for any rows filled up to 3/8 past 250 terms a row and site.
+//   terms per possible transition: below one in a hundred next to none of the
+//     pairs within two moves are connected (lattices).
 bool scan_pays(const qmbx_table_header* h, int64_t n_i, int64_t n_j) {
     const double walked = (double)(n_i < n_j ? n_i : n_j), other = (double)(n_i < n_j ? n_j : n_i);
     const double terms = (double)h->part[QMBX_PART_FWD].n, sites = (double)h->n_sites;
     const double moves = sites * (sites - 1) / 2;
-    return other * sites < 250.0 * terms && walked * terms > 1e8 && terms > 0.01 * moves * moves;
+    return other * sites < 250.0 * terms && walked * terms > 2e8 && terms > 0.01 * moves * moves;
 }
 
 // Calls on more rows have no scratch for a scan that QMBX_WALK forces on them.

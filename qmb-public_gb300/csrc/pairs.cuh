@@ -132,7 +132,8 @@ inline bool pairs_swapped(const PairWork& p) { return !p.same && p.i.n > p.j.n; 
 // pairs are close, and the walk on how many terms a row reaches, so a sample of both is taken on the device.
 // Costs, fitted to whole FP64 calls (times in ps, summed over the GPU): a pair of rows 0.0075 a particle; a close
 // pair 80 within one set (100 for its two lookups and hits, less 20 for the two hits a walk would find), 40 between
-// two; a reached term 5 in the walk.  (scan and walk, us)
+// two; a reached term 5 in the walk; against the grouped walk 35 us for the scan's two kernels, whose blocks are few
+// and uneven on small sets (clustered sets of that size are no better in the pivot-major walk).  (scan and walk, us)
 //   every determinant of 3 + 3 in 14 orbitals, 132,496 rows    11,934   4,093 (all of a row's 1,485 neighbours present)
 //   a random third of them, 40,000 rows                          1,184   1,016
 //   200,000 of the 4.0M of 5 + 5                                 2,783   7,914
