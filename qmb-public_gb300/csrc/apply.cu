@@ -92,7 +92,7 @@ __device__ __forceinline__ void comp_diag_add(CompSum& dre, CompSum& dim, float4
     const float sg = parity ? -1.f : 1.f;
     const float ih = CONJ ? -cf.z : cf.z, il = CONJ ? -cf.w : cf.w;
     dre.add2(sg * cf.x, sg * cf.y);
-    if (ih != 0.f || il != 0.f) dim.add2(sg * ih, sg * il);
+    dim.add2(sg * ih, sg * il);
 }
 
 // coef (hi/lo split, sign already folded) times psi, added to (re, im) with
@@ -327,7 +327,7 @@ struct DiagonalF64 : VisitorBase {
     __device__ __forceinline__ void visit_diag(Acc& a, const Key<W>&, int parity, int64_t slot) const {
         double2 cf = __ldg(dcoef + slot);
         a.re += parity ? -cf.x : cf.x;
-        if (cf.y != 0.0) a.im += parity ? -cf.y : cf.y;  // real operators: no second FP64 add
+        a.im += parity ? -cf.y : cf.y;
     }
     __device__ __forceinline__ void reduce(Acc& a) const {
         a.re = warp_sum(a.re);
@@ -570,7 +570,7 @@ struct DiagAdd : VisitorBase {
             const double2 cf = __ldg(dcoef + slot);
             const double ci = CONJ ? -cf.y : cf.y;
             a.dre += parity ? -cf.x : cf.x;
-            if (ci != 0.0) a.dim += parity ? -ci : ci;  // real operators: no second FP64 add
+            a.dim += parity ? -ci : ci;
         }
     }
     __device__ __forceinline__ void reduce(Acc& a) const {

@@ -202,6 +202,9 @@ __device__ __forceinline__ int64_t hash_find(const HashView& h, const Key<W>& ke
     return -1;
 }
 
+// Whether x is neither zero nor minus zero, on the integer pipe: a comparison in FP64 costs what an addition does.
+__device__ __forceinline__ bool nonzero(double x) { return __double_as_longlong(x) << 1 != 0; }
+
 // Sum of a double over aligned groups of L lanes (butterfly: every lane gets
 // its group's total), and across the warp.
 template <int L>

@@ -140,7 +140,7 @@ struct MatrixDiagonal : VisitorBase {
     __device__ __forceinline__ void visit_diag(Acc& a, const Key<W>&, int parity, int64_t slot) const {
         const double2 cf = __ldg(dcoef + slot);
         a.re += parity ? -cf.x : cf.x;
-        if (cf.y != 0.0) a.im += parity ? -cf.y : cf.y;
+        a.im += parity ? -cf.y : cf.y;
     }
     __device__ __forceinline__ void reduce(Acc& a) const {
         a.re = warp_sum(a.re);
@@ -221,7 +221,7 @@ __device__ __forceinline__ double2 row_times(const int64_t* __restrict__ row_ptr
             if (c[u] >= 0) {
                 re = fma(v[u].x, p[u].x, re);
                 im = fma(v[u].x, p[u].y, im);
-                whole = whole || v[u].y != 0.0 || !finite_bits(p[u].x) || !finite_bits(p[u].y);
+                whole = whole || nonzero(v[u].y) || !finite_bits(p[u].x) || !finite_bits(p[u].y);
             }
         }
         if (__any_sync(0xffffffffu, whole)) {
