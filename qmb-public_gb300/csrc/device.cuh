@@ -1166,7 +1166,7 @@ __global__ void __launch_bounds__(kThreads) grouped_split_kernel(V v, Src src, i
     v.block_flush(sh);
 }
 
-// Diagonal passes over parts of many small groups (an ab-initio table's
+// Diagonal passes over bare parts (format.h) of many small groups (an ab-initio table's
 // n_p n_q terms, about one a pair group): a row visits the non-empty groups of
 // its occupied positions and pairs instead of testing every term.  Eight lanes
 // share a row; lane s takes positions s, 15 - s, 16 + s, ... of its occupied
@@ -1210,18 +1210,7 @@ __global__ void __launch_bounds__(kThreads) diag_groups_kernel(V v, Src src, con
     v.init(acc, row, c, nullptr);
     auto visit = [&](int64_t g) {
         const int2 se = __ldg(diag.groups + g);
-        for (int t = se.x; t < se.y; ++t) {
-            if (diag.bare) {
-                v.visit_diag(acc, c, 0, t);
-                continue;
-            }
-            TermRec<W> rec;
-            load_test<W>(rec, diag, t);
-            load_apply<W>(rec, diag, t);
-            if (!rec.applies(c)) continue;
-            Key<W> img;
-            v.visit_diag(acc, c, rec.image(c, img), t);
-        }
+        for (int t = se.x; t < se.y; ++t) v.visit_diag(acc, c, 0, t);
     };
     if (live && sub == L - 1) visit(0);
     for (int r = 0; 8 * r < occ; ++r) {
@@ -1419,11 +1408,14 @@ bool walk_forced();  // QMBX_WALK names tiled, grouped or pivot
 int grouped_grid(int64_t n_rows);
 
 // A pass over the diagonal terms of n_max rows (or *n_rows of them): by the
-// rows' own groups where the part has many terms in small groups, else tiled,
-// a row shared by 8 lanes where the rows are few; parts of large groups and
-// QMBX_WALK take the walk of choose_walk.  Terms up to which testing them all
-// from shared memory is the faster: at 211 terms 20,000 rows of 8 particles
-// take 15 us by groups and 30 us tiled, a tile holds 128 terms.
+// rows' own groups where the part is bare with many terms in small groups,
+// else tiled, a row shared by 8 lanes where the rows are few; parts of large
+// groups, parts that are not bare and QMBX_WALK take the walk of choose_walk.
+// (Terms that ask for empty sites crowd into the groups of few pivots: n n
+// and (1-n)(1-n) on every pair of 64 sites, 200,000 rows, 23 ms by groups, 4.4
+// tiled.)  Terms up to which testing them all from shared memory is the
+// faster: at 211 terms 20,000 rows of 8 particles take 15 us by groups and 30
+// us tiled, a tile holds 128 terms.
 constexpr int64_t kDiagTiled = 128;
 
 template <int W, class V, class Src>
@@ -1432,9 +1424,10 @@ int launch_diagonal(const V& v, const Src& src, const int* n_rows, int64_t n_max
     PartView none = diag;
     none.n = 0;
     const Walk kind = choose_walk(diag, n_max, false);
-    if (walk_forced() ? kind == Walk::kGrouped : diag.wide && kind == Walk::kGrouped) {
+    const bool by_groups = !walk_forced() && diag.bare && !diag.wide;
+    if (!by_groups && kind == Walk::kGrouped) {
         QMBX_KERNEL(group, s, grouped_kernel<W><<<grouped_grid(n_max), kThreads, 0, s>>>(v, src, n_rows, n_max, none, diag));
-    } else if (!walk_forced() && !diag.wide && diag.n > kDiagTiled) {
+    } else if (by_groups && diag.n > kDiagTiled) {
         QMBX_KERNEL(group, s, diag_groups_kernel<W><<<grid_for(n_max * 8, kThreads), kThreads, 0, s>>>(v, src, n_rows, n_max, diag));
     } else if (diag_lanes(n_max) == 8) {
         QMBX_KERNEL(group, s, diag_split_kernel<W, 8><<<grid_for(n_max * 8, kThreads), kThreads, 0, s>>>(v, src, n_rows, n_max, diag));
