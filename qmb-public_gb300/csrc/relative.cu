@@ -1106,12 +1106,12 @@ struct SingleVisitor : VisitorBase {
 // every row, so a row's neighbour is given by the first term, in descending
 // key order, that applies and leads outside the input.  Terms apply to a few
 // per cent of the rows, so a row finds it among the first hundred or so: the
-// best couple of thousand terms are gathered and sorted once, and a warp takes a
+// best thousand terms are gathered and sorted once, and a warp takes a
 // row through them 32 at a time.  Rows that find none there are walked.
 //   20,000 rows under 55,371 terms: walk 648 us; bins, gather, sort and rows 26 us
 // ---------------------------------------------------------------------------
 
-constexpr int kBestTerms = 2048;
+constexpr int kBestTerms = 1024;
 constexpr int kKeyBins = 1 << 14;  // exponent and three mantissa bits of |key|: bins of a ratio of at most 1.125
 
 struct BestTerm {
@@ -1182,10 +1182,12 @@ __global__ void __launch_bounds__(kTailThreads) single_gather_kernel(const doubl
 
 // Sort the gathered terms by (key, input order), which no two share: a warp
 // counts the terms ahead of one.  (A bitonic sort of 4,096 terms in one block
-// took 112 us; the counts of 2,048 take a few.)
+// took 112 us; the counts of 1,024 take a few.)
+// The terms' tests go with them: word q of the k-th term at tests[q kBestTerms + k].
 __global__ void __launch_bounds__(kThreads) single_sort_kernel(const BestTerm* __restrict__ best,
-                                                               const SingleCtl* __restrict__ ctl,
-                                                               BestTerm* __restrict__ sorted) {
+                                                               const SingleCtl* __restrict__ ctl, PartView off, int words,
+                                                               BestTerm* __restrict__ sorted,
+                                                               ulonglong2* __restrict__ tests) {
     __shared__ unsigned long long s_key[kBestTerms];
     __shared__ int32_t s_orig[kBestTerms];
     const int n = ctl->gathered;
@@ -1204,39 +1206,69 @@ __global__ void __launch_bounds__(kThreads) single_sort_kernel(const BestTerm* _
     for (int i = lane; i < n; i += 32) ahead += s_key[i] < key || (s_key[i] == key && s_orig[i] < orig) ? 1u : 0u;
     ahead = __reduce_add_sync(0xffffffffu, ahead);
     if (lane == 0) sorted[ahead] = best[me];
+    if (lane < words) tests[lane * kBestTerms + ahead] = __ldg(off.test + (int64_t)lane * off.stride + best[me].slot);
 }
+
+// A warp takes a row through the terms in order, 32 at first and up to
+// kSingleStep at a time: those that apply queue up, and the images of 32 of
+// them are looked up at once.  The terms' tests lie in order, so that a warp
+// reads 32 in four lines.  On sets whose rows have no relative the terms are
+// tried in vain: on every determinant of 3 + 3 electrons in 14 orbitals (the
+// walk alone 2.43 ms) 2,048 terms gathered from the table's own places took
+// the call to 3.24 ms, in order to 2.91, and 1,024 in order to 2.74.
+constexpr int kSingleStep = 256;
 
 template <int W>
 __global__ void __launch_bounds__(kThreads) single_first_kernel(const uint64_t* __restrict__ keys, int64_t n, HashView set,
                                                                 PartView off, const BestTerm* __restrict__ best,
+                                                                const ulonglong2* __restrict__ tests,
                                                                 SingleCtl* __restrict__ ctl,
                                                                 int32_t* __restrict__ unresolved, int nq,
                                                                 uint8_t* __restrict__ out) {
+    __shared__ int32_t s_term[kWarpsPerBlock][kSingleStep];
     const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    int32_t* queue = s_term[threadIdx.x >> 5];
     const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (row >= n) return;
     const int terms = ctl->gathered;
     const Key<W> c = load_key<W>(keys, row);
-    for (int base = 0; base < terms; base += 32) {
-        bool on = false;
-        Key<W> img{};
-        if (base + lane < terms) {
-            const int32_t slot = __ldg(&best[base + lane].slot);
-            TermRec<W> rec;
-            load_test<W>(rec, off, slot);
-            if (rec.applies(c)) {
-                load_apply<W>(rec, off, slot);
-                rec.image(c, img);
-                on = hash_find<W>(set, img) < 0;
+    for (int base = 0, step = 32; base < terms; base += step, step = base < kSingleStep ? base : kSingleStep) {
+        int waiting = 0;
+        __syncwarp();  // the queue has been read
+        for (int at = base; at < base + step && at < terms; at += 32) {
+            bool on = at + lane < terms;
+            if (on) {
+                uint64_t bad = 0;
+#pragma unroll
+                for (int q = 0; q < W; ++q) {
+                    const ulonglong2 test = __ldg(tests + q * kBestTerms + at + lane);
+                    bad |= (c.w[q] ^ test.y) & test.x;
+                }
+                on = bad == 0;
             }
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            if (on) queue[waiting + __popc(m & lt)] = at + lane;
+            waiting += __popc(m);
         }
-        const unsigned m = __ballot_sync(0xffffffffu, on);
-        if (m != 0) {
-            if (lane == __ffs(m) - 1) {
-                uint8_t* r = out + row * nq;
-                for (int b = 0; b < nq; ++b) r[b] = (uint8_t)(img.w[b >> 3] >> (8 * (7 - (b & 7))));
+        __syncwarp();
+        for (int k = 0; k < waiting; k += 32) {
+            bool out_of_set = false;
+            Key<W> img{};
+            if (k + lane < waiting) {
+                TermRec<W> rec;
+                load_apply<W>(rec, off, __ldg(&best[queue[k + lane]].slot));
+                rec.image(c, img);
+                out_of_set = hash_find<W>(set, img) < 0;
             }
-            return;
+            const unsigned m = __ballot_sync(0xffffffffu, out_of_set);
+            if (m != 0) {
+                if (lane == __ffs(m) - 1) {
+                    uint8_t* r = out + row * nq;
+                    for (int b = 0; b < nq; ++b) r[b] = (uint8_t)(img.w[b >> 3] >> (8 * (7 - (b & 7))));
+                }
+                return;
+            }
         }
     }
     if (lane == 0) unresolved[atomicAdd(&ctl->unresolved, 1)] = (int32_t)row;
@@ -1262,15 +1294,17 @@ struct SingleOrder {
     int* bins;
     BestTerm* best;
     BestTerm* sorted;
+    ulonglong2* tests;
     int32_t* unresolved;
 };
 
-SingleOrder take_single_order(Arena& ws, int64_t n) {
+SingleOrder take_single_order(Arena& ws, int64_t n, int words) {
     SingleOrder o;
     o.ctl = ws.take<SingleCtl>(1);
     o.bins = ws.take<int>(kKeyBins);
     o.best = ws.take<BestTerm>(kBestTerms);
     o.sorted = ws.take<BestTerm>(kBestTerms);
+    o.tests = ws.take<ulonglong2>((uint64_t)words * kBestTerms);
     o.unresolved = ws.take<int32_t>((uint64_t)(n > 0 ? n : 1));
     return o;
 }
@@ -1312,14 +1346,14 @@ int single_impl(const void* table_host, const void* table_dev, const uint8_t* co
     none.n = 0;
     SingleVisitor<W> v{{}, L.set.hash(), L.kf, off.orig, out, h->n_qubytes, nullptr};
     Arena behind = ws;
-    const SingleOrder o = take_single_order(behind, n);
+    const SingleOrder o = take_single_order(behind, n, W);
     if (single_ordered(off, n) && behind.fits()) {
         QMBX_CUDA_TRY(cudaMemsetAsync(o.ctl, 0, (size_t)(reinterpret_cast<char*>(o.bins + kKeyBins) - reinterpret_cast<char*>(o.ctl)), s));
         const unsigned blocks = grid_for(off.n, kTailThreads) < 152u ? grid_for(off.n, kTailThreads) : 152u;
         QMBX_KERNEL(kGroupSelect, s, single_bins_kernel<<<grid_for(off.n, kThreads), kThreads, 0, s>>>(L.kf, off.n, o.bins));
         QMBX_KERNEL(kGroupSelect, s, single_gather_kernel<<<blocks, kTailThreads, 0, s>>>(L.kf, off.orig, off.n, o.bins, o.best, o.ctl));
-        QMBX_KERNEL(kGroupSort, s, single_sort_kernel<<<kBestTerms / kWarpsPerBlock, kThreads, 0, s>>>(o.best, o.ctl, o.sorted));
-        QMBX_KERNEL(kGroupEnumerate, s, single_first_kernel<W><<<grid_for(n, kWarpsPerBlock), kThreads, 0, s>>>(L.set.keys, n, L.set.hash(), off, o.sorted, o.ctl, o.unresolved, h->n_qubytes, out));
+        QMBX_KERNEL(kGroupSort, s, single_sort_kernel<<<kBestTerms / kWarpsPerBlock, kThreads, 0, s>>>(o.best, o.ctl, off, W, o.sorted, o.tests));
+        QMBX_KERNEL(kGroupEnumerate, s, single_first_kernel<W><<<grid_for(n, kWarpsPerBlock), kThreads, 0, s>>>(L.set.keys, n, L.set.hash(), off, o.sorted, o.tests, o.ctl, o.unresolved, h->n_qubytes, out));
         // rows that none of these terms serves: the walk over all terms
         v.rows = o.unresolved;
         ListedRows<W> rest{L.set.keys, o.unresolved};
@@ -1427,7 +1461,7 @@ extern "C" int qmbx_single_relative_workspace(const void* table_host, int64_t n,
         case 4: take_single<4>(probe, n, n_off); break;
         default: return fail(QMBX_ERR_ARGUMENT, "unsupported word count");
     }
-    take_single_order(probe, n);
+    take_single_order(probe, n, h->n_words);
     *bytes = probe.used;
     return QMBX_OK;
 }
