@@ -235,6 +235,7 @@ struct PartView {
     int64_t n_nonempty;
     int64_t n;
     int wide;                  // groups are large: walk each with lanes over its terms
+    int falling;               // the norms fall within its groups, but for a few (format.h)
     int bare;                  // diagonal part: its groups' terms apply as they are (format.h)
     const uint4* narrow;       // (mask, val, flip, par) >> 32 of every term (tables of <= 32 sites), or NULL
 };
@@ -259,6 +260,7 @@ inline PartView part_view(const void* table_host, const void* table_dev, int whi
     v.n_nonempty = p.n_nonempty;
     v.n = p.n;
     v.wide = p.wide_groups;
+    v.falling = p.falling;
     v.bare = which == QMBX_PART_DIAG ? h->diag_bare : 0;
     v.narrow = p.off_narrow != 0 ? reinterpret_cast<const uint4*>(base + p.off_narrow) : nullptr;
     return v;

@@ -63,7 +63,7 @@
 #include <stdint.h>
 
 #define QMBX_MAGIC 0x58424D51u  // "QMBX"
-#define QMBX_TABLE_VERSION 8u
+#define QMBX_TABLE_VERSION 9u
 #define QMBX_MAX_WORDS 4
 #define QMBX_ALIGN 256
 
@@ -87,7 +87,8 @@ struct qmbx_table_part {
     int64_t n_groups;        // 1 + 64W + 64W(64W-1)/2
     int64_t n_nonempty;      // groups holding at least one term
     int32_t wide_groups;     // 1 when non-empty groups hold 8 or more terms on average
-    int32_t reserved;
+    int32_t falling;         // 1 when at least 7 of 8 terms have no larger norm behind them in their group (parts with
+                             // bounds; tables sorted by |coef|)
 };
 
 struct qmbx_table_header {

@@ -32,6 +32,8 @@
 namespace qmbx {
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int kBuckets = 4096;
 
 // Figures of the calling thread's last find_relative call (qmbx_find_relative_stats).
@@ -73,6 +75,13 @@ struct FindCtl {
     unsigned long long n_unique;   // distinct rows returned
     int overflow;
     int emit_from;                 // lowest bucket the emission pass keeps
+    int count_from;                // the first count's bucket (> 0) if a whole count from it follows, else 0
+    unsigned int n_long[2];        // groups queued for their rest (LongGroup): by the threshold's count, by the emission
+};
+
+// The rest of a pivot group that a row reaches far into: terms t .. end of row `row`.
+struct LongGroup {
+    int row, t, end;
 };
 
 // The histogram (EMIT = false) and emission (EMIT = true) passes as
@@ -88,6 +97,9 @@ struct RelativeArgs {
     unsigned long long* hist;
     int hist_exact;          // 1: count only records outside the exclusion set (the exact rerun);
                              // 0: count every record (a threshold estimate: no exclusion lookups)
+    unsigned long long* deep;  // bounded passes: by bucket, terms that the truncated count left out (an estimate)
+    LongGroup* queue;
+    unsigned int queue_cap;
     // pass 2 (emit_from, the record counter and the overflow flag live in ctl)
     FindCtl* ctl;
     int64_t cap_emit;
@@ -179,64 +191,201 @@ struct RelativeVisitor : VisitorBase {
     __device__ __forceinline__ void finish(Acc&, int64_t, const Key<W>&) const {}
 };
 
-// The same passes over parts whose groups hold many terms (PartView::wide),
-// bounded by the terms' norms.  A warp takes a row (or one of `split` shares
-// of it); the lanes take its pivot groups, and a group's terms are read, eight
-// lanes a group, only while the bound of the rest of the group (the norms
+// Inclusive scan of v over the T threads of a block in thread order (s_warp: 32 values).
+template <int Threads = 1024, class T>
+__device__ __forceinline__ T block_inclusive_scan(T v, T* s_warp) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T x = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const T y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        T w = lane < Threads / 32 ? s_warp[lane] : T(0);
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const T y = __shfl_up_sync(0xffffffffu, w, d);
+            if (lane >= d) w += y;
+        }
+        s_warp[lane] = w;
+    }
+    __syncthreads();
+    return warp > 0 ? x + s_warp[warp - 1] : x;
+}
+
+// The highest bucket b > 0 whose buckets >= b hold at least `target` records
+// by the counts of a histogram pass (scaled by `scale`), 0 when there is none.
+// Every thread of the block's `Threads` gets it: thread t sums the buckets
+// [4096 - P (t + 1), 4096 - P t), a scan over the threads (highest buckets
+// first) finds the one thread where the running count reaches the target, and
+// that thread walks its buckets.
+template <int Threads>
+__device__ __forceinline__ int choose_bucket(const unsigned long long* hist, double scale, double target,
+                                             unsigned long long* s_warp, int* s_found) {
+    constexpr int kPer = kBuckets / Threads;
+    const int t = threadIdx.x;
+    const int hi = kBuckets - kPer * t;  // thread t covers buckets [hi - kPer, hi)
+    if (t == 0) *s_found = 0;
+    // integer counts, scaled only where compared: the running count is exact and monotone, so
+    // exactly one thread sees it cross the target
+    unsigned long long mine = 0;
+    for (int b = hi - 1; b >= hi - kPer && b >= 1; --b) mine += __ldcg(hist + b);
+    const unsigned long long run = block_inclusive_scan<Threads>(mine, s_warp);
+    if (scale * (double)run >= target && scale * (double)(run - mine) < target) {
+        // the one thread whose buckets reach the target
+        unsigned long long above = run - mine;
+        for (int b = hi - 1; b >= hi - kPer && b >= 1; --b) {
+            above += __ldcg(hist + b);
+            if (scale * (double)above >= target) {
+                *s_found = b;
+                break;
+            }
+        }
+    }
+    __syncthreads();
+    const int found = *s_found;
+    __syncthreads();  // s_found and s_warp are written again
+    return found;
+}
+
+// emit_from from the counts of a histogram pass: one bucket below the one
+// that choose_bucket finds (0 when all buckets above 0 hold fewer).  deep (or
+// NULL): by bucket, what the pass left out; where that could be more than half
+// of the target from the bucket on, count_from asks for a whole count.  The
+// counts are left cleared.
+constexpr int kChooseThreads = 1024;
+
+__global__ void __launch_bounds__(kChooseThreads) choose_emit_kernel(unsigned long long* __restrict__ hist,
+                                                                     const unsigned long long* __restrict__ deep,
+                                                                     double scale, double target,
+                                                                     FindCtl* __restrict__ ctl) {
+    __shared__ unsigned long long s_warp[32];
+    __shared__ int s_found;
+    const int b = choose_bucket<kChooseThreads>(hist, scale, target, s_warp, &s_found);
+    unsigned long long left_out = 0;
+    for (int k = threadIdx.x; k < kBuckets; k += kChooseThreads) {
+        if (deep != nullptr && k >= (b > 1 ? b : 1)) left_out += deep[k];
+        hist[k] = 0;
+    }
+    left_out = block_inclusive_scan<kChooseThreads>(left_out, s_warp);
+    if (threadIdx.x == kChooseThreads - 1) {
+        ctl->emit_from = b > 1 ? b - 1 : 0;
+        ctl->count_from = scale * (double)left_out > 0.5 * target ? (b > 1 ? b : 1) : 0;
+    }
+}
+
+// The same passes over parts whose groups hold many terms (PartView::wide) in
+// falling order of their norms, bounded by the norms.  A warp takes a row (or
+// one of `split` shares of it); the lanes take its pivot groups, and a group's
+// terms are read only while the bound of the rest of the group (the norms
 // themselves for tables sorted by |coef|) can still reach the threshold.
 // Selections take few records of a row (121k of 5.7e7 for the top 50,000 of
 // 20,000 rows under 55,371 terms), so most groups end at their first bound:
 // the pass is a few instructions per group instead of a test per term, and is
-// bound by the latency of its reads.  On GB300,
-// emission passes against the walks: those rows 428 -> 70 us, the top
-// 1,000,000 of 8,192 rows under 3.1M terms 4.58 -> 0.50 ms (pivot-major walk
-// and diagonal pass), the top 200,000 of 4,099 rows under 669,579 terms 1.42
-// -> 0.21 ms; their histograms 124 -> 23, 473 -> 42 and 139 -> 19 us.
+// bound by the latency of its reads.  On GB300, emission passes against the
+// walks: those rows 428 -> 70 us, the top 1,000,000 of 8,192 rows under 3.1M
+// terms 4.58 -> 0.50 ms (pivot-major walk and diagonal pass), the top 200,000
+// of 4,099 rows under 669,579 terms 1.42 -> 0.21 ms.
 //
-// The histogram reads the first `depth` steps of 32 terms of every group and
-// counts what applies: the records near the threshold are the first of their
-// groups.  Counts that miss deeper records only lower the threshold.
+// Three passes share the code:
+//   kFirst  counts the first `depth` steps of 32 terms of every group, all
+//           buckets: the records near the threshold are the first of their
+//           groups.  What it leaves out only lowers the threshold; an estimate
+//           of it goes to a.deep.
+//   kAbove  counts every record of the buckets from `from` on.
+//   kEmit   emits them.
+// The last two leave a group after kInline steps of eight lanes and queue its
+// rest, which a warp each takes up afterwards (bounded_rest): a row with most
+// of the weight, as configurations of a wave function have them, reaches
+// thousands of terms of every group, one after the other a chain of
+// milliseconds for the one warp that has the row.
 //
 // Diagonal terms give the row itself: one exclusion lookup per row, and a
 // group a lane (their groups hold a term or two).
-template <int W, bool EMIT>
-__global__ void __launch_bounds__(kThreads) relative_bounded_kernel(RelativeArgs a, const uint64_t* __restrict__ keys,
-                                                                    int64_t n, int split, int depth) {
-    __shared__ int s_hist[EMIT ? 1 : kBuckets];
-    __shared__ uint8_t s_pos[kWarpsPerBlock][64 * W];
-    if (!EMIT) {
-        for (int k = threadIdx.x; k < kBuckets; k += kThreads) s_hist[k] = 0;
-        __syncthreads();
+enum BoundedPass { kFirst, kAbove, kEmit };
+constexpr int kInline = 2;
+
+// A record of bucket b per lane where `on`: counted, or emitted.
+template <int W, int Pass>
+__device__ __forceinline__ void bounded_take(const RelativeArgs& a, int* hist, bool on, int b, const Key<W>& img, int part,
+                                             int parity, int64_t slot, int64_t row, int lane) {
+    if (Pass != kEmit) {
+        if (on) atomicAdd(hist + b, 1);
+        return;
     }
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (m == 0) return;
+    unsigned long long at = 0;
+    if (lane == __ffs(m) - 1) at = atomicAdd(&a.ctl->n_emit, (unsigned long long)__popc(m));
+    at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
+    if (!on) return;
+    if ((int64_t)at >= a.cap_emit) {
+        a.ctl->overflow = 1;
+        return;
+    }
+    a.emit_rank[2 * at + 0] = (uint64_t)slot | ((uint64_t)part << 62) | ((uint64_t)parity << 63);
+    a.emit_rank[2 * at + 1] = (uint64_t)row;
+#pragma unroll
+    for (int q = 0; q < W; ++q) a.emit_keys[at * W + q] = img.w[q];
+}
+
+// A term whose bound is not below the threshold (NaN: not known to be).
+__device__ __forceinline__ bool bounded_reaches(float bound, float m, int from) {
+    const float e = __fmul_rn(bound, m);
+    return e != e || weight_bucket(e) >= from;
+}
+
+// Term t of the changing part for the row (c, m): whether it can still reach the threshold is returned, its record
+// taken.  Everything a term needs is read at once: one trip to L2 before its lookup.
+template <int W, int Pass>
+__device__ __forceinline__ bool bounded_term(const RelativeArgs& a, int* hist, bool in, int t, const Key<W>& c, float m,
+                                             int from, int64_t row, int lane) {
+    const PartView& pv = a.off;
+    bool on = false;
+    int par = 0, b = 0;
+    Key<W> img{};
+    if (in) {
+        TermRec<W> rec;
+        bool narrow = false;
+        if constexpr (W == 1) narrow = pv.narrow != nullptr;
+        if (narrow) {
+            load_narrow<W>(rec, pv, t);
+        } else {
+            load_test<W>(rec, pv, t);
+            if (Pass == kEmit) load_apply<W>(rec, pv, t);
+        }
+        b = weight_bucket(__fmul_rn(__ldg(pv.norm + t), m));
+        if (Pass != kFirst) in = bounded_reaches(__ldg(pv.bound + t), m, from);
+        on = in && b >= from && rec.applies(c);
+        if (Pass == kEmit && on) {
+            par = rec.image(c, img);
+            on = hash_find<W>(a.excl, img) < 0;
+        }
+    }
+    bounded_take<W, Pass>(a, hist, on, b, img, 0, par, t, row, lane);
+    return in;
+}
+
+__device__ __forceinline__ float bounded_weight(const double2* psi, int64_t row) {
+    const double2 p = __ldg(psi + row);
+    const float px = (float)p.x, py = (float)p.y;
+    return __fadd_rn(__fmul_rn(px, px), __fmul_rn(py, py));
+}
+
+template <int W, int Pass>
+__device__ void bounded_rows(const RelativeArgs& a, const uint64_t* __restrict__ keys, int64_t n, int split, int depth,
+                             int from, int* hist, int* deep, uint8_t* pos, unsigned int* n_long) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    uint8_t* pos = s_pos[warp];
-    const int from = EMIT ? a.ctl->emit_from : 0;
-    // records whose estimate reaches the threshold, one a lane
-    auto take = [&](bool on, const Key<W>& img, int part, int parity, int64_t slot, int64_t row) {
-        const unsigned m = __ballot_sync(0xffffffffu, on);
-        if (m == 0) return;
-        unsigned long long at = 0;
-        if (lane == __ffs(m) - 1) at = atomicAdd(&a.ctl->n_emit, (unsigned long long)__popc(m));
-        at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1) + __popc(m & lt);
-        if (!on) return;
-        if ((int64_t)at >= a.cap_emit) {
-            a.ctl->overflow = 1;
-            return;
-        }
-        a.emit_rank[2 * at + 0] = (uint64_t)slot | ((uint64_t)part << 62) | ((uint64_t)parity << 63);
-        a.emit_rank[2 * at + 1] = (uint64_t)row;
-#pragma unroll
-        for (int q = 0; q < W; ++q) a.emit_keys[at * W + q] = img.w[q];
-    };
     const int64_t items = n * split, stride = (int64_t)gridDim.x * kWarpsPerBlock;
     for (int64_t u = (int64_t)blockIdx.x * kWarpsPerBlock + warp; u < items; u += stride) {
         const int64_t row = u / split;
         const int share = (int)(u - row * split);
         const Key<W> c = load_key<W>(keys, row);
-        const double2 p = __ldg(a.psi + row);
-        const float px = (float)p.x, py = (float)p.y;
-        const float m = __fadd_rn(__fmul_rn(px, px), __fmul_rn(py, py));
+        const float m = bounded_weight(a.psi, row);
         // occupied key positions, ascending
         int occ = 0;
         __syncwarp();
@@ -247,11 +396,6 @@ __global__ void __launch_bounds__(kThreads) relative_bounded_kernel(RelativeArgs
             occ += __popc(bits);
         }
         __syncwarp();
-        // a term whose bound is not below the threshold (NaN: not known to be)
-        auto reaches = [&](float bound) {
-            const float e = __fmul_rn(bound, m);
-            return e != e || weight_bucket(e) >= from;
-        };
         const bool row_excluded = hash_find<W>(a.excl, c) >= 0;
         for (int part = 0; part < (row_excluded ? 1 : 2); ++part) {
             const PartView& pv = part == 0 ? a.off : a.diag;
@@ -268,71 +412,64 @@ __global__ void __launch_bounds__(kThreads) relative_bounded_kernel(RelativeArgs
                         se = __ldg(pv.groups + g);
                     }
                     bool alive = se.x < se.y;
-                    if (EMIT && alive) alive = reaches(__ldg(pv.bound + se.x));
+                    if (Pass != kFirst && alive) alive = bounded_reaches(__ldg(pv.bound + se.x), m, from);
                     if (part == 1) {
                         // a group a lane
                         for (int t = se.x; __any_sync(0xffffffffu, alive && t < se.y); ++t) {
                             bool on = false;
-                            int par = 0;
+                            int par = 0, b = 0;
                             if (alive && t < se.y) {
                                 TermRec<W> rec;
                                 load_test<W>(rec, pv, t);
-                                const int b = weight_bucket(__fmul_rn(__ldg(pv.norm + t), m));
+                                b = weight_bucket(__fmul_rn(__ldg(pv.norm + t), m));
                                 on = rec.applies(c) && b >= from;
-                                if (on) {
+                                if (Pass == kEmit && on) {
                                     load_apply<W>(rec, pv, t);
                                     Key<W> img;
                                     par = rec.image(c, img);
-                                    if (!EMIT) atomicAdd(&s_hist[b], 1);
                                 }
                             }
-                            if (EMIT) take(on, c, 1, par, t, row);
+                            bounded_take<W, Pass>(a, hist, on, b, c, 1, par, t, row, lane);
                         }
                         continue;
                     }
-                    // emission: four groups at a time, eight lanes each (a group gives a record or
-                    // two); histogram: a group at a time
-                    constexpr int L = EMIT ? 8 : 32;
+                    if (Pass == kFirst && alive && se.y - se.x > 32 * depth) {
+                        // what is left out, half of it taken to apply, goes to the bucket of its bound
+                        const float rest = __fmul_rn(__ldg(pv.bound + se.x + 32 * depth), m);
+                        const int b = rest == rest ? weight_bucket(rest) : kBuckets - 1;
+                        atomicAdd(deep + b, (se.y - se.x - 32 * depth + 1) / 2);
+                        se.y = se.x + 32 * depth;
+                    }
+                    // above a threshold: four groups at a time, eight lanes each (a group gives a record or
+                    // two); the first count: a group at a time
+                    constexpr int L = Pass == kFirst ? 32 : 8;
                     const int sub = lane / L;
                     for (unsigned todo = __ballot_sync(0xffffffffu, alive); todo != 0;) {
                         int src = -1;
 #pragma unroll
-                        for (int k = 0; k < 32 / L; ++k) {
+                        for (int q = 0; q < 32 / L; ++q) {
                             const int next = __ffs(todo) - 1;
-                            if (sub == k) src = next;
+                            if (sub == q) src = next;
                             todo &= todo - 1;  // (0 stays 0)
                         }
                         const int start = __shfl_sync(0xffffffffu, se.x, src < 0 ? 0 : src);
                         const int end = __shfl_sync(0xffffffffu, se.y, src < 0 ? 0 : src);
-                        const int stop = src < 0 ? start : (!EMIT && end - start > 32 * depth ? start + 32 * depth : end);
                         int t = start + lane % L;
                         bool open = src >= 0;
-                        while (__any_sync(0xffffffffu, open)) {
-                            // everything a term needs is read at once: one trip to L2 before its lookup
-                            bool in = open && t < stop;
-                            bool on = false;
-                            int par = 0;
-                            Key<W> img{};
-                            if (in) {
-                                TermRec<W> rec;
-                                bool narrow = false;
-                                if constexpr (W == 1) narrow = pv.narrow != nullptr;
-                                if (narrow) {
-                                    load_narrow<W>(rec, pv, t);
-                                } else {
-                                    load_test<W>(rec, pv, t);
-                                    if (EMIT) load_apply<W>(rec, pv, t);
+                        for (int step = 0; __any_sync(0xffffffffu, open); ++step) {
+                            if (Pass != kFirst && step == kInline) {
+                                // queue the rest; a full queue leaves it here
+                                bool placed = false;
+                                if (open && lane % L == 0) {
+                                    const unsigned int at = atomicAdd(n_long, 1u);
+                                    placed = at < a.queue_cap;
+                                    if (placed) a.queue[at] = LongGroup{(int)row, t, end};
                                 }
-                                const int b = weight_bucket(__fmul_rn(__ldg(pv.norm + t), m));
-                                if (EMIT) in = reaches(__ldg(pv.bound + t));
-                                on = in && b >= from && rec.applies(c);
-                                if (!EMIT && on) atomicAdd(&s_hist[b], 1);
-                                if (EMIT && on) {
-                                    par = rec.image(c, img);
-                                    on = hash_find<W>(a.excl, img) < 0;
-                                }
+                                placed = __shfl_sync(0xffffffffu, placed, sub * L);
+                                open = open && !placed;
+                                if (!__any_sync(0xffffffffu, open)) break;
                             }
-                            if (EMIT) take(on, img, 0, par, t, row);
+                            const bool in = bounded_term<W, Pass>(a, hist, open && t < end, t, c, m, from, row, lane);
                             // the bounds fall: a group ends at the first lane that stops
                             const unsigned ins = __ballot_sync(0xffffffffu, in);
                             constexpr unsigned kAll = 0xffffffffu >> (32 - L);
@@ -344,19 +481,95 @@ __global__ void __launch_bounds__(kThreads) relative_bounded_kernel(RelativeArgs
             }
         }
     }
-    if (!EMIT) {
-        __syncthreads();
-        for (int k = threadIdx.x; k < kBuckets; k += kThreads) {
-            const int v = s_hist[k];
-            if (v) atomicAdd(a.hist + k, (unsigned long long)v);
+}
+
+// The queued rests, a warp each, 32 terms a step.
+template <int W, int Pass>
+__device__ void bounded_rest(const RelativeArgs& a, const uint64_t* __restrict__ keys, int from, int* hist,
+                             const unsigned int* n_long) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned int queued = __ldcg(n_long);
+    const unsigned int n = queued < a.queue_cap ? queued : a.queue_cap;
+    for (unsigned int k = blockIdx.x * kWarpsPerBlock + warp; k < n; k += gridDim.x * kWarpsPerBlock) {
+        const LongGroup g{__ldcg(&a.queue[k].row), __ldcg(&a.queue[k].t), __ldcg(&a.queue[k].end)};
+        const Key<W> c = load_key<W>(keys, g.row);
+        const float m = bounded_weight(a.psi, g.row);
+        bool open = true;
+        for (int t = g.t + lane; open; t += 32) {
+            const bool in = bounded_term<W, Pass>(a, hist, t < g.end, t, c, m, from, g.row, lane);
+            open = __all_sync(0xffffffffu, in);
         }
     }
+}
+
+__device__ __forceinline__ void bounded_flush(int* shared, unsigned long long* counts) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < kBuckets; k += kThreads) {
+        const int v = shared[k];
+        if (v) atomicAdd(counts + k, (unsigned long long)v);
+        shared[k] = 0;
+    }
+    __syncthreads();
+}
+
+// The first count.
+template <int W>
+__global__ void __launch_bounds__(kThreads) find_first_kernel(RelativeArgs a, const uint64_t* __restrict__ keys, int64_t n,
+                                                              int split, int depth) {
+    __shared__ int s_hist[kBuckets], s_deep[kBuckets];
+    __shared__ uint8_t s_pos[kWarpsPerBlock][64 * W];
+    for (int k = threadIdx.x; k < kBuckets; k += kThreads) s_hist[k] = s_deep[k] = 0;
+    __syncthreads();
+    bounded_rows<W, kFirst>(a, keys, n, split, depth, 0, s_hist, s_deep, s_pos[threadIdx.x >> 5], nullptr);
+    bounded_flush(s_hist, a.hist);
+    bounded_flush(s_deep, a.deep);
+}
+
+// The whole count from the first one's bucket on, where choose_emit_kernel asks
+// for it (rows of very different weights), and the threshold by it, in one
+// cooperative launch.  The counts are left cleared.
+//   top 200,000 of 4,099 rows of 14 on 52, amplitudes falling exponentially:
+//   1,699,998 records emitted by the first count alone, 369,709 by both
+template <int W>
+__global__ void __launch_bounds__(kThreads) find_above_kernel(RelativeArgs a, const uint64_t* keys, int64_t n, int split,
+                                                              double scale, double target) {
+    __shared__ int s_hist[kBuckets];
+    __shared__ uint8_t s_pos[kWarpsPerBlock][64 * W];
+    __shared__ unsigned long long s_warp[32];
+    __shared__ int s_found;
+    const cg::grid_group grid = cg::this_grid();
+    const int from = a.ctl->count_from;
+    if (from == 0) return;  // (the same for every block)
+    for (int k = threadIdx.x; k < kBuckets; k += kThreads) s_hist[k] = 0;
+    __syncthreads();
+    bounded_rows<W, kAbove>(a, keys, n, split, 0, from, s_hist, nullptr, s_pos[threadIdx.x >> 5], a.ctl->n_long);
+    grid.sync();
+    bounded_rest<W, kAbove>(a, keys, from, s_hist, a.ctl->n_long);
+    bounded_flush(s_hist, a.hist);
+    grid.sync();
+    if (blockIdx.x != 0) return;
+    const int b = choose_bucket<kThreads>(a.hist, scale, target, s_warp, &s_found);
+    if (threadIdx.x == 0) a.ctl->emit_from = b > 1 ? b - 1 : 0;
+    for (int k = threadIdx.x; k < kBuckets; k += kThreads) a.hist[k] = 0;
+}
+
+// The emission pass: the rows, and the queued rests behind them.
+template <int W>
+__global__ void __launch_bounds__(kThreads) find_emit_kernel(RelativeArgs a, const uint64_t* __restrict__ keys, int64_t n,
+                                                             int split) {
+    __shared__ uint8_t s_pos[kWarpsPerBlock][64 * W];
+    bounded_rows<W, kEmit>(a, keys, n, split, 0, a.ctl->emit_from, nullptr, nullptr, s_pos[threadIdx.x >> 5], a.ctl->n_long + 1);
+}
+
+template <int W>
+__global__ void __launch_bounds__(kThreads) find_rest_kernel(RelativeArgs a, const uint64_t* __restrict__ keys) {
+    bounded_rest<W, kEmit>(a, keys, a.ctl->emit_from, nullptr, a.ctl->n_long + 1);
 }
 
 // Whether the bounded passes serve the part (QMBX_WALK forces the walks).
 bool relative_bounded(const PartView& off) {
     const char* e = getenv("QMBX_WALK");
-    return off.n >= kGroupedMinTerms && off.wide && off.bound != nullptr &&
+    return off.n >= kGroupedMinTerms && off.wide && off.falling && off.bound != nullptr &&
            !(e != nullptr && (e[0] == 't' || e[0] == 'g' || e[0] == 'p'));
 }
 
@@ -376,10 +589,36 @@ int emission_split(int64_t k, int64_t n_i) {
     return (int)(shares > 16 ? 16 : shares > fill ? shares : fill);
 }
 
-template <int W, bool EMIT>
-int launch_bounded(const RelativeArgs& r, const uint64_t* keys, int64_t n, int split, int depth, cudaStream_t s) {
-    QMBX_KERNEL(kGroupEnumerate, s, relative_bounded_kernel<W, EMIT><<<grouped_grid(n * split), kThreads, 0, s>>>(r, keys, n, split, depth));
-    QMBX_LAUNCH_CHECK(EMIT ? "find_relative emission pass" : "find_relative histogram pass");
+// Blocks of a cooperative launch over `items` warps' work: as many as run at once at most.
+template <class Kernel>
+int cooperative_blocks(Kernel kernel, int64_t items, unsigned* blocks) {
+    int per_sm = 0;
+    QMBX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
+    const int64_t most = (int64_t)per_sm * (pivot_grid() / 4), need = (items + kWarpsPerBlock - 1) / kWarpsPerBlock;
+    *blocks = (unsigned)(need < 1 ? 1 : need < most ? need : most);
+    return QMBX_OK;
+}
+
+template <int W>
+int launch_threshold(RelativeArgs r, const uint64_t* keys, int64_t n, int64_t k, int64_t n_i, double target, cudaStream_t s) {
+    int split = row_split(n);
+    double scale = (double)n_i / (double)n;
+    QMBX_KERNEL(kGroupEnumerate, s, find_first_kernel<W><<<grouped_grid(n * split), kThreads, 0, s>>>(r, keys, n, split, histogram_depth(k, n_i)));
+    QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(r.hist, r.deep, scale, target, r.ctl));
+    unsigned blocks = 0;
+    int st = cooperative_blocks(find_above_kernel<W>, n * split, &blocks);
+    if (st != QMBX_OK) return st;
+    void* args[] = {&r, &keys, &n, &split, &scale, &target};
+    QMBX_KERNEL(kGroupOther, s, QMBX_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)find_above_kernel<W>, dim3(blocks), dim3(kThreads), args, 0, s)));
+    return QMBX_OK;
+}
+
+template <int W>
+int launch_emit(const RelativeArgs& r, const uint64_t* keys, int64_t n, int64_t k, cudaStream_t s) {
+    const int split = emission_split(k, n);
+    QMBX_KERNEL(kGroupEnumerate, s, find_emit_kernel<W><<<grouped_grid(n * split), kThreads, 0, s>>>(r, keys, n, split));
+    QMBX_KERNEL(kGroupOther, s, find_rest_kernel<W><<<2 * pivot_grid(), kThreads, 0, s>>>(r, keys));
+    QMBX_LAUNCH_CHECK("find_relative emission pass");
     return QMBX_OK;
 }
 
@@ -434,73 +673,6 @@ __global__ void sample_rows_kernel(const uint64_t* __restrict__ keys, const doub
     psi_s[j] = psi[r];
 }
 
-// Inclusive scan of v over the 1024 threads of a block in thread order.
-template <class T>
-__device__ __forceinline__ T block_inclusive_scan(T v, T* s_warp) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    T x = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const T y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= d) x += y;
-    }
-    if (lane == 31) s_warp[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        T w = s_warp[lane];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const T y = __shfl_up_sync(0xffffffffu, w, d);
-            if (lane >= d) w += y;
-        }
-        s_warp[lane] = w;
-    }
-    __syncthreads();
-    return warp > 0 ? x + s_warp[warp - 1] : x;
-}
-
-constexpr int kChooseThreads = 1024;
-
-// emit_from from the counts of a histogram pass (scaled by `scale`): one
-// bucket below the highest bucket b whose buckets >= b hold at least
-// `target` records (0 when all buckets above 0 hold fewer); then the counts
-// are cleared.  One block of 1024 threads: thread t sums the 4 buckets
-// [4096 - 4(t + 1), 4096 - 4t), a scan over the threads (highest buckets
-// first) finds the one thread where the running count reaches the target,
-// and that thread walks its buckets.
-__global__ void __launch_bounds__(kChooseThreads) choose_emit_kernel(unsigned long long* __restrict__ hist,
-                                                                     double scale, double target,
-                                                                     FindCtl* __restrict__ ctl) {
-    __shared__ unsigned long long s_warp[32];
-    __shared__ int s_found;
-    constexpr int kPer = kBuckets / kChooseThreads;
-    const int t = threadIdx.x;
-    const int hi = kBuckets - kPer * t;  // thread t covers buckets [hi - kPer, hi)
-    if (t == 0) s_found = 0;
-    // integer counts, scaled only where compared: the running count is exact and monotone, so
-    // exactly one thread sees it cross the target
-    unsigned long long mine = 0;
-    for (int b = hi - 1; b >= hi - kPer && b >= 1; --b) mine += hist[b];
-    const unsigned long long run = block_inclusive_scan(mine, s_warp);
-    if (scale * (double)run >= target && scale * (double)(run - mine) < target) {
-        // the one thread whose buckets reach the target
-        unsigned long long above = run - mine;
-        int b_k = 0;
-        for (int b = hi - 1; b >= hi - kPer && b >= 1; --b) {
-            above += hist[b];
-            if (scale * (double)above >= target) {
-                b_k = b;
-                break;
-            }
-        }
-        ctl->emit_from = b_k > 1 ? b_k - 1 : 0;
-        s_found = 1;
-    }
-    __syncthreads();
-    if (t == 0 && !s_found) ctl->emit_from = 0;
-    for (int b = t; b < kBuckets; b += kChooseThreads) hist[b] = 0;
-}
-
 // ---------------------------------------------------------------------------
 // The tail of a call in two cooperative launches (one block of 1,024 threads
 // per SM, the blocks in step through grid barriers) that take their counts
@@ -509,8 +681,6 @@ __global__ void __launch_bounds__(kChooseThreads) choose_emit_kernel(unsigned lo
 // with two host round trips between them the tail was bound by launching them
 // (the top 50,000 of 121k records: 156 us of kernels in 0.4 ms).
 // ---------------------------------------------------------------------------
-
-namespace cg = cooperative_groups;
 
 constexpr int kTailThreads = 1024;
 constexpr int kTailWarps = kTailThreads / 32;
@@ -824,6 +994,8 @@ struct FindLayout {
     double2* psi_s;         // and its amplitude
     unsigned long long* hist;  // bucket counts; the selection's bins afterwards
     FindCtl* ctl;
+    unsigned long long* deep;
+    LongGroup* queue;
     uint64_t* sel_keys;     // the selected rows' keys, and the buffer they are sorted with
     uint64_t* sort_keys;
     int32_t* sort_counts;
@@ -831,6 +1003,12 @@ struct FindLayout {
     uint64_t* emit_rank;
     uint64_t* emit_keys;
 };
+
+// Places for rests of groups: a few rows with most of the weight have one in each of their groups.
+unsigned int queue_places(int64_t n_i) {
+    const int64_t places = 64 * n_i;
+    return (unsigned int)(places < 1024 ? 1024 : places < (1 << 18) ? places : 1 << 18);
+}
 
 template <int W>
 FindLayout<W> take_find(Arena& ws, int64_t n_i, int64_t k, int64_t n_ex, int64_t cap) {
@@ -842,6 +1020,8 @@ FindLayout<W> take_find(Arena& ws, int64_t n_i, int64_t k, int64_t n_ex, int64_t
     L.psi_s = ws.take<double2>((uint64_t)n_s);
     L.hist = ws.take<unsigned long long>(kBuckets);
     L.ctl = ws.take<FindCtl>(1);
+    L.deep = ws.take<unsigned long long>(kBuckets);
+    L.queue = ws.take<LongGroup>(queue_places(n_i));
     int64_t kk = k > 0 ? k : 1;
     L.sel_keys = ws.take<uint64_t>((uint64_t)kk * W);
     L.sort_keys = ws.take<uint64_t>((uint64_t)kk * W);
@@ -895,8 +1075,8 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
         if ((st = pack_rows<W>(a.configs_i, a.n_i, nq, L.keys_i, s)) != QMBX_OK) return st;
         keys_i = L.keys_i;
     }
-    QMBX_CUDA_TRY(cudaMemsetAsync(L.ctl, 0, sizeof(FindCtl), s));
-    QMBX_CUDA_TRY(cudaMemsetAsync(L.hist, 0, kBuckets * sizeof(unsigned long long), s));
+    // hist, ctl and deep lie one behind the other
+    QMBX_CUDA_TRY(cudaMemsetAsync(L.hist, 0, (size_t)(reinterpret_cast<char*>(L.deep + kBuckets) - reinterpret_cast<char*>(L.hist)), s));
 
     RelativeArgs r{};
     r.psi = reinterpret_cast<const double2*>(a.psi_i);
@@ -906,6 +1086,9 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
     r.diag = part_view(a.table_host, a.table_dev, QMBX_PART_DIAG);
     r.hist = L.hist;
     r.hist_exact = 1;
+    r.deep = L.deep;
+    r.queue = L.queue;
+    r.queue_cap = queue_places(a.n_i);
     r.ctl = L.ctl;
     r.cap_emit = cap;
     r.emit_rank = L.emit_rank;
@@ -928,22 +1111,25 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
         rs.psi = L.psi_s;
         rs.n_i = n_s;
         rs.hist_exact = 0;  // an estimate: every record counted, no exclusion lookups
-        st = bounded ? launch_bounded<W, false>(rs, L.keys_s, n_s, row_split(n_s), histogram_depth(k, a.n_i), s)
-                     : launch_relative<W, false>(rs, L.keys_s, n_s, s);
-        if (st != QMBX_OK) return st;
-        ++g_find_stats.walks;
         // aim at about twice k records above the chosen bucket, one more bucket of slack
-        QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, (double)a.n_i / (double)n_s, 2.0 * (double)k, L.ctl));
+        if (bounded) {
+            if ((st = launch_threshold<W>(rs, L.keys_s, n_s, k, a.n_i, 2.0 * (double)k, s)) != QMBX_OK) return st;
+        } else {
+            if ((st = launch_relative<W, false>(rs, L.keys_s, n_s, s)) != QMBX_OK) return st;
+            QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, nullptr, (double)a.n_i / (double)n_s, 2.0 * (double)k, L.ctl));
+        }
     } else {
         RelativeArgs r1 = r;
         r1.hist_exact = 0;
-        st = bounded ? launch_bounded<W, false>(r1, keys_i, a.n_i, row_split(a.n_i), histogram_depth(k, a.n_i), s)
-                     : launch_relative<W, false>(r1, keys_i, a.n_i, s);
-        if (st != QMBX_OK) return st;
-        ++g_find_stats.walks;
-        QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, 1.0, (double)k, L.ctl));
+        if (bounded) {
+            if ((st = launch_threshold<W>(r1, keys_i, a.n_i, k, a.n_i, (double)k, s)) != QMBX_OK) return st;
+        } else {
+            if ((st = launch_relative<W, false>(r1, keys_i, a.n_i, s)) != QMBX_OK) return st;
+            QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, nullptr, 1.0, (double)k, L.ctl));
+        }
     }
-    QMBX_LAUNCH_CHECK("choose_emit_kernel");
+    ++g_find_stats.walks;
+    QMBX_LAUNCH_CHECK("find_relative threshold");
 
     // bits of the visiting order (term index * n_i + row < n_terms * n_i), in whole bytes
     int order_bytes = 1;
@@ -962,11 +1148,10 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
     // tests drive it).
     FindCtl ctl{};
     for (int attempt = 0;; ++attempt) {
-        st = bounded ? launch_bounded<W, true>(r, keys_i, a.n_i, emission_split(k, a.n_i), 0, s)
-                     : launch_relative<W, true>(r, keys_i, a.n_i, s);
+        st = bounded ? launch_emit<W>(r, keys_i, a.n_i, k, s) : launch_relative<W, true>(r, keys_i, a.n_i, s);
         if (st != QMBX_OK) return st;
         ++g_find_stats.walks;
-        unsigned int* bins = reinterpret_cast<unsigned int*>(L.hist);  // cleared by choose_emit_kernel
+        unsigned int* bins = reinterpret_cast<unsigned int*>(L.hist);  // left cleared by the threshold
         {
             int64_t n_i = a.n_i, want = k, places = cap;
             const double2* psi = r.psi;
@@ -995,7 +1180,7 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
         if ((st = launch_relative<W, false>(r, keys_i, a.n_i, s)) != QMBX_OK) return st;
         ++g_find_stats.walks;
         QMBX_CUDA_TRY(cudaMemsetAsync(L.ctl, 0, sizeof(FindCtl), s));
-        QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, 1.0, (double)k, L.ctl));
+        QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, nullptr, 1.0, (double)k, L.ctl));
         QMBX_LAUNCH_CHECK("choose_emit_kernel");
     }
     const int64_t keep = (int64_t)ctl.n_sel;

@@ -339,8 +339,9 @@ void build_classes(char* blob, const qmbx_table_header& h) {
 
 // Bounds of a part's norms (format.h); the input table is usually sorted by
 // |coef|, and the bounds are then the norms themselves.
-void build_bounds(char* blob, const qmbx_table_header& h, int which) {
-    const qmbx_table_part& p = h.part[which];
+void build_bounds(char* blob, qmbx_table_header& h, int which) {
+    qmbx_table_part& p = h.part[which];
+    int64_t largest = 0;  // terms with no larger norm behind them
     const int32_t* groups = reinterpret_cast<const int32_t*>(blob + p.off_groups);
     const float* norm = reinterpret_cast<const float*>(blob + p.off_norm);
     float* bound = reinterpret_cast<float*>(blob + h.off_bound[which]);
@@ -350,8 +351,10 @@ void build_bounds(char* blob, const qmbx_table_header& h, int which) {
             // a NaN norm stays in the bound: nothing is cut before it
             most = norm[t] == norm[t] && !(norm[t] > most) ? most : norm[t];
             bound[t] = most;
+            if (!(most > norm[t])) ++largest;
         }
     }
+    p.falling = 8 * largest >= 7 * p.n ? 1 : 0;
 }
 
 qmbx_table_header make_header(int64_t n_terms, int32_t n_qubytes, int32_t particle_cut, int64_t n_off, int64_t n_diag,
