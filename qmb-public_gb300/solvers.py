@@ -93,34 +93,17 @@ def _lowest(alpha, beta):
     return float(vals[0]), vecs[:, 0]
 
 
-# Iterations between two looks at most.  The host looks at the norms of some iterations while the next ones run,
-# so that at most seven run past the end of the recurrence; with 16 iterations and then a look, a start that ends
-# after two of them cost 16 (1,000,000 rows of an entry each: 1.2 ms of products became 25).
-_LOOK_EVERY = 4
-
-
-class _Look:
-    """A copy of the iterations' scalars on its way to the host."""
-
-    def __init__(self, values: torch.Tensor):
-        self.count = values.shape[1]
-        if values.is_cuda:
-            self.host = torch.empty(values.shape, dtype=values.dtype, pin_memory=True)
-            self.host.copy_(values, non_blocking=True)
-            self.done = torch.cuda.Event()
-            self.done.record(torch.cuda.current_stream(values.device))
-        else:
-            self.host, self.done = values.clone(), None
-
-    def get(self) -> np.ndarray:
-        if self.done is not None:
-            self.done.synchronize()
-        return self.host.numpy()
+# Iterations between two looks at most; the first looks come after 2, 6 and 14 iterations, so that seven at most run
+# past the end of the recurrence.  A look is a wait of 30 us; without the early ones, a start that ends after two
+# iterations cost 16 (1,000,000 rows of an entry each: 1.2 ms of products became 25).
+_LOOK_EVERY = 8
+# rows up to which vectors are allocated 16 at a time (64 MB at most); more rows take as many as there are so far
+_SMALL_ROWS = 1 << 18
 
 
 def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
     """The recurrence on a stored matrix: its scalars stay on the device, and the host looks for a norm
-    below the threshold a few iterations behind (what ran past it is dropped)."""
+    below the threshold every few iterations (what ran past it is dropped)."""
     n, device = mat.n, start.device
     if start.shape != (n,) or device != mat.val.device:
         raise RuntimeError(f"start must have shape [{n}] and be on the matrix's device.")
@@ -128,29 +111,25 @@ def _lanczos_on_matrix(mat, start: torch.Tensor, step: int, threshold: float):
     start = start.to(torch.complex128).resolve_conj().resolve_neg()
     first = start / torch.linalg.norm(torch.view_as_real(start))
     blocks = [first.reshape(1, n).contiguous()]
-    looks, seen, at = [], [], 0
+    seen = []
     v, v_prev, beta_prev, done, stop = blocks[0][0], None, None, 0, None
-    # iteration k forms alpha[k], beta[k] and vector k + 1; the last one's beta and vector are not used
     room = 0  # vectors that the last of `blocks` still has room for
+    # iteration k forms alpha[k], beta[k] and vector k + 1; the last one's beta and vector are not used
     while done < step + 2 and stop is None:
-        count = min(_LOOK_EVERY, max(1, done // 2), step + 2 - done)
+        count = min(done + 2, _LOOK_EVERY, step + 2 - done)
         scalars = torch.empty((2, count), dtype=torch.float64, device=device)  # alpha and beta of the iterations
         for k in range(count):
             if room == 0:
-                room = min(16, max(1, done + k))
+                room = 16 if n <= _SMALL_ROWS else min(16, max(1, done + k))
                 blocks.append(torch.empty((room, n), dtype=torch.complex128, device=device))
             v_next = blocks[-1][-room]
             mat.lanczos_step(v_prev, beta_prev, v, v_next, scalars[0, k], scalars[1, k], scratch)
             v_prev, v, beta_prev, room = v, v_next, scalars[1, k], room - 1
-        looks.append(_Look(scalars))
+        seen.append(scalars.cpu().numpy())
+        small = np.nonzero(seen[-1][1] < threshold)[0]
+        if len(small) and done + small[0] < step + 1:
+            stop = int(done + small[0])
         done += count
-        # two iterations stay queued while the host looks at the ones before, so that the device does not wait
-        while stop is None and looks and (done == step + 2 or at + looks[0].count <= done - 2):
-            seen.append(looks.pop(0).get())
-            small = np.nonzero(seen[-1][1] < threshold)[0]
-            if len(small) and at + small[0] < step + 1:
-                stop = int(at + small[0])
-            at += seen[-1].shape[1]
     used = (step + 1 if stop is None else stop) + 1  # vectors 0 .. used - 1
     host = np.concatenate(seen, axis=1)[:, :used]
     if used == 1:
