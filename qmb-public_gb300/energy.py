@@ -16,7 +16,7 @@ from __future__ import annotations
 import torch
 
 from . import _native
-from .hamiltonian import Hamiltonian
+from .hamiltonian import Hamiltonian, _plain
 
 __all__ = ["variational_energy"]
 
@@ -26,7 +26,7 @@ class _HermitianEnergy(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, ham: Hamiltonian, configs, psi):
-        given, psi = psi, psi.detach().resolve_conj().resolve_neg().contiguous()
+        given, psi = psi, _plain(psi.detach())
         if psi.dtype == torch.complex64:
             hpsi = ham.apply_within_compensated(configs, psi, configs)
         else:

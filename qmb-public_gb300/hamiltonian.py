@@ -52,6 +52,11 @@ def _workspace(nbytes: int, device: torch.device) -> torch.Tensor:
     return ws
 
 
+def _plain(x: torch.Tensor) -> torch.Tensor:
+    """x as its memory has it: contiguous, with conjugations and signs that torch only marks carried out."""
+    return x.resolve_conj().resolve_neg().contiguous()
+
+
 def _pinned(nbytes: int) -> torch.Tensor:
     """A host buffer for a table blob: page-locked where a GPU is present, so the device copy is one DMA."""
     buf = torch.empty(nbytes, dtype=torch.uint8)
@@ -210,7 +215,7 @@ class Hamiltonian:
             raise RuntimeError(f"{name} must have shape [{n}].")
         if psi.device != device:
             raise RuntimeError(f"{name} must be on the same device as others.")
-        return psi.contiguous()
+        return _plain(psi)
 
     # -- apply_within ---------------------------------------------------------
 
@@ -313,7 +318,7 @@ class Hamiltonian:
         forward found more hits than the record holds.  The hit count is copied back without
         waiting and sizes the next log of this shape."""
         device = record.buf.device
-        g = g.to(record.dtype).contiguous()
+        g = _plain(g.to(record.dtype))
         if g.shape != (record.n_j,):
             raise RuntimeError(f"g must have shape [{record.n_j}].")
         table = record.table
@@ -521,8 +526,8 @@ class Hamiltonian:
 class HamiltonianMatrix:
     """H restricted to one set of distinct rows, stored on the device as a sparse matrix (CSR).
 
-    Built by ``Hamiltonian.matrix``: two term walks over the rows (count, then
-    fill); ``apply(x)`` is then a sparse matrix-vector product, which is what
+    Built by ``Hamiltonian.matrix`` in two passes over the rows (count, then
+    fill; pair scans or term walks); ``apply(x)`` is then a sparse matrix-vector product, which is what
     an iterative eigensolver on a fixed basis (qmb/rldiag.py:19-52,
     qmb/haar.py:107-183) needs once per iteration.  Row j holds its diagonal
     entry first, then one entry per (term, row i) pair mapping row i onto row
@@ -543,7 +548,7 @@ class HamiltonianMatrix:
             raise RuntimeError(f"x must be complex128 of shape [{self.n}] or [{self.n}, m].")
         if x.device != self.val.device:
             raise RuntimeError("x must be on the matrix's device.")
-        x = x.contiguous()
+        x = _plain(x)
         y = torch.empty_like(x)
         m = 1 if x.dim() == 1 else x.shape[1]
         with torch.cuda.device(x.device):
