@@ -317,12 +317,14 @@ def measured_peaks() -> tuple[float, str]:
 # Sources whose change invalidates a committed ncu figure of the engine's kernels.
 KERNEL_SOURCES = ("qmb-public_gb300/csrc/device.cuh", "qmb-public_gb300/csrc/apply.cu",
                   "qmb-public_gb300/csrc/keys.cu", "qmb-public_gb300/csrc/relative.cu",
+                  "qmb-public_gb300/csrc/pairs.cuh", "qmb-public_gb300/csrc/pairs.cu",
                   "qmb-public_gb300/csrc/format.h", "qmb-public_gb300/csrc/table.cpp")
-# the sources of the apply_within walks (profiles of grouped_kernel / enumerate_kernel under apply_within)
+# the sources of apply_within's walks and of the pair scan
 APPLY_SOURCES = ("qmb-public_gb300/csrc/device.cuh", "qmb-public_gb300/csrc/apply.cu",
+                 "qmb-public_gb300/csrc/pairs.cuh", "qmb-public_gb300/csrc/pairs.cu",
                  "qmb-public_gb300/csrc/keys.cu", "qmb-public_gb300/csrc/format.h",
                  "qmb-public_gb300/csrc/table.cpp")
-# the sources of find_relative's walks
+# the sources of find_relative's passes
 RELATIVE_SOURCES = ("qmb-public_gb300/csrc/device.cuh", "qmb-public_gb300/csrc/relative.cu",
                     "qmb-public_gb300/csrc/keys.cu", "qmb-public_gb300/csrc/format.h",
                     "qmb-public_gb300/csrc/table.cpp")
@@ -339,8 +341,8 @@ def kernel_sources_sha(sources=KERNEL_SOURCES) -> str:
     return h.hexdigest()[:16]
 
 
-# the committed ncu summary (profiles/<name>.json) of each workload's dominant walk kernel
-WALK_FIGURES = {"c2": "term_walk_c2", "c4": "tiled_walk_c4", "c5": "pivot_walk_c5", "c3": "pivot_walk_c3"}
+# the committed ncu summary (profiles/<name>.json) of the kernel that the workload's enumeration time is
+WALK_FIGURES = {"c2": "pair_scan_c2", "c3": "pair_scan_c3", "c4": "reach_walk_c4"}
 
 
 def ncu_figures(name: str) -> dict | None:
@@ -613,7 +615,7 @@ def run_ours(args, wl, rank: int, world: int) -> dict | None:
     alg_adj = n_i * (nq + 16) + n_j * (nq + 8) + T * 28
     alg = alg_fwd if walks_per_step < 1.5 else (alg_fwd + alg_adj) / 2
     per_launch_ms = ms_enum / max(n_enum, 1)
-    figs = ncu_figures(WALK_FIGURES.get(args.workload, f"term_walk_{args.workload}"))
+    figs = ncu_figures(WALK_FIGURES.get(args.workload, ""))
     ms_step32 = ms32 / args.steps
     value = replica_value(units, ms_step32, world)
     # the radix sorts of find_relative: passes x 2 x records x record bytes over their device time
@@ -754,7 +756,7 @@ def run_extra(args, wl) -> dict:
     def walk_roofline(prof, n_walk, n_look, amp, kernel):
         cnt, ms = prof["groups"]["enumerate"]
         return hbm_roofline(walk_alg(n_walk, n_look, amp), ms / max(cnt, 1), kernel,
-                            ncu_figures(WALK_FIGURES.get(args.workload, f"term_walk_{args.workload}")), launches=cnt)
+                            ncu_figures(WALK_FIGURES.get(args.workload, "")), launches=cnt)
 
     if args.workload == "c3":
         mlp = _Mlp(8 * nq, device, seed=wl["spec"]["seed"])
@@ -886,7 +888,7 @@ def run_extra(args, wl) -> dict:
                      "higher_is_better": False, "dtype": "f64", "count_selected": K, "e0": result["e"][0],
                      "e2": result["e"][1],
                      "roofline": walk_roofline(prof, n, n, 16,
-                                           "find_relative passes (relative_bounded_kernel) and pair scan"),
+                                           "find_relative passes (find_first_kernel, find_emit_kernel) and pair scan"),
                      "kernel_groups_ms_per_run": {g: v[1] for g, v in prof["groups"].items()}})
     elif args.workload == "sampler":
         from oracle import sampler as oracle_sampler
@@ -936,7 +938,7 @@ def run_extra(args, wl) -> dict:
                      "ms_per_step": ms, "higher_is_better": False, "dtype": "f64", "count_selected": K,
                      "rows_out": int(rel.shape[0]), "term_applications_per_s": T * n / (ms * 1e-3),
                      "stats": stats,
-                     "roofline": walk_roofline(prof, n, ci.shape[0], 16, "find_relative passes (relative_bounded_kernel)"),
+                     "roofline": walk_roofline(prof, n, ci.shape[0], 16, "find_relative passes (find_first_kernel, find_emit_kernel)"),
                      "sort_roofline": hbm_roofline(stats["sort_bytes"], ms_sort, "sort and output of the selected rows",
                                                    None, launches_per_call=n_sort) if ms_sort > 0 else None,
                      "kernel_groups_ms_per_run": {g: v[1] for g, v in prof["groups"].items()}})

@@ -2,10 +2,11 @@
 //
 // The reference's Lanczos loops (qmb/rldiag.py:19-52, qmb/haar.py:107-183)
 // call apply_within on the same rows once per iteration, so every iteration
-// walks the whole term table again.  Here the walk runs twice in total (count
-// the entries of every row, then fill them) and each iteration is a sparse
-// matrix-vector product over the stored entries, which reads nnz x 20 bytes
-// from HBM instead of walking T terms per row.
+// walks the whole term table again.  Here the rows are compared with each
+// other, or their terms walked, twice in total (count the entries of every
+// row, then fill them) and each iteration is a sparse matrix-vector product
+// over the stored entries, which reads nnz x 20 bytes from HBM instead of
+// walking T terms per row.
 //
 // Layout (CSR): row j holds, at [row_ptr[j], row_ptr[j + 1]), first the
 // diagonal entry (column j, the sum of the diagonal terms, possibly zero),

@@ -77,7 +77,8 @@ struct PairWork {
     bool same;
 };
 
-// Blocks of the scan: four resident per SM on 152 SMs.
+// Blocks of the scan at most.  Three are resident on each of 152 SMs (80 registers a thread; two at 256 positions); the
+// rest start behind them and mostly find every work item handed out.
 constexpr int kPairBlocks = 608;
 constexpr int kPairCounters = 6;
 // Words of 64 bits for a set's hist (a count for each of 0 .. 64 W particles, twice, as ints).

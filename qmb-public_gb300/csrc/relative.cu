@@ -39,7 +39,7 @@ constexpr int kBuckets = 4096;
 // Figures of the calling thread's last find_relative call (qmbx_find_relative_stats).
 struct FindStats {
     int64_t records;      // records emitted by the selection pass
-    int64_t walks;        // term walks run (histogram and emission passes)
+    int64_t walks;        // threshold and emission passes run
     int64_t sort_passes;  // radix passes over records and selected rows
     int64_t sort_bytes;   // passes x 2 (read + write) x items x item bytes
     int64_t selected;     // records selected before de-duplication
