@@ -991,9 +991,24 @@ bool take_pairs_behind(const ApplyArgs& a, const Arena& ws, uint64_t base, PairW
 
 // Whether a call has scratch for Reach: tables of few terms (their walks are
 // tiled) over enough rows to outweigh building it, 1,000,000 rows of two words
-// take 35 us, their walk 1.12 ms without and 0.31 ms with it.
+// take 35 us, their walk 1.12 ms without and 0.31 ms with it.  The words that
+// stay when one is left out have to tell the rows apart: two words of 72 sites
+// leave 8 with the second one, which all rows share (and whose few places in
+// the filter every row's atomic meets).  Lattices, whole calls without and
+// with it in us, FP64 at half filling and FP32 at an eighth:
+//   sites  rows          half             an eighth
+//      72  400,000     376   451        227   578
+//      80  400,000     441   383        273   323
+//      96  150,000     229   134        154   163
+//      96  400,000     531   231        321   304
+//     112   65,536     185   138        132   134
+//     112  400,000     611   244        366   301
+//     128   65,536     206   143        145   128
 bool reach_scratch(const qmbx_table_header* h, int64_t n_i, int64_t n_j) {
-    return h->n_words > 1 && h->part[QMBX_PART_FWD].n < kGroupedMinTerms && n_i >= kFewWideRows && n_j >= kFewWideRows;
+    if (h->n_words < 2 || h->part[QMBX_PART_FWD].n >= kGroupedMinTerms) return false;
+    const int64_t rows = n_i < n_j ? n_i : n_j;
+    const int left = h->n_sites - 64;  // sites of the words that stay, at least
+    return left >= 48 ? rows >= kFewWideRows : left >= 32 && rows >= 4 * kFewWideRows;
 }
 
 // Forward maps amplitudes on configs_i (input side) to configs_j (output

@@ -1174,10 +1174,10 @@ __global__ void __launch_bounds__(kThreads) grouped_split_kernel(V v, Src src, i
 // share a row; lane s takes positions s, 15 - s, 16 + s, ... of its occupied
 // ones (the early ones have more partners).  The visitor's init must read
 // nothing: it also runs for the lanes past the last row.
-// Bound by the gathers of groups and coefficients from L1.  On GB300, FP64,
-// against the faster of the tiled and the grouped walk: 200,000 rows of 14
-// under 1,379 terms 515 -> 217 us, 20,000 rows of 10 under 407 terms 54 -> 20
-// us, 4,000 rows of 20 under 2,927 terms 72 -> 28 us.
+// Bound by the gathers of groups and coefficients from L1 and by FP64
+// additions.  On GB300, FP64, against the faster of the tiled and the grouped
+// walk: 20,000 rows of 10 under 407 terms 54 -> 15 us, of 8 under 301 terms 39
+// -> 12 us, 4,000 rows of 20 under 2,927 terms 72 -> 24 us.
 template <int W, class V, class Src>
 __global__ void __launch_bounds__(kThreads) diag_groups_kernel(V v, Src src, const int* __restrict__ n_rows,
                                                                int64_t n_max, PartView diag) {

@@ -1495,7 +1495,10 @@ SingleOrder take_single_order(Arena& ws, int64_t n, int words) {
 }
 
 // Whether rows are taken through the terms in key order: where the walks would
-// visit enough terms to outweigh ordering them.
+// visit enough terms to outweigh ordering them.  (rows x terms, whole calls by
+// the walk and in order, us: 400 x 55,371, rows of 10, 175 and 84, of 4, 68
+// and 82; 1,500 x 14,251 100 and 90; 6,000 x 14,251 121 and 91; below the line
+// 200 x 55,371 171 by the walk.)
 bool single_ordered(const PartView& off, int64_t n) {
     const char* e = getenv("QMBX_WALK");
     const char f = e != nullptr ? e[0] : 0;

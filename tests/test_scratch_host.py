@@ -55,3 +55,28 @@ def test_sizes_that_may_scan_ask_for_it_whatever_is_forced(blob, monkeypatch):
         monkeypatch.setenv("QMBX_WALK", walk)
         assert _asked(blob, 60000, 60000) == free
     assert free["apply"] >= 8 * (1 << 22)
+
+
+def _lattice_bytes(sites, n_qubytes, n):
+    out = {}
+    for a in range(sites - 1):
+        out[((a, 1), (a + 1, 0))] = out[((a + 1, 1), (a, 0))] = -1.0
+    site, kind, coef = (x.numpy() for x in terms.sort_terms(*terms.prepare(out)))
+    lattice = compile_table(native.library(), site, kind, coef, n_qubytes, 1)
+    size = ctypes.c_uint64()
+    native.check(native.library().qmbx_apply_within_workspace(lattice.ctypes.data, n, n, ctypes.byref(size)))
+    return size.value
+
+
+@pytest.mark.parametrize("sites,n,bounded", [(72, 1000000, False), (80, 1000000, False), (96, 100000, False), (96, 300000, True),
+                                             (112, 65535, False), (112, 65536, True), (136, 65536, True)])
+def test_walks_are_bounded_where_the_other_words_tell_rows_apart(sites, n, bounded, monkeypatch):
+    # the bound's filters take 32 bits a row and word, twice at most for rounding; row sets and sums of two and three
+    # words are compared with those of a table that is never bounded (72 sites; 136 without its rows)
+    monkeypatch.delenv("QMBX_WALK", raising=False)
+    if sites > 128:
+        assert bounded
+        assert _lattice_bytes(sites, 17, n) - _lattice_bytes(sites, 17, n - 1) > 4 * 3 * n // 2
+        return
+    extra = _lattice_bytes(sites, (sites + 7) // 8, n) - _lattice_bytes(66, 9, n)
+    assert (extra >= 4 * 2 * n // 2) == bounded
