@@ -76,6 +76,8 @@ struct FindCtl {
     int overflow;
     int emit_from;                 // lowest bucket the emission pass keeps
     int count_from;                // the first count's bucket (> 0) if a whole count from it follows, else 0
+    unsigned int first_done;       // blocks of the first count that have finished, and of the whole one
+    unsigned int above_done;
     unsigned int n_long[2];        // groups queued for their rest (LongGroup): by the threshold's count, by the emission
 };
 
@@ -251,30 +253,34 @@ __device__ __forceinline__ int choose_bucket(const unsigned long long* hist, dou
     return found;
 }
 
-// emit_from from the counts of a histogram pass: one bucket below the one
-// that choose_bucket finds (0 when all buckets above 0 hold fewer).  deep (or
-// NULL): by bucket, what the pass left out; where that could be more than half
-// of the target from the bucket on, count_from asks for a whole count.  The
-// counts are left cleared.
-constexpr int kChooseThreads = 1024;
-
-__global__ void __launch_bounds__(kChooseThreads) choose_emit_kernel(unsigned long long* __restrict__ hist,
-                                                                     const unsigned long long* __restrict__ deep,
-                                                                     double scale, double target,
-                                                                     FindCtl* __restrict__ ctl) {
-    __shared__ unsigned long long s_warp[32];
-    __shared__ int s_found;
-    const int b = choose_bucket<kChooseThreads>(hist, scale, target, s_warp, &s_found);
+// emit_from from the counts of a histogram pass, by one block: one bucket
+// below the one that choose_bucket finds (0 when all buckets above 0 hold
+// fewer).  deep (or NULL): by bucket, what the pass left out; where that could
+// be more than half of the target from the bucket on, count_from asks for a
+// whole count.  The counts are left cleared.
+template <int Threads>
+__device__ __forceinline__ void choose_emit(unsigned long long* hist, const unsigned long long* deep, double scale,
+                                            double target, FindCtl* ctl, unsigned long long* s_warp, int* s_found) {
+    const int b = choose_bucket<Threads>(hist, scale, target, s_warp, s_found);
     unsigned long long left_out = 0;
-    for (int k = threadIdx.x; k < kBuckets; k += kChooseThreads) {
-        if (deep != nullptr && k >= (b > 1 ? b : 1)) left_out += deep[k];
+    for (int k = threadIdx.x; k < kBuckets; k += Threads) {
+        if (deep != nullptr && k >= (b > 1 ? b : 1)) left_out += __ldcg(deep + k);
         hist[k] = 0;
     }
-    left_out = block_inclusive_scan<kChooseThreads>(left_out, s_warp);
-    if (threadIdx.x == kChooseThreads - 1) {
+    left_out = block_inclusive_scan<Threads>(left_out, s_warp);
+    if (threadIdx.x == Threads - 1) {
         ctl->emit_from = b > 1 ? b - 1 : 0;
         ctl->count_from = scale * (double)left_out > 0.5 * target ? (b > 1 ? b : 1) : 0;
     }
+}
+
+constexpr int kChooseThreads = 1024;
+
+__global__ void __launch_bounds__(kChooseThreads) choose_emit_kernel(unsigned long long* hist, double scale, double target,
+                                                                     FindCtl* ctl) {
+    __shared__ unsigned long long s_warp[32];
+    __shared__ int s_found;
+    choose_emit<kChooseThreads>(hist, nullptr, scale, target, ctl, s_warp, &s_found);
 }
 
 // The same passes over parts whose groups hold many terms (PartView::wide) in
@@ -512,45 +518,67 @@ __device__ __forceinline__ void bounded_flush(int* shared, unsigned long long* c
     __syncthreads();
 }
 
-// The first count.
+// The first count; the last block to finish chooses the threshold by it.
 template <int W>
 __global__ void __launch_bounds__(kThreads) find_first_kernel(RelativeArgs a, const uint64_t* __restrict__ keys, int64_t n,
-                                                              int split, int depth) {
+                                                              int split, int depth, double scale, double target) {
     __shared__ int s_hist[kBuckets], s_deep[kBuckets];
     __shared__ uint8_t s_pos[kWarpsPerBlock][64 * W];
+    __shared__ unsigned long long s_warp[32];
+    __shared__ int s_found;
+    __shared__ bool s_last;
     for (int k = threadIdx.x; k < kBuckets; k += kThreads) s_hist[k] = s_deep[k] = 0;
     __syncthreads();
     bounded_rows<W, kFirst>(a, keys, n, split, depth, 0, s_hist, s_deep, s_pos[threadIdx.x >> 5], nullptr);
     bounded_flush(s_hist, a.hist);
     bounded_flush(s_deep, a.deep);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&a.ctl->first_done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    choose_emit<kThreads>(a.hist, a.deep, scale, target, a.ctl, s_warp, &s_found);
 }
 
-// The whole count from the first one's bucket on, where choose_emit_kernel asks
-// for it (rows of very different weights), and the threshold by it, in one
-// cooperative launch.  The counts are left cleared.
+// The whole count from the first one's bucket on, where choose_emit asks for
+// it (rows of very different weights): the rows, then the queued rests and, by
+// the last block to finish, the threshold.  The counts are left cleared.
 //   top 200,000 of 4,099 rows of 14 on 52, amplitudes falling exponentially:
 //   1,699,998 records emitted by the first count alone, 369,709 by both
 template <int W>
-__global__ void __launch_bounds__(kThreads) find_above_kernel(RelativeArgs a, const uint64_t* keys, int64_t n, int split,
-                                                              double scale, double target) {
+__global__ void __launch_bounds__(kThreads) find_above_kernel(RelativeArgs a, const uint64_t* __restrict__ keys, int64_t n,
+                                                              int split) {
     __shared__ int s_hist[kBuckets];
     __shared__ uint8_t s_pos[kWarpsPerBlock][64 * W];
-    __shared__ unsigned long long s_warp[32];
-    __shared__ int s_found;
-    const cg::grid_group grid = cg::this_grid();
     const int from = a.ctl->count_from;
-    if (from == 0) return;  // (the same for every block)
+    if (from == 0) return;
     for (int k = threadIdx.x; k < kBuckets; k += kThreads) s_hist[k] = 0;
     __syncthreads();
     bounded_rows<W, kAbove>(a, keys, n, split, 0, from, s_hist, nullptr, s_pos[threadIdx.x >> 5], a.ctl->n_long);
-    grid.sync();
+    bounded_flush(s_hist, a.hist);
+}
+
+template <int W>
+__global__ void __launch_bounds__(kThreads) find_above_rest_kernel(RelativeArgs a, const uint64_t* __restrict__ keys,
+                                                                   double scale, double target) {
+    __shared__ int s_hist[kBuckets];
+    __shared__ unsigned long long s_warp[32];
+    __shared__ int s_found;
+    __shared__ bool s_last;
+    const int from = a.ctl->count_from;
+    if (from == 0) return;
+    for (int k = threadIdx.x; k < kBuckets; k += kThreads) s_hist[k] = 0;
+    __syncthreads();
     bounded_rest<W, kAbove>(a, keys, from, s_hist, a.ctl->n_long);
     bounded_flush(s_hist, a.hist);
-    grid.sync();
-    if (blockIdx.x != 0) return;
-    const int b = choose_bucket<kThreads>(a.hist, scale, target, s_warp, &s_found);
-    if (threadIdx.x == 0) a.ctl->emit_from = b > 1 ? b - 1 : 0;
-    for (int k = threadIdx.x; k < kBuckets; k += kThreads) a.hist[k] = 0;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&a.ctl->above_done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    choose_emit<kThreads>(a.hist, nullptr, scale, target, a.ctl, s_warp, &s_found);
 }
 
 // The emission pass: the rows, and the queued rests behind them.
@@ -589,27 +617,14 @@ int emission_split(int64_t k, int64_t n_i) {
     return (int)(shares > 16 ? 16 : shares > fill ? shares : fill);
 }
 
-// Blocks of a cooperative launch over `items` warps' work: as many as run at once at most.
-template <class Kernel>
-int cooperative_blocks(Kernel kernel, int64_t items, unsigned* blocks) {
-    int per_sm = 0;
-    QMBX_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
-    const int64_t most = (int64_t)per_sm * (pivot_grid() / 4), need = (items + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    *blocks = (unsigned)(need < 1 ? 1 : need < most ? need : most);
-    return QMBX_OK;
-}
-
 template <int W>
-int launch_threshold(RelativeArgs r, const uint64_t* keys, int64_t n, int64_t k, int64_t n_i, double target, cudaStream_t s) {
-    int split = row_split(n);
-    double scale = (double)n_i / (double)n;
-    QMBX_KERNEL(kGroupEnumerate, s, find_first_kernel<W><<<grouped_grid(n * split), kThreads, 0, s>>>(r, keys, n, split, histogram_depth(k, n_i)));
-    QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(r.hist, r.deep, scale, target, r.ctl));
-    unsigned blocks = 0;
-    int st = cooperative_blocks(find_above_kernel<W>, n * split, &blocks);
-    if (st != QMBX_OK) return st;
-    void* args[] = {&r, &keys, &n, &split, &scale, &target};
-    QMBX_KERNEL(kGroupOther, s, QMBX_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)find_above_kernel<W>, dim3(blocks), dim3(kThreads), args, 0, s)));
+int launch_threshold(const RelativeArgs& r, const uint64_t* keys, int64_t n, int64_t k, int64_t n_i, double target, cudaStream_t s) {
+    const int split = row_split(n);
+    const double scale = (double)n_i / (double)n;
+    QMBX_KERNEL(kGroupEnumerate, s, find_first_kernel<W><<<grouped_grid(n * split), kThreads, 0, s>>>(r, keys, n, split, histogram_depth(k, n_i), scale, target));
+    QMBX_KERNEL(kGroupOther, s, find_above_kernel<W><<<grouped_grid(n * split), kThreads, 0, s>>>(r, keys, n, split));
+    QMBX_KERNEL(kGroupOther, s, find_above_rest_kernel<W><<<pivot_grid(), kThreads, 0, s>>>(r, keys, scale, target));
+    QMBX_LAUNCH_CHECK("find_relative threshold");
     return QMBX_OK;
 }
 
@@ -1116,7 +1131,7 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
             if ((st = launch_threshold<W>(rs, L.keys_s, n_s, k, a.n_i, 2.0 * (double)k, s)) != QMBX_OK) return st;
         } else {
             if ((st = launch_relative<W, false>(rs, L.keys_s, n_s, s)) != QMBX_OK) return st;
-            QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, nullptr, (double)a.n_i / (double)n_s, 2.0 * (double)k, L.ctl));
+            QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, (double)a.n_i / (double)n_s, 2.0 * (double)k, L.ctl));
         }
     } else {
         RelativeArgs r1 = r;
@@ -1125,7 +1140,7 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
             if ((st = launch_threshold<W>(r1, keys_i, a.n_i, k, a.n_i, (double)k, s)) != QMBX_OK) return st;
         } else {
             if ((st = launch_relative<W, false>(r1, keys_i, a.n_i, s)) != QMBX_OK) return st;
-            QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, nullptr, 1.0, (double)k, L.ctl));
+            QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, 1.0, (double)k, L.ctl));
         }
     }
     ++g_find_stats.walks;
@@ -1180,7 +1195,7 @@ int find_impl(const FindArgs& a, void* workspace, uint64_t workspace_bytes, uint
         if ((st = launch_relative<W, false>(r, keys_i, a.n_i, s)) != QMBX_OK) return st;
         ++g_find_stats.walks;
         QMBX_CUDA_TRY(cudaMemsetAsync(L.ctl, 0, sizeof(FindCtl), s));
-        QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, nullptr, 1.0, (double)k, L.ctl));
+        QMBX_KERNEL(kGroupSelect, s, choose_emit_kernel<<<1, kChooseThreads, 0, s>>>(L.hist, 1.0, (double)k, L.ctl));
         QMBX_LAUNCH_CHECK("choose_emit_kernel");
     }
     const int64_t keep = (int64_t)ctl.n_sel;

@@ -54,7 +54,11 @@ def _workspace(nbytes: int, device: torch.device) -> torch.Tensor:
 
 def _plain(x: torch.Tensor) -> torch.Tensor:
     """x as its memory has it: contiguous, with conjugations and signs that torch only marks carried out."""
-    return x.resolve_conj().resolve_neg().contiguous()
+    if x.is_conj():
+        x = x.resolve_conj()
+    if x.is_neg():
+        x = x.resolve_neg()
+    return x.contiguous()
 
 
 def _pinned(nbytes: int) -> torch.Tensor:
