@@ -291,10 +291,10 @@ __global__ void __launch_bounds__(kChooseThreads) choose_emit_kernel(unsigned lo
 // Selections take few records of a row (121k of 5.7e7 for the top 50,000 of
 // 20,000 rows under 55,371 terms), so most groups end at their first bound:
 // the pass is a few instructions per group instead of a test per term, and is
-// bound by the latency of its reads.  On GB300, emission passes against the
-// walks: those rows 428 -> 70 us, the top 1,000,000 of 8,192 rows under 3.1M
-// terms 4.58 -> 0.50 ms (pivot-major walk and diagonal pass), the top 200,000
-// of 4,099 rows under 669,579 terms 1.42 -> 0.21 ms.
+// bound by the latency of its reads.  On GB300, emission passes (with the
+// rests) against the walks: those rows 428 -> 81 us, the top 1,000,000 of
+// 8,192 rows under 3.1M terms 4.58 -> 0.35 ms (pivot-major walk and diagonal
+// pass), the top 200,000 of 4,099 rows under 669,579 terms 1.42 -> 0.08 ms.
 //
 // Three passes share the code:
 //   kFirst  counts the first `depth` steps of 32 terms of every group, all
